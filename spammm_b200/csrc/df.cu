@@ -9,17 +9,16 @@
 //   df_loss_seed        spammm/SPM/AFM.py:3125-3200
 // All arithmetic is FP64, as on the reference host.  The FEs volume is
 // (nx,ny,nz,4) float32 with z fastest.  The amplitude df is FP64-arithmetic
-// bound (9 quadrature nodes x 2 interpolations per output): the z-column
-// kernels tabulate each interpolated sample once per column, and the finite
-// differences multiply by 1/dr and 1/(2 dr) instead of dividing (within an
+// bound, so the nine quadrature nodes are folded into one filter per direction
+// and the finite differences multiply by 1/dr and 1/(2 dr) instead of dividing (within an
 // FP64 ulp of numpy.gradient's division; the float32 results are unchanged at
 // the reference fixtures' tolerance).  Compiled with -fmad=false so the FP64
 // expression order otherwise matches NumPy's.
 #include "spm_internal.cuh"
 #include "spm_diss.cuh"
 #include "spm_batch.cuh"
+#include <algorithm>
 #include <cmath>
-#include <vector>
 
 namespace spm {
 namespace {
@@ -145,30 +144,137 @@ df_amp_dir_kernel(const T* __restrict__ FEs, DfGeom P, const int* __restrict__ o
 }
 
 // Oscillation along +-z only (the common case): one warp per pixel column.
-// The column's F_n values are staged once in shared memory (coalesced reads of
-// nz contiguous rows); each lane then evaluates its output heights with the
-// same expression sequence as df_amp_dir_kernel (x/y weights are exactly 1
-// there and the zero-weight corners are skipped), so results are identical.
+//
+// The nine shifted samples of a height are one fixed filter on the column: node
+// k reads F_n at floor(u_k shift) and the next height with constant linear
+// weights, so A[j] = sum_k wk S(j, u_k) is at most 18 taps (ZTaps, merged on the
+// host), and the average of the nine central differences is the central
+// difference of A.  Per output that is 18 FP64 FMAs and one difference where the
+// node-by-node form took 9 x (floor, conversions, two products, a difference):
+// the FP64 and conversion instructions bound it (0.32 ms on a 480 x 480 x 60
+// volume against 0.04 ms for its bytes), this form is bound by the shared-memory
+// reads of the taps.  Column ends clamp the tap's height (mode='nearest'): the
+// staged column is padded with its end values so that the tap loop has no
+// clamps, as far as pads and column fit the buffer; a longer one clamps.
 constexpr int DFZ_WARPS = 8;
 constexpr int DFZ_MAXNZ = 512;
-constexpr int DFZ_TAB = 64;  // columns up to this height take each quadrature sample once (a table row)
+constexpr int DFZ_TAB = 64;  // columns up to this height take A of each height once (a table row)
+constexpr double TAP_SNAP = 1e-14;  // a linear weight this close to 0 or 1 is that (the rounding of j + u shift)
 
-// acc - wk * (central difference of the tabulated samples at height iz): the
-// per-node step of the amplitude average, the one-sided difference at the
-// column's ends (iz < 0 or >= nz: no output, acc unchanged).
-__device__ __forceinline__ double df_accumulate(double acc, int iz, int nz, const double* row, double idr,
-                                                double idr2, double wkn) {
-    if (iz < 0 || iz >= nz) return acc;
-    double g;
-    if (iz == 0) g = (row[1] - row[0]) * idr;
-    else if (iz == nz - 1) g = (row[nz - 1] - row[nz - 2]) * idr;
-    else g = (row[iz + 1] - row[iz - 1]) * idr2;
-    return acc - wkn * g;
+struct ZTaps {
+    int n, padl, padr;
+    int off[2 * NQ];
+    double w[2 * NQ];
+};
+
+// floor and linear weight of a constant shift x in samples.
+void split_shift(double x, long long& m, double& t) {
+    const double f = floor(x);
+    m = (long long)std::min(std::max(f, -1e15), 1e15);
+    t = x - f;
+    if (t < TAP_SNAP) t = 0.0;
+    if (t > 1.0 - TAP_SNAP) { t = 0.0; m += 1; }
+}
+
+// The taps of a shift of `sh` samples.  Offsets beyond +-2^30 read the column's ends like any other
+// beyond them; a shift that is not finite makes every value NaN.
+ZTaps make_ztaps(const DfGeom& P, double sh) {
+    ZTaps T = {};
+    if (!std::isfinite(sh)) {
+        T.n = 1;
+        T.w[0] = std::nan("");
+        return T;
+    }
+    auto add = [&](long long off, double w) {
+        if (w == 0.0) return;  // never read: a non-finite neighbour does not count
+        const int o = (int)std::min(std::max(off, -(1LL << 30)), 1LL << 30);
+        for (int i = 0; i < T.n; i++)
+            if (T.off[i] == o) { T.w[i] += w; return; }
+        T.off[T.n] = o;
+        T.w[T.n++] = w;
+    };
+    for (int k = 0; k < NQ; k++) {
+        long long m;
+        double t;
+        split_shift(P.uk[k] * sh, m, t);
+        add(m, P.wk * (1.0 - t));
+        add(m + 1, P.wk * t);
+    }
+    for (int i = 0; i < T.n; i++) {
+        if (-T.off[i] > T.padl) T.padl = -T.off[i];
+        if (T.off[i] > T.padr) T.padr = T.off[i];
+    }
+    return T;
+}
+
+// Heights of a column and its pads fit the staging buffer.
+__device__ __forceinline__ bool z_padded(const ZTaps& T, int nz) {
+    return (long long)nz + T.padl + T.padr <= DFZ_MAXNZ;
+}
+
+// A[j] from the staged column (fn[j] = height j; PAD: heights -padl .. nz-1+padr hold the clamped
+// values).  Two partial sums in a fixed order.
+template <bool PAD>
+__device__ __forceinline__ double tap_sum(const double* fn, int nz, int j, const ZTaps& T) {
+    double a = 0.0, b = 0.0;
+    auto at = [&](int i) { return fn[PAD ? j + T.off[i] : clampi(j + T.off[i], nz)]; };
+    // unrolled over the most taps there can be: offsets and weights are then immediate constant-bank
+    // operands (indexed constant loads per tap bound the rolled loop: 140 us on the 480 x 480 x 60 volume)
+#pragma unroll
+    for (int i = 0; i < 2 * NQ; i += 2) {
+        if (i < T.n) a = __fma_rn(T.w[i], at(i), a);
+        if (i + 1 < T.n) b = __fma_rn(T.w[i + 1], at(i + 1), b);
+    }
+    return a + b;
+}
+
+// df of one staged column by a warp: store(o, value) for every output o, whose height is iz_of(o)
+// (outside [0, nz): NaN); c1, c2: -n_z^2 / dr and -n_z^2 / (2 dr).  nz >= 2.
+template <bool PAD, class IzOf, class Store>
+__device__ __forceinline__ void df_column(const double* fn, double* row, int nz, int l, const ZTaps& T, double c1,
+                                          double c2, int n_out, const IzOf& iz_of, const Store& store) {
+    const bool tab = nz <= DFZ_TAB;
+    if (tab) {
+        for (int j = l; j < nz; j += 32) row[j] = tap_sum<PAD>(fn, nz, j, T);
+        __syncwarp();
+    }
+    auto A = [&](int j) { return tab ? row[j] : tap_sum<PAD>(fn, nz, j, T); };
+    for (int o = l; o < n_out; o += 32) {
+        const int iz = iz_of(o);
+        if (iz < 0 || iz >= nz) {
+            store(o, __int_as_float(0x7fc00000));
+            continue;
+        }
+        const int jp = iz + 1 < nz ? iz + 1 : nz - 1, jm = iz > 0 ? iz - 1 : 0;
+        store(o, (float)((A(jp) - A(jm)) * (jp - jm == 2 ? c2 : c1)));
+    }
+}
+
+// Fz of row i of a z-only oscillation, NaN where Fx or Fy is not finite (the general sum F.n multiplies
+// them by 0).  A float row takes no FP64 arithmetic beyond its one conversion; n_z is applied to the
+// difference.
+__device__ __forceinline__ double z_at(const float* __restrict__ v, size_t i) {
+    const float4 f = __ldg(reinterpret_cast<const float4*>(v) + i);
+    return (double)((f.x * 0.f + f.y * 0.f) + f.z);
+}
+__device__ __forceinline__ double z_at(const double* __restrict__ v, size_t i) {
+    const Row f = load_row(v, i);
+    return (f.x * 0.0 + f.y * 0.0) + f.z;
+}
+
+// Stage a column (fn_at(z), z < nz) with its end values repeated over the pads.
+template <class FnAt>
+__device__ __forceinline__ void stage_column(double* buf, int nz, int l, int padl, int padr, const FnAt& fn_at_z) {
+    for (int z = l; z < nz; z += 32) buf[padl + z] = fn_at_z(z);
+    __syncwarp();
+    for (int i = l; i < padl; i += 32) buf[i] = buf[padl];
+    for (int i = l; i < padr; i += 32) buf[padl + nz + i] = buf[padl + nz - 1];
+    __syncwarp();
 }
 
 template <typename T>
 __global__ void __launch_bounds__(DFZ_WARPS * 32)
-df_amp_z_kernel(const T* __restrict__ FEs, DfGeom P, const int* __restrict__ out_iz, int n_out,
+df_amp_z_kernel(const T* __restrict__ FEs, DfGeom P, ZTaps Z, const int* __restrict__ out_iz, int n_out,
                 float* __restrict__ df) {
     __shared__ double s_fn[DFZ_WARPS][DFZ_MAXNZ];
     __shared__ double s_row[DFZ_WARPS][DFZ_TAB];
@@ -176,71 +282,171 @@ df_amp_z_kernel(const T* __restrict__ FEs, DfGeom P, const int* __restrict__ out
     const long long pix = (long long)blockIdx.x * DFZ_WARPS + w;
     if (pix >= (long long)P.nx * P.ny) return;  // whole warp exits together: no CTA barrier below
     const int nz = P.nz;
-    double* fn = s_fn[w];
-    for (int z = l; z < nz; z += 32) {
-        const Row f = load_row(FEs, (size_t)pix * nz + z);
-        fn[z] = (f.x * P.n[0] + f.y * P.n[1]) + f.z * P.n[2];
+    const bool pad = z_padded(Z, nz);
+    double* fn = s_fn[w] + (pad ? Z.padl : 0);
+    stage_column(s_fn[w], nz, l, pad ? Z.padl : 0, pad ? Z.padr : 0, [&](int z) { return z_at(FEs, (size_t)pix * nz + z); });
+    const double n2 = -P.n[2] * P.n[2], c1 = n2 * P.idr[2], c2 = n2 * P.idr2[2];
+    auto iz_of = [&](int o) { return out_iz ? out_iz[o] : o; };
+    auto store = [&](int o, float v) { df[pix * n_out + o] = v; };
+    if (pad) df_column<true>(fn, s_row[w], nz, l, Z, c1, c2, n_out, iz_of, store);
+    else df_column<false>(fn, s_row[w], nz, l, Z, c1, c2, n_out, iz_of, store);
+}
+
+// Any other oscillation direction: the same filter in three dimensions.  Node k
+// reads the eight corners of one cell at a constant offset with constant
+// weights, so A = sum_k wk S(., u_k) is at most 72 taps (merged on the host) and
+// df = -sum_a n_a dA/dr_a.  A CTA stages F_n of its tile, widened by the taps'
+// reach and one sample for the differences, in shared memory (indices clamped to
+// the volume, mode='nearest'), forms A once per point of the tile and takes the
+// differences from it.  df_amp_dir_kernel evaluates 9 nodes x 3 axes x 2 samples
+// x 8 corners per output from global memory, 432 rows against 72 shared doubles
+// and 2 staged rows: 482 -> 41 us on a 101 x 97 x 41 float64 volume.
+constexpr int DFT_THREADS = 256;
+constexpr int DFT_MAX = 8 * NQ;
+
+struct TileTaps {
+    int n;
+    int lo[3], hi[3];        // reach of the taps along each axis
+    int t[3];                // outputs per tile
+    int a[3], f[3];          // points of A and of F_n per tile
+    int e[3];                // 1 along the axes that are differentiated
+    int off[DFT_MAX];        // linear offsets in the staged F_n
+    double w[DFT_MAX];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(DFT_THREADS)
+df_amp_tile_kernel(const T* __restrict__ FEs, DfGeom P, TileTaps Q, int nty, int ntz, const int* __restrict__ out_iz,
+                   int n_out, float* __restrict__ df) {
+    extern __shared__ double s_tile[];
+    double* s_f = s_tile;
+    double* s_a = s_tile + Q.f[0] * Q.f[1] * Q.f[2];
+    const int b = blockIdx.x;
+    const int o0[3] = {b / (nty * ntz) * Q.t[0], b / ntz % nty * Q.t[1], b % ntz * Q.t[2]};
+    const int nf = Q.f[0] * Q.f[1] * Q.f[2], na = Q.a[0] * Q.a[1] * Q.a[2];
+    for (int i = threadIdx.x; i < nf; i += DFT_THREADS) {
+        const int z = i % Q.f[2], y = i / Q.f[2] % Q.f[1], x = i / Q.f[2] / Q.f[1];
+        s_f[i] = fn_at(FEs, P, clampi(o0[0] - Q.e[0] + Q.lo[0] + x, P.nx), clampi(o0[1] - Q.e[1] + Q.lo[1] + y, P.ny),
+                       clampi(o0[2] - Q.e[2] + Q.lo[2] + z, P.nz));
     }
-    __syncwarp();
-    const double sh = P.shift[2], nzc = P.n[2];
-    auto S = [&](int j, double u) {
-        const double c = (double)j + u * sh;
-        const double fl = floor(c);
-        const double t = c - fl;
-        const int i0 = (int)fl;
-        const double w0 = 1.0 - t, w1 = t;
+    __syncthreads();
+    for (int i = threadIdx.x; i < na; i += DFT_THREADS) {
+        const int z = i % Q.a[2], y = i / Q.a[2] % Q.a[1], x = i / Q.a[2] / Q.a[1];
+        const double* f = s_f + ((x - Q.lo[0]) * Q.f[1] + (y - Q.lo[1])) * Q.f[2] + (z - Q.lo[2]);
+        double s0 = 0.0, s1 = 0.0;
+        int k = 0;
+#pragma unroll 4
+        for (; k + 1 < Q.n; k += 2) {
+            s0 = __fma_rn(Q.w[k], f[Q.off[k]], s0);
+            s1 = __fma_rn(Q.w[k + 1], f[Q.off[k + 1]], s1);
+        }
+        if (k < Q.n) s0 = __fma_rn(Q.w[k], f[Q.off[k]], s0);
+        s_a[i] = s0 + s1;
+    }
+    __syncthreads();
+    // with a height list (out_iz) ntz is 1 and the tile holds every height
+    const int zo = out_iz ? n_out : min(Q.t[2], P.nz - o0[2]);
+    const int xo = min(Q.t[0], P.nx - o0[0]), yo = min(Q.t[1], P.ny - o0[1]);
+    const int dims[3] = {P.nx, P.ny, P.nz}, st[3] = {Q.a[1] * Q.a[2], Q.a[2], 1};
+    for (int i = threadIdx.x; i < xo * yo * zo; i += DFT_THREADS) {
+        const int o = i % zo, y = i / zo % yo, x = i / zo / yo;
+        const int iz = out_iz ? out_iz[o] : o0[2] + o;
+        const size_t at = ((size_t)(o0[0] + x) * P.ny + (o0[1] + y)) * n_out + (out_iz ? o : iz);
+        if (iz < 0 || iz >= P.nz) {
+            df[at] = __int_as_float(0x7fc00000);
+            continue;
+        }
+        const int g[3] = {o0[0] + x, o0[1] + y, iz};
+        const double* A = s_a + ((x + Q.e[0]) * Q.a[1] + (y + Q.e[1])) * Q.a[2] + (iz - o0[2] + Q.e[2]);
         double acc = 0.0;
-        if (w0 != 0.0) acc += fn[clampi(i0, nz)] * w0;
-        if (w1 != 0.0) acc += fn[clampi(i0 + 1, nz)] * w1;
-        return acc;
-    };
-    if (nz >= 2 && nz <= DFZ_TAB && n_out <= DFZ_TAB) {
-        // each S(j, u_k) once: per quadrature node the warp tabulates the column's nz samples, then
-        // every output takes its central difference from the table (same values, same order)
-        double* row = s_row[w];
-        int izs[DFZ_TAB / 32];
-        double acc[DFZ_TAB / 32];
 #pragma unroll
-        for (int m = 0; m < DFZ_TAB / 32; m++) {
-            const int o = l + 32 * m;
-            izs[m] = o < n_out ? (out_iz ? out_iz[o] : o) : -1;
-            acc[m] = 0.0;
+        for (int d = 0; d < 3; d++) {
+            if (!Q.e[d]) continue;
+            const int up = g[d] + 1 < dims[d] ? 1 : 0, dn = g[d] > 0 ? 1 : 0;
+            acc -= P.n[d] * ((A[up * st[d]] - A[-dn * st[d]]) * (up + dn == 2 ? P.idr2[d] : P.idr[d]));
         }
-        for (int k = 0; k < NQ; k++) {
-            const double u = P.uk[k];
-            for (int j = l; j < nz; j += 32) row[j] = S(j, u);
-            __syncwarp();
-#pragma unroll
-            for (int m = 0; m < DFZ_TAB / 32; m++) acc[m] = df_accumulate(acc[m], izs[m], nz, row, P.idr[2], P.idr2[2], P.wk * nzc);
-            __syncwarp();  // the row is rewritten for the next node
-        }
-#pragma unroll
-        for (int m = 0; m < DFZ_TAB / 32; m++) {
-            const int o = l + 32 * m;
-            if (o < n_out)
-                df[pix * n_out + o] = (izs[m] < 0 || izs[m] >= nz) ? __int_as_float(0x7fc00000) : (float)acc[m];
-        }
-        return;
+        df[at] = (float)acc;
     }
-    for (int o = l; o < n_out; o += 32) {
-        const int iz = out_iz ? out_iz[o] : o;
-        float res;
-        if (iz < 0 || iz >= nz) {
-            res = __int_as_float(0x7fc00000);
-        } else {
-            double acc = 0.0;
-            for (int k = 0; k < NQ; k++) {
-                const double u = P.uk[k];
-                double g;
-                if (iz == 0) g = (S(1, u) - S(0, u)) * P.idr[2];
-                else if (iz == nz - 1) g = (S(nz - 1, u) - S(nz - 2, u)) * P.idr[2];
-                else g = (S(iz + 1, u) - S(iz - 1, u)) * P.idr2[2];
-                acc -= (P.wk * nzc) * g;
+}
+
+// Taps and tile of a direction; false when the shift's reach leaves no tile that fits shared memory
+// (the general kernel then).  The tile: 4 x 8 columns of up to 32 heights (all of them with a height
+// list), halved along x, y while it does not fit 96 KB (two CTAs per SM).
+bool make_tile(const DfGeom& P, bool list, TileTaps& Q) {
+    const int dims[3] = {P.nx, P.ny, P.nz};
+    Q = TileTaps{};
+    struct Tap { int o[3]; double w; } tap[DFT_MAX];
+    for (int d = 0; d < 3; d++)
+        if (!(fabs(P.shift[d]) < 1e6)) return false;
+    for (int a = 0; a < P.nact; a++) Q.e[P.act[a]] = 1;
+    for (int k = 0; k < NQ; k++) {
+        long long m[3];
+        double t[3];
+        for (int d = 0; d < 3; d++) split_shift(P.uk[k] * P.shift[d], m[d], t[d]);
+        for (int c = 0; c < 8; c++) {
+            double w = P.wk;
+            int o[3];
+            for (int d = 0; d < 3; d++) {
+                const int hi = (c >> (2 - d)) & 1;
+                w *= hi ? t[d] : 1.0 - t[d];
+                o[d] = (int)m[d] + hi;
             }
-            res = (float)acc;
+            if (w == 0.0) continue;
+            int i = 0;
+            while (i < Q.n && !(tap[i].o[0] == o[0] && tap[i].o[1] == o[1] && tap[i].o[2] == o[2])) i++;
+            if (i < Q.n) {
+                tap[i].w += w;
+                continue;
+            }
+            tap[Q.n].w = w;
+            for (int d = 0; d < 3; d++) tap[Q.n].o[d] = o[d];
+            Q.n++;
         }
-        df[pix * n_out + o] = res;
     }
+    for (int d = 0; d < 3; d++) {
+        Q.lo[d] = Q.hi[d] = tap[0].o[d];
+        for (int i = 1; i < Q.n; i++) {
+            Q.lo[d] = Q.lo[d] < tap[i].o[d] ? Q.lo[d] : tap[i].o[d];
+            Q.hi[d] = Q.hi[d] > tap[i].o[d] ? Q.hi[d] : tap[i].o[d];
+        }
+    }
+    Q.t[0] = 4;
+    Q.t[1] = 8;
+    const int nzt = list ? 1 : (P.nz + 31) / 32;
+    Q.t[2] = (P.nz + nzt - 1) / nzt;
+    while (true) {
+        long long nf = 1, na = 1;
+        for (int d = 0; d < 3; d++) {
+            if (Q.t[d] > dims[d]) Q.t[d] = dims[d];
+            Q.a[d] = Q.t[d] + 2 * Q.e[d];
+            Q.f[d] = Q.a[d] + Q.hi[d] - Q.lo[d];
+            nf *= Q.f[d];
+            na *= Q.a[d];
+        }
+        if ((nf + na) * 8 <= 96 * 1024) break;
+        const int d = Q.t[0] >= Q.t[1] ? 0 : 1;
+        if (Q.t[d] == 1) return false;
+        Q.t[d] = (Q.t[d] + 1) / 2;
+    }
+    for (int i = 0; i < Q.n; i++) {
+        Q.w[i] = tap[i].w;
+        Q.off[i] = (tap[i].o[0] * Q.f[1] + tap[i].o[1]) * Q.f[2] + tap[i].o[2];
+    }
+    return true;
+}
+
+template <typename T>
+int launch_df_tile(const T* FEs, const DfGeom& P, const TileTaps& Q, const int* out_iz, int n_out, float* df,
+                   cudaStream_t st) {
+    const size_t smem = ((size_t)Q.f[0] * Q.f[1] * Q.f[2] + (size_t)Q.a[0] * Q.a[1] * Q.a[2]) * sizeof(double);
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(df_amp_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem) != cudaSuccess)
+        return set_error(SPM_ERR_CUDA, "spm_df_amp_dir: cannot enable %zu B of shared memory", smem);
+    const int ntx = (P.nx + Q.t[0] - 1) / Q.t[0], nty = (P.ny + Q.t[1] - 1) / Q.t[1];
+    const int ntz = (P.nz + Q.t[2] - 1) / Q.t[2];
+    df_amp_tile_kernel<<<(unsigned)((long long)ntx * nty * ntz), DFT_THREADS, smem, st>>>(FEs, P, Q, nty, ntz, out_iz,
+                                                                                        n_out, df);
+    return check_launch("spm_df_amp_dir");
 }
 
 template <typename T>
@@ -444,13 +650,20 @@ extern "C" int spm_df_amp_dir(const void* FEs, int fes_dtype, int nx, int ny, in
     if (n[0] == 0.0 && n[1] == 0.0 && nz <= DFZ_MAXNZ) {  // z-only oscillation: column kernel
         const long long npix = (long long)nx * ny;
         const unsigned nb = (unsigned)((npix + DFZ_WARPS - 1) / DFZ_WARPS);
+        const ZTaps Z = make_ztaps(P, P.shift[2]);
         if (fes_dtype == SPM_F32)
-            df_amp_z_kernel<<<nb, DFZ_WARPS * 32, 0, as_stream(stream)>>>(static_cast<const float*>(FEs), P, out_iz,
+            df_amp_z_kernel<<<nb, DFZ_WARPS * 32, 0, as_stream(stream)>>>(static_cast<const float*>(FEs), P, Z, out_iz,
                                                                            n_out, df);
         else
-            df_amp_z_kernel<<<nb, DFZ_WARPS * 32, 0, as_stream(stream)>>>(static_cast<const double*>(FEs), P, out_iz,
+            df_amp_z_kernel<<<nb, DFZ_WARPS * 32, 0, as_stream(stream)>>>(static_cast<const double*>(FEs), P, Z, out_iz,
                                                                            n_out, df);
         return check_launch("spm_df_amp_dir");
+    }
+    TileTaps Q;
+    if (make_tile(P, out_iz != nullptr, Q)) {
+        if (fes_dtype == SPM_F32)
+            return launch_df_tile(static_cast<const float*>(FEs), P, Q, out_iz, n_out, df, as_stream(stream));
+        return launch_df_tile(static_cast<const double*>(FEs), P, Q, out_iz, n_out, df, as_stream(stream));
     }
     const unsigned nb = (unsigned)((total + DF_THREADS - 1) / DF_THREADS);
     if (fes_dtype == SPM_F32)
@@ -561,7 +774,7 @@ namespace {
 // are written back in stroke order.
 __global__ void __launch_bounds__(DFZ_WARPS * 32)
 batch_df_amp_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, long long n_pix,
-                    const float* __restrict__ FEs, DfGeom P, float* __restrict__ df) {
+                    const float* __restrict__ FEs, DfGeom P, ZTaps Z, float* __restrict__ df) {
     __shared__ double s_fn[DFZ_WARPS][DFZ_MAXNZ];
     __shared__ double s_row[DFZ_WARPS][DFZ_TAB];
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -574,56 +787,14 @@ batch_df_amp_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, long long
         for (int o = l; o < nz; o += 32) df[s0 + o] = __int_as_float(0x7fc00000);
         return;
     }
-    double* fn = s_fn[w];
-    for (int z = l; z < nz; z += 32) {
-        const Row f = load_row(FEs, (size_t)(s0 + (nz - 1 - z)));
-        fn[z] = (f.x * P.n[0] + f.y * P.n[1]) + f.z * P.n[2];
-    }
-    __syncwarp();
-    const double sh = P.shift[2], nzc = P.n[2];
-    auto S = [&](int j, double u) {
-        const double c = (double)j + u * sh;
-        const double fl = floor(c);
-        const double t = c - fl;
-        const int i0 = (int)fl;
-        const double w0 = 1.0 - t, w1 = t;
-        double acc = 0.0;
-        if (w0 != 0.0) acc += fn[clampi(i0, nz)] * w0;
-        if (w1 != 0.0) acc += fn[clampi(i0 + 1, nz)] * w1;
-        return acc;
-    };
-    if (nz <= DFZ_TAB) {  // each S(j, u_k) once, as df_amp_z_kernel
-        double* row = s_row[w];
-        double acc[DFZ_TAB / 32];
-#pragma unroll
-        for (int m = 0; m < DFZ_TAB / 32; m++) acc[m] = 0.0;
-        for (int k = 0; k < NQ; k++) {
-            const double u = P.uk[k];
-            for (int j = l; j < nz; j += 32) row[j] = S(j, u);
-            __syncwarp();
-#pragma unroll
-            for (int m = 0; m < DFZ_TAB / 32; m++) acc[m] = df_accumulate(acc[m], l + 32 * m, nz, row, P.idr[2], P.idr2[2], P.wk * nzc);
-            __syncwarp();  // the row is rewritten for the next node
-        }
-#pragma unroll
-        for (int m = 0; m < DFZ_TAB / 32; m++) {
-            const int iz = l + 32 * m;
-            if (iz < nz) df[s0 + (nz - 1 - iz)] = (float)acc[m];
-        }
-        return;
-    }
-    for (int iz = l; iz < nz; iz += 32) {
-        double acc = 0.0;
-        for (int k = 0; k < NQ; k++) {
-            const double u = P.uk[k];
-            double g;
-            if (iz == 0) g = (S(1, u) - S(0, u)) * P.idr[2];
-            else if (iz == nz - 1) g = (S(nz - 1, u) - S(nz - 2, u)) * P.idr[2];
-            else g = (S(iz + 1, u) - S(iz - 1, u)) * P.idr2[2];
-            acc -= (P.wk * nzc) * g;
-        }
-        df[s0 + (nz - 1 - iz)] = (float)acc;
-    }
+    const bool pad = z_padded(Z, nz);
+    double* fn = s_fn[w] + (pad ? Z.padl : 0);
+    stage_column(s_fn[w], nz, l, pad ? Z.padl : 0, pad ? Z.padr : 0, [&](int z) { return z_at(FEs, (size_t)(s0 + (nz - 1 - z))); });
+    const double c1 = -P.idr[2], c2 = -P.idr2[2];  // n = z
+    auto iz_of = [](int o) { return o; };
+    auto store = [&](int o, float v) { df[s0 + (nz - 1 - o)] = v; };
+    if (pad) df_column<true>(fn, s_row[w], nz, l, Z, c1, c2, nz, iz_of, store);
+    else df_column<false>(fn, s_row[w], nz, l, Z, c1, c2, nz, iz_of, store);
 }
 
 // Loss chunks per CTA of the partials and gradient kernels.  The first
@@ -792,7 +963,8 @@ extern "C" int spm_batch_df_amp(int n_mol, const spm_batch_mol* mols, long long 
     if (rc) return rc;
     const long long nb = (n_pixels + DFZ_WARPS - 1) / DFZ_WARPS;
     SPM_REQUIRE(nb < (1LL << 31), "spm_batch_df_amp: too many pixels");
-    batch_df_amp_kernel<<<(unsigned)nb, DFZ_WARPS * 32, 0, as_stream(stream)>>>(n_mol, mols, n_pixels, FEs, P, df);
+    batch_df_amp_kernel<<<(unsigned)nb, DFZ_WARPS * 32, 0, as_stream(stream)>>>(n_mol, mols, n_pixels, FEs, P,
+                                                                                make_ztaps(P, P.shift[2]), df);
     return check_launch("spm_batch_df_amp");
 }
 
