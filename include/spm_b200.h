@@ -370,7 +370,7 @@ long long spm_adjoint_grid_scratch_bytes(int n_atoms, long long n_state);
  * fields and the buffer offsets: atom_off, pix_off and state_off contiguous
  * from 0 (each molecule's rows right after the previous molecule's), grid_off
  * increasing with non-overlapping slabs;
- * spm_batch_prepare fills tile_off, slot_off, unit_off and chunk_off for a
+ * spm_batch_prepare fills tile_off, slot_off, unit_off, chunk_off and block_off for a
  * given spm_batch_shape, which every launch on these descriptors must then
  * be given unchanged.  The descriptor array is copied to device memory by the
  * caller; launches take the DEVICE copy.  Layouts:
@@ -405,7 +405,7 @@ typedef struct spm_batch_mol {
     int raster_ny;        /* > 0: points form an (n_scan/raster_ny) x raster_ny raster */
     int x_lo, nx_slab;    /* stored columns */
     int y_lo, ny_slab;    /* stored rows */
-    int reserved;
+    int block_off;        /* first far-field lattice cell of the grid build (spm_batch_prepare) */
     float p0[4], dA[4], dB[4], dC[4];   /* node geometry (dA,dB,dC as spm_grid_build) */
     float dinvA[4], dinvB[4], dinvC[4]; /* sampling transform (as spm_scan_params) */
 } spm_batch_mol;

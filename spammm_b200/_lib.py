@@ -100,7 +100,7 @@ class BatchMol(ctypes.Structure):
         ("z_lo", ctypes.c_int), ("nz_slab", ctypes.c_int),
         ("nz_steps", ctypes.c_int), ("raster_ny", ctypes.c_int),
         ("x_lo", ctypes.c_int), ("nx_slab", ctypes.c_int), ("y_lo", ctypes.c_int), ("ny_slab", ctypes.c_int),
-        ("reserved", ctypes.c_int),
+        ("block_off", ctypes.c_int),
         ("p0", _f4), ("dA", _f4), ("dB", _f4), ("dC", _f4),
         ("dinvA", _f4), ("dinvB", _f4), ("dinvC", _f4),
     ]

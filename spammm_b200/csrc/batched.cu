@@ -8,9 +8,11 @@
 //   unit_off   adjoint node units    ceil(slab nodes/adj_chunk) (0 without states)
 //   chunk_off  loss chunks           ceil(states/256)
 //   row_off    adjoint partial rows  units x n_atoms
+//   block_off  far-field lattice cells of the grid build (far_cells, spm_batch.cuh)
 // The kernels find the molecule of a work item by binary search over these
 // prefixes, so one launch per stage covers any mix of molecule sizes.
 #include "spm_internal.cuh"
+#include "spm_batch.cuh"
 #include <cmath>
 
 extern "C" spm_batch_shape spm_batch_default_shape(void) {
@@ -54,7 +56,7 @@ extern "C" int spm_batch_prepare(spm_batch_mol* mols, int n_mol, const spm_batch
     SPM_REQUIRE(S.adj_stage == 0 || (S.adj_stage == 1 && S.adj_ilp == 1), "spm_batch_prepare: adj_stage=%d",
                 S.adj_stage);
     const long long th = S.rx_tile_h, tw = 32 / S.rx_tile_h;
-    long long tiles = 0, slots = 0, units = 0, chunks = 0, states = 0, atoms = 0, pixels = 0, grid_end = 0, rows = 0;
+    long long tiles = 0, slots = 0, units = 0, chunks = 0, states = 0, atoms = 0, pixels = 0, grid_end = 0, rows = 0, blocks = 0;
     for (int m = 0; m < n_mol; m++) {
         spm_batch_mol& D = mols[m];
         SPM_REQUIRE(D.n_atoms >= 0 && D.n_scan >= 0 && D.nz_steps >= 0, "spm_batch_prepare: molecule %d: negative counts",
@@ -83,6 +85,8 @@ extern "C" int spm_batch_prepare(spm_batch_mol* mols, int n_mol, const spm_batch
         if (D.raster_ny > 0 && D.n_scan % D.raster_ny != 0) D.raster_ny = 0;  // not a full raster: 1D order
         const long long nst = (long long)D.n_scan * D.nz_steps;
         D.tile_off = tiles;
+        D.block_off = (int)blocks;
+        blocks += far_cells(D);
         D.slot_off = slots;
         D.unit_off = units;
         D.chunk_off = chunks;
@@ -105,7 +109,7 @@ extern "C" int spm_batch_prepare(spm_batch_mol* mols, int n_mol, const spm_batch
         atoms += D.n_atoms;
         pixels += D.n_scan;
         grid_end = D.grid_off + slab;
-        SPM_REQUIRE(atoms < (1LL << 30) && pixels < (1LL << 31), "spm_batch_prepare: batch too large");
+        SPM_REQUIRE(atoms < (1LL << 30) && pixels < (1LL << 31) && blocks < (1LL << 31), "spm_batch_prepare: batch too large");
     }
     SPM_REQUIRE(tiles < (1LL << 31) && slots < (1LL << 31) && units < (1LL << 31) && chunks < (1LL << 31) &&
                 rows < (1LL << 40), "spm_batch_prepare: batch too large for one launch per stage");

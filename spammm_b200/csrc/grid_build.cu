@@ -18,9 +18,15 @@
 //     MUFU rsqrt per pair in total for LJ + on-node Coulomb); sites with a
 //     non-zero offset get their own rsqrt.
 // Transcendentals use MUFU approximations (rsqrt.approx, ex2.approx).
+//
+// That direct sum is for systems of few atoms.  From SPM_FAR_MIN_ATOMS atoms on the
+// nodes are built in blocks of 16^3, each atom at a block's nodes only when it is
+// near the block; the smooth field of the distant atoms is evaluated at 8^3
+// Chebyshev points of the block and interpolated (build_block below).
 #include "spm_internal.cuh"
 #include "spm_batch.cuh"
 #include "spm_f32x2.cuh"
+#include <cmath>
 
 namespace spm {
 namespace {
@@ -79,6 +85,128 @@ struct StoreBox {
     int x_lo, nxs, y_lo, nys, zst_lo, zst_hi;
 };
 
+// One atom's pair law and tip-charge terms added to ZP node pairs of a z-column at (px, py): a =
+// (x, y, z, Q*qs_on), c = the transformed pair parameters, q[k] = Q*Qs[k]*C of the off-node sites.
+template <int KIND, bool ON, int NOFF, int ZP>
+__device__ __forceinline__ void add_atom(const float4 a, const float4 c, const float* q, float px, float py,
+                                         const f2 (&pz)[ZP], const TipSites& S, f2 (&fx)[ZP], f2 (&fy)[ZP],
+                                         f2 (&fz)[ZP], f2 (&fe)[ZP]) {
+    const f2 one = bc(1.f);
+                    const float dxs = px - a.x;
+                    const float dys = py - a.y;
+                    const float dxy2s = fmaf(dxs, dxs, fmaf(dys, dys, R2SAFE));
+                    const f2 dx = bc(dxs), dy = bc(dys), dxy2 = bc(dxy2s), az = bc(a.z);
+                    const f2 c0 = bc(c.x), c1 = bc(c.y), c2 = bc(c.z), c3 = bc(c.w);
+                    const f2 qon = bc(a.w);
+    #pragma unroll
+                    for (int p = 0; p < ZP; p++) {
+                        const f2 dz = sub2(pz[p], az);
+                        const f2 r2 = fma2(dz, dz, dxy2);
+                        const f2 rs = rsqrt2(r2);
+                        // s = |F|/r of the pair law plus the on-node charges; the charges' Q/r^3 is
+                        // added before the last factor 1/r (Morse) or 1/r^2 (LJ) the two terms share
+                        f2 s;
+                        if (KIND == SPM_KIND_MORSE) {
+                            // E = E0 e (e-2) = E0 (w - e), F = dp * (-2 K E0) w / r, w = e (e-1), e = exp(K (r-R0))
+                            const f2 r = mul2(r2, rs);
+                            const f2 e = ex2_2(fma2(c0, r, c1));
+                            const f2 w = mul2(e, sub2(e, one));
+                            fe[p] = fma2(c2, sub2(w, e), fe[p]);
+                            const f2 m = mul2(c3, w);
+                            if (ON) {
+                                const f2 Ek = mul2(qon, rs);
+                                fe[p] = add2(fe[p], Ek);
+                                s = mul2(fma2(Ek, rs, m), rs);
+                            } else {
+                                s = mul2(m, rs);
+                            }
+                        } else {
+                            // E = (c12 ir6 - c6) ir6, F = dp * (12 c12 ir6 - 6 c6) ir6 ir2
+                            const f2 ir2 = mul2(rs, rs);
+                            const f2 ir6 = mul2(mul2(ir2, ir2), ir2);
+                            fe[p] = fma2(fma2(c1, ir6, c0), ir6, fe[p]);
+                            if (ON) {
+                                const f2 Ek = mul2(qon, rs);
+                                fe[p] = add2(fe[p], Ek);
+                                s = mul2(fma2(fma2(c3, ir6, c2), ir6, Ek), ir2);
+                            } else {
+                                s = mul2(mul2(fma2(c3, ir6, c2), ir6), ir2);
+                            }
+                        }
+                        fx[p] = fma2(dx, s, fx[p]);
+                        fy[p] = fma2(dy, s, fy[p]);
+                        fz[p] = fma2(dz, s, fz[p]);
+    #pragma unroll
+                        for (int k = 0; k < NOFF; k++) {
+                            // Coulomb at the tip-charge site node + zhat*QZs[k]
+                            const f2 dzk = add2(dz, bc(S.qz[k]));
+                            const f2 rsk = rsqrt2(fma2(dzk, dzk, dxy2));
+                            const f2 Ek = mul2(bc(q[k]), rsk);
+                            fe[p] = add2(fe[p], Ek);
+                            const f2 sk = mul2(mul2(Ek, rsk), rsk);
+                            fx[p] = fma2(dx, sk, fx[p]);
+                            fy[p] = fma2(dy, sk, fy[p]);
+                            fz[p] = fma2(dzk, sk, fz[p]);
+                        }
+                    }
+}
+
+// The staged form of an atom (pr: its parameter row).
+template <int KIND>
+__device__ __forceinline__ float4 atom_params(const float* __restrict__ pr) {
+    if (KIND == SPM_KIND_MORSE) {
+        const float R0 = __ldg(pr + 0), E0 = __ldg(pr + 1), K = __ldg(pr + 2);
+        return make_float4(K * LOG2E, -K * R0 * LOG2E, E0, -2.f * K * E0);
+    }
+    const float c6 = __ldg(pr + 0), c12 = __ldg(pr + 1);
+    return make_float4(-c6, c12, -6.f * c6, 12.f * c12);
+}
+
+// The ZP node pairs of column (xl, yl) (box indices) from layer ic0 on, capped, into the box's storage;
+// layers outside the box are left out.
+template <int ZP, int LAYOUT>
+__device__ __forceinline__ void store_column(float4* __restrict__ out, const StoreBox& B, int xl, int yl, int ic0,
+                                             const f2 (&fx)[ZP], const f2 (&fy)[ZP], const f2 (&fz)[ZP],
+                                             const f2 (&fe)[ZP]) {
+#pragma unroll
+    for (int p = 0; p < ZP; p++) {
+        float x[2], y[2], z[2], e[2];
+        upk(fx[p], x[0], x[1]);
+        upk(fy[p], y[0], y[1]);
+        upk(fz[p], z[0], z[1]);
+        upk(fe[p], e[0], e[1]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int ic = ic0 + 2 * p + h;
+            if (ic >= B.zst_hi) break;
+            if (ic < B.zst_lo) continue;
+            float4 o = make_float4(x[h], y[h], z[h], e[h]);
+            // |E| > 100 cap of the reference builders (AFM.cl:1053-1054)
+            // (the division only where it can scale: 100/|E| < 1 needs |E| > 100; NaN compares false)
+            if (fabsf(o.w) > 100.f) {
+                const float renorm = __fdiv_rn(100.f, fabsf(o.w));
+                if (renorm < 1.f) { o.x *= renorm; o.y *= renorm; o.z *= renorm; o.w *= renorm; }
+            }
+            const int zl = ic - B.zst_lo;
+            const size_t row = ((size_t)zl * B.nys + yl) * B.nxs;
+            const int il = xl > 0 ? xl - 1 : B.nxs - 1;
+            if (LAYOUT == 2) {
+                out[2 * (row + xl)] = o;
+                out[2 * (row + il) + 1] = o;
+            } else if (LAYOUT == 4) {
+                const int nzs = B.zst_hi - B.zst_lo;
+                const size_t rowb = ((size_t)(zl > 0 ? zl - 1 : nzs - 1) * B.nys + yl) * B.nxs;
+                out[4 * (row + xl) + 0] = o;
+                out[4 * (row + il) + 1] = o;
+                out[4 * (rowb + xl) + 2] = o;
+                out[4 * (rowb + il) + 3] = o;
+            } else {
+                out[row + xl] = o;
+            }
+        }
+    }
+}
+
 // One CTA tile: a (blockDim.x x blockDim.y) patch of z-columns (full-grid
 // column ia, row ib), ZB nodes each starting at global layer ic0; nodes
 // outside the box B are not stored, the rest go to out[idx], idx = (zl*nys +
@@ -116,7 +244,6 @@ __device__ __forceinline__ void build_tile(int na, const float4* __restrict__ at
     f2 fx[ZP], fy[ZP], fz[ZP], fe[ZP];
 #pragma unroll
     for (int p = 0; p < ZP; p++) { fx[p] = zero; fy[p] = zero; fz[p] = zero; fe[p] = zero; }
-    const f2 one = bc(1.f);
 
     for (int t0 = 0; t0 < na; t0 += GB_TILE) {
         const int nt = min(GB_TILE, na - t0);
@@ -124,13 +251,7 @@ __device__ __forceinline__ void build_tile(int na, const float4* __restrict__ at
             float4 a = __ldg(atoms + t0 + j);
             const float* pr = params + (size_t)(t0 + j) * pstride;
             s_pos[j] = make_float4(a.x, a.y, a.z, a.w * S.qs_on);
-            if (KIND == SPM_KIND_MORSE) {
-                float R0 = __ldg(pr + 0), E0 = __ldg(pr + 1), K = __ldg(pr + 2);
-                s_prm[j] = make_float4(K * LOG2E, -K * R0 * LOG2E, E0, -2.f * K * E0);
-            } else {
-                float c6 = __ldg(pr + 0), c12 = __ldg(pr + 1);
-                s_prm[j] = make_float4(-c6, c12, -6.f * c6, 12.f * c12);
-            }
+            s_prm[j] = atom_params<KIND>(pr);
 #pragma unroll
             for (int k = 0; k < NOFF; k++) s_q[k][j] = a.w * S.qs[k];
         }
@@ -138,106 +259,16 @@ __device__ __forceinline__ void build_tile(int na, const float4* __restrict__ at
         if (active) {
 #pragma unroll 1
             for (int j = 0; j < nt; j++) {
-                const float4 a = s_pos[j];
-                const float4 c = s_prm[j];
-                const float dxs = px - a.x;
-                const float dys = py - a.y;
-                const float dxy2s = fmaf(dxs, dxs, fmaf(dys, dys, R2SAFE));
-                const f2 dx = bc(dxs), dy = bc(dys), dxy2 = bc(dxy2s), az = bc(a.z);
-                const f2 c0 = bc(c.x), c1 = bc(c.y), c2 = bc(c.z), c3 = bc(c.w);
-                const f2 qon = bc(a.w);
+                float q[NOFF > 0 ? NOFF : 1];
 #pragma unroll
-                for (int p = 0; p < ZP; p++) {
-                    const f2 dz = sub2(pz[p], az);
-                    const f2 r2 = fma2(dz, dz, dxy2);
-                    const f2 rs = rsqrt2(r2);
-                    // s = |F|/r of the pair law plus the on-node charges; the charges' Q/r^3 is
-                    // added before the last factor 1/r (Morse) or 1/r^2 (LJ) the two terms share
-                    f2 s;
-                    if (KIND == SPM_KIND_MORSE) {
-                        // E = E0 e (e-2) = E0 (w - e), F = dp * (-2 K E0) w / r, w = e (e-1), e = exp(K (r-R0))
-                        const f2 r = mul2(r2, rs);
-                        const f2 e = ex2_2(fma2(c0, r, c1));
-                        const f2 w = mul2(e, sub2(e, one));
-                        fe[p] = fma2(c2, sub2(w, e), fe[p]);
-                        const f2 m = mul2(c3, w);
-                        if (ON) {
-                            const f2 Ek = mul2(qon, rs);
-                            fe[p] = add2(fe[p], Ek);
-                            s = mul2(fma2(Ek, rs, m), rs);
-                        } else {
-                            s = mul2(m, rs);
-                        }
-                    } else {
-                        // E = (c12 ir6 - c6) ir6, F = dp * (12 c12 ir6 - 6 c6) ir6 ir2
-                        const f2 ir2 = mul2(rs, rs);
-                        const f2 ir6 = mul2(mul2(ir2, ir2), ir2);
-                        fe[p] = fma2(fma2(c1, ir6, c0), ir6, fe[p]);
-                        if (ON) {
-                            const f2 Ek = mul2(qon, rs);
-                            fe[p] = add2(fe[p], Ek);
-                            s = mul2(fma2(fma2(c3, ir6, c2), ir6, Ek), ir2);
-                        } else {
-                            s = mul2(mul2(fma2(c3, ir6, c2), ir6), ir2);
-                        }
-                    }
-                    fx[p] = fma2(dx, s, fx[p]);
-                    fy[p] = fma2(dy, s, fy[p]);
-                    fz[p] = fma2(dz, s, fz[p]);
-#pragma unroll
-                    for (int k = 0; k < NOFF; k++) {
-                        // Coulomb at the tip-charge site node + zhat*QZs[k]
-                        const f2 dzk = add2(dz, bc(S.qz[k]));
-                        const f2 rsk = rsqrt2(fma2(dzk, dzk, dxy2));
-                        const f2 Ek = mul2(bc(s_q[k][j]), rsk);
-                        fe[p] = add2(fe[p], Ek);
-                        const f2 sk = mul2(mul2(Ek, rsk), rsk);
-                        fx[p] = fma2(dx, sk, fx[p]);
-                        fy[p] = fma2(dy, sk, fy[p]);
-                        fz[p] = fma2(dzk, sk, fz[p]);
-                    }
-                }
+                for (int k = 0; k < NOFF; k++) q[k] = s_q[k][j];
+                add_atom<KIND, ON, NOFF, ZP>(s_pos[j], s_prm[j], q, px, py, pz, S, fx, fy, fz, fe);
             }
         }
         __syncthreads();
     }
     if (!active) return;
-#pragma unroll
-    for (int p = 0; p < ZP; p++) {
-        float x[2], y[2], z[2], e[2];
-        upk(fx[p], x[0], x[1]);
-        upk(fy[p], y[0], y[1]);
-        upk(fz[p], z[0], z[1]);
-        upk(fe[p], e[0], e[1]);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int ic = ic0 + 2 * p + h;
-            if (ic >= B.zst_hi) break;
-            float4 o = make_float4(x[h], y[h], z[h], e[h]);
-            // |E| > 100 cap of the reference builders (AFM.cl:1053-1054)
-            // (the division only where it can scale: 100/|E| < 1 needs |E| > 100; NaN compares false)
-            if (fabsf(o.w) > 100.f) {
-                const float renorm = __fdiv_rn(100.f, fabsf(o.w));
-                if (renorm < 1.f) { o.x *= renorm; o.y *= renorm; o.z *= renorm; o.w *= renorm; }
-            }
-            const int zl = ic - B.zst_lo;
-            const size_t row = ((size_t)zl * B.nys + yl) * B.nxs;
-            const int il = xl > 0 ? xl - 1 : B.nxs - 1;
-            if (LAYOUT == 2) {
-                out[2 * (row + xl)] = o;
-                out[2 * (row + il) + 1] = o;
-            } else if (LAYOUT == 4) {
-                const int nzs = B.zst_hi - B.zst_lo;
-                const size_t rowb = ((size_t)(zl > 0 ? zl - 1 : nzs - 1) * B.nys + yl) * B.nxs;
-                out[4 * (row + xl) + 0] = o;
-                out[4 * (row + il) + 1] = o;
-                out[4 * (rowb + xl) + 2] = o;
-                out[4 * (rowb + il) + 3] = o;
-            } else {
-                out[row + xl] = o;
-            }
-        }
-    }
+    store_column<ZP, LAYOUT>(out, B, xl, yl, ic0, fx, fy, fz, fe);
 }
 
 template <int KIND, bool ON, int NOFF>
@@ -249,9 +280,424 @@ grid_build_kernel(int na, const float4* __restrict__ atoms, const float* __restr
                                       blockIdx.y * GB_TY + threadIdx.y, blockIdx.z * GB_ZB);
 }
 
+// ---- blocks with a far field -------------------------------------------------
+// The grid's nodes in blocks of FB^3 on the lattice of multiples of FB (so a batch
+// slab and the full grid build a node from the same block: the same bits).  An
+// atom FAR_RATIO half-edges or more from a block's centre is far: its four
+// channels are smooth over the block and are summed at the block's FP^3 Chebyshev
+// points (512 instead of 4096 evaluations), then interpolated to the nodes as a
+// tensor product along x, y and z; near atoms are summed at the nodes as in
+// build_tile, on top of the interpolated values.
+//
+// Interpolation error of one atom relative to its largest value in the block
+// (float64, worst direction, at 9 half-edges): 1/r^2 4e-9, r^-7 3e-7, the LJ and
+// Morse laws 1e-7 and 5e-7, falling as the eighth power of the distance -- not
+// above the rounding of the direct float32 sum (rsqrt.approx alone puts 8e-7 on
+// r^-7), and the sums are 2-17 times shorter.  Morse exponentials grow with |K| times the half-edge,
+// not with the distance: an atom with |K| h > FAR_KH is near everywhere.  Measured error of the forces at the
+// nodes a probe reaches (|E| < 0.5 eV), relative to their norm, direct sum -> blocks: 1200 LJ atoms on an
+// ionic slab 1.98e-6 -> 1.89e-6 (energy 2.9e-6 -> 1.7e-6), 57 Morse atoms with offset charges 7.7e-7 -> 7.7e-7.
+//
+// Time, direct sum -> blocks: 1200 atoms on 480 x 480 x 240 nodes 32.0 -> 2.24 ms, 57 Morse atoms with two
+// offset charges on 187 x 203 x 149 442 -> 186 us, 38 atoms on 200^3 211 -> 138 us.  What is left is the near
+// sums (FP32 issue), the far sums and the interpolation in about equal parts.  Below SPM_FAR_MIN_ATOMS most
+// atoms are near most blocks and the interpolation does not pay.
+//
+// Systems of SPM_FAR_GROUP_ATOMS atoms or more take the blocks in groups of 2^3 whose
+// common far atoms (FAR_RATIO group half-edges away) are summed once at the
+// group's Chebyshev points; a block takes that field at its own points by
+// interpolation and adds the atoms that are far for it alone.
+constexpr int FB = SPM_FAR_BLOCK;
+constexpr int FP = 8;
+constexpr int FN = FP * FP * FP;
+constexpr int FAR_CHUNK = 256;       // atoms gathered at a time
+constexpr float FAR_RATIO = 9.f;
+constexpr float FAR_KH = 1.5f;
+constexpr int FAR_FEWEST = 8;        // far atoms that pay for an interpolation (it costs about 4 atoms at the nodes)
+
+// Lagrange weights of the Chebyshev points c at the nodes of a block (L), and of a
+// group's points at the points of its lower and upper blocks (T).
+struct FarTab {
+    float L[FB][FP];
+    float T[2][FP][FP];
+    float c[FP];
+};
+
+FarTab make_far_tab() {
+    FarTab t;
+    double c[FP];
+    for (int k = 0; k < FP; k++) c[k] = cos((2 * k + 1) * 3.14159265358979323846 / (2 * FP));
+    auto weight = [&](double x, int k) {
+        double w = 1.0;
+        for (int j = 0; j < FP; j++)
+            if (j != k) w *= (x - c[j]) / (c[k] - c[j]);
+        return w;
+    };
+    for (int i = 0; i < FB; i++)
+        for (int k = 0; k < FP; k++) t.L[i][k] = (float)weight((2.0 * i - (FB - 1)) / (FB - 1), k);
+    for (int s = 0; s < 2; s++)
+        for (int i = 0; i < FP; i++)
+            for (int k = 0; k < FP; k++)
+                t.T[s][i][k] = (float)weight(((s ? 0.5 : -0.5) * FB + 0.5 * (FB - 1) * c[i]) / (0.5 * (2 * FB - 1)), k);
+    for (int k = 0; k < FP; k++) t.c[k] = (float)c[k];
+    return t;
+}
+
+template <int NOFF>
+struct FarShared {
+    float4 part[4][FN];  // far sums of the four atom subsets; later the interpolation's stages
+    float4 group[FN];    // the group's far field at its points
+    float4 pos[FAR_CHUNK], prm[FAR_CHUNK];
+    float q[NOFF > 0 ? NOFF : 1][FAR_CHUNK];
+    FarTab tab;
+    float2 Lz[FB / 2][FP];  // L of node pairs
+    int warp[8];
+};
+
+// Centre and squared far distance of a cube of nodes with corner (x, y, z) and edge n.  h: half-edge,
+// the largest of the three axes' and of the corner distance over sqrt(3) (skew cells).  Fixed operation
+// order: batch and single builds classify alike.
+struct FarCube {
+    float x, y, z, lim2, h, half;
+};
+
+__device__ __forceinline__ float len3(float x, float y, float z) {
+    return __fsqrt_rn(__fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x))));
+}
+
+__device__ __forceinline__ FarCube far_cube(const GridGeom& G, int x, int y, int z, int n) {
+    FarCube C;
+    C.half = 0.5f * (float)(n - 1);
+    const float cx = (float)x + C.half, cy = (float)y + C.half, cz = (float)z + C.half;
+    C.x = __fmaf_rn(G.dB.x, cy, __fmaf_rn(G.dA.x, cx, G.p0.x));
+    C.y = __fmaf_rn(G.dB.y, cy, __fmaf_rn(G.dA.y, cx, G.p0.y));
+    C.z = __fmaf_rn(G.dC.z, cz, __fmaf_rn(G.dB.z, cy, __fmaf_rn(G.dA.z, cx, G.p0.z)));
+    float e = fmaxf(fmaxf(len3(G.dA.x, G.dA.y, G.dA.z), len3(G.dB.x, G.dB.y, G.dB.z)), fabsf(G.dC.z));
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+        const float sb = s & 1 ? -1.f : 1.f, sc = s & 2 ? -1.f : 1.f;
+        e = fmaxf(e, __fmul_rn(0.57735027f, len3(__fmaf_rn(sb, G.dB.x, G.dA.x), __fmaf_rn(sb, G.dB.y, G.dA.y),
+                                                 __fmaf_rn(sc, G.dC.z, __fmaf_rn(sb, G.dB.z, G.dA.z)))));
+    }
+    C.h = __fmul_rn(e, C.half);
+    C.lim2 = __fmul_rn(__fmul_rn(FAR_RATIO, C.h), __fmul_rn(FAR_RATIO, C.h));
+    return C;
+}
+
+// Far of the cube: the pair law and every off-node charge (seen from the node moved by its offset).
+// A NaN position or parameter is near.
+template <int KIND, int NOFF>
+__device__ __forceinline__ bool is_far(const FarCube& C, const TipSites& S, float4 a, const float* __restrict__ pr) {
+    const float dx = C.x - a.x, dy = C.y - a.y, dz = C.z - a.z;
+    const float dxy2 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
+    bool far = __fmaf_rn(dz, dz, dxy2) >= C.lim2;
+#pragma unroll
+    for (int k = 0; k < NOFF; k++) {
+        const float dk = __fadd_rn(dz, S.qz[k]);
+        far = far && __fmaf_rn(dk, dk, dxy2) >= C.lim2;
+    }
+    if (KIND == SPM_KIND_MORSE) far = far && __fmul_rn(fabsf(__ldg(pr + 2)), C.h) <= FAR_KH;
+    return far;
+}
+
+// Stages the atoms of [c0, c0 + FAR_CHUNK) that satisfy pick(atom, parameter row), in atom order; returns
+// their number to every thread.
+template <int KIND, int NOFF, class Pick>
+__device__ __forceinline__ int gather_atoms(FarShared<NOFF>& M, int tid, int nthr, int c0, int na,
+                                            const float4* __restrict__ atoms, const float* __restrict__ params,
+                                            int pstride, const TipSites& S, const Pick& pick) {
+    const int lane = tid & 31, warp = tid >> 5, nw = nthr >> 5;
+    const int c1 = min(c0 + FAR_CHUNK, na);
+    int n = 0;
+    for (int b = c0; b < c1; b += nthr) {
+        const int j = b + tid;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* pr = params + (size_t)(j < c1 ? j : c0) * pstride;
+        bool take = false;
+        if (j < c1) {
+            a = __ldg(atoms + j);
+            take = pick(a, pr);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, take);
+        __syncthreads();  // the previous round's warp counts and the previous chunk's atoms are read
+        if (lane == 0) M.warp[warp] = __popc(m);
+        __syncthreads();
+        int at = n + __popc(m & ((1u << lane) - 1u));
+        for (int w = 0; w < nw; w++) {
+            const int c = M.warp[w];
+            if (w < warp) at += c;
+            n += c;
+        }
+        if (take) {
+            M.pos[at] = make_float4(a.x, a.y, a.z, a.w * S.qs_on);
+            M.prm[at] = atom_params<KIND>(pr);
+#pragma unroll
+            for (int k = 0; k < NOFF; k++) M.q[k][at] = a.w * S.qs[k];
+        }
+    }
+    __syncthreads();
+    return n;
+}
+
+template <class Pick>
+__device__ __forceinline__ int count_atoms(int tid, int nthr, int na, const float4* __restrict__ atoms,
+                                           const float* __restrict__ params, int pstride, const Pick& pick) {
+    int n = 0;
+    for (int b = 0; b < na; b += nthr) {
+        const int j = b + tid;
+        n += __syncthreads_count(j < na && pick(__ldg(atoms + j), params + (size_t)(j < na ? j : 0) * pstride));
+    }
+    return n;
+}
+
+// Sum of the picked atoms at the cube's Chebyshev points -> part[0] (point (kx, ky, kz) at kz*64 + kx*8 +
+// ky).  Four runs of consecutive atoms go side by side and are added in a fixed order (consecutive: the
+// charges of an ionic crystal listed in lattice order alternate, and every fourth of them would add up to a
+// partial sum far above the total).
+template <int KIND, bool ON, int NOFF, class Pick>
+__device__ __forceinline__ void far_points(FarShared<NOFF>& M, int tid, int nthr, int na,
+                                           const float4* __restrict__ atoms, const float* __restrict__ params,
+                                           int pstride, const GridGeom& G, const TipSites& S, const FarCube& C,
+                                           const Pick& pick) {
+    constexpr int ZP = FP / 2;
+    for (int c0 = 0; c0 < na; c0 += FAR_CHUNK) {
+        const int n = gather_atoms<KIND, NOFF>(M, tid, nthr, c0, na, atoms, params, pstride, S, pick);
+        for (int i = tid; i < 4 * FP * FP; i += nthr) {
+            const int g = i >> 6, col = i & 63;
+            const float ux = C.half * M.tab.c[col >> 3], uy = C.half * M.tab.c[col & 7];
+            const float px = __fmaf_rn(G.dB.x, uy, __fmaf_rn(G.dA.x, ux, C.x));
+            const float py = __fmaf_rn(G.dB.y, uy, __fmaf_rn(G.dA.y, ux, C.y));
+            const float pzb = __fmaf_rn(G.dB.z, uy, __fmaf_rn(G.dA.z, ux, C.z)), hz = __fmul_rn(G.dC.z, C.half);
+            const f2 zero = bc(0.f);
+            f2 pz[ZP], fx[ZP], fy[ZP], fz[ZP], fe[ZP];
+#pragma unroll
+            for (int p = 0; p < ZP; p++) {
+                pz[p] = pk(__fmaf_rn(hz, M.tab.c[2 * p], pzb), __fmaf_rn(hz, M.tab.c[2 * p + 1], pzb));
+                fx[p] = zero; fy[p] = zero; fz[p] = zero; fe[p] = zero;
+            }
+#pragma unroll 1
+            for (int j = g * n / 4; j < (g + 1) * n / 4; j++) {
+                float q[NOFF > 0 ? NOFF : 1];
+#pragma unroll
+                for (int k = 0; k < NOFF; k++) q[k] = M.q[k][j];
+                add_atom<KIND, ON, NOFF, ZP>(M.pos[j], M.prm[j], q, px, py, pz, S, fx, fy, fz, fe);
+            }
+#pragma unroll
+            for (int p = 0; p < ZP; p++) {
+                float x[2], y[2], z[2], e[2];
+                upk(fx[p], x[0], x[1]);
+                upk(fy[p], y[0], y[1]);
+                upk(fz[p], z[0], z[1]);
+                upk(fe[p], e[0], e[1]);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float4& o = M.part[g][(2 * p + h) * 64 + col];
+                    const float4 v = c0 == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : o;
+                    o = make_float4(__fadd_rn(v.x, x[h]), __fadd_rn(v.y, y[h]), __fadd_rn(v.z, z[h]),
+                                    __fadd_rn(v.w, e[h]));
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < FN; i += nthr) {
+        const float4 a = M.part[0][i], b = M.part[1][i], c = M.part[2][i], d = M.part[3][i];
+        M.part[0][i] = make_float4(__fadd_rn(__fadd_rn(a.x, b.x), __fadd_rn(c.x, d.x)),
+                                   __fadd_rn(__fadd_rn(a.y, b.y), __fadd_rn(c.y, d.y)),
+                                   __fadd_rn(__fadd_rn(a.z, b.z), __fadd_rn(c.z, d.z)),
+                                   __fadd_rn(__fadd_rn(a.w, b.w), __fadd_rn(c.w, d.w)));
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ float4 fma4(float w, float4 v, float4 s) {
+    return make_float4(__fmaf_rn(w, v.x, s.x), __fmaf_rn(w, v.y, s.y), __fmaf_rn(w, v.z, s.z), __fmaf_rn(w, v.w, s.w));
+}
+
+// out[i] = sum_k W[index of i along the axis][k] in[i with k there]; stride: of the axis in the point index.
+__device__ __forceinline__ float4 far_axis(const float (*W)[FP], const float4* in, int i, int stride) {
+    const int a = (i / stride) & (FP - 1), base = i - a * stride;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < FP; k++) s = fma4(W[a][k], in[base + k * stride], s);
+    return s;
+}
+
+// Blocks [child0, child1) of one lattice cell (x0, y0, z0: its first node; group: a cell of 2^3 blocks, else
+// one), nodes inside the box B stored as build_tile does.  ZB: nodes along z per thread in the near sums, 8 or 16.
+template <int KIND, bool ON, int NOFF, int ZB, int LAYOUT>
+__device__ __forceinline__ void build_block(FarShared<NOFF>& M, bool group, int child0, int child1, int na, const float4* __restrict__ atoms,
+                                            const float* __restrict__ params, int pstride, float4* __restrict__ out,
+                                            const GridGeom& G, const TipSites& S, const StoreBox& B, int x0, int y0,
+                                            int z0) {
+    constexpr int ZP = ZB / 2;
+    const int nthr = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
+    FarCube C2 = {};
+    bool use2 = false;
+    if (group) {
+        C2 = far_cube(G, x0, y0, z0, 2 * FB);
+        auto far2 = [&](float4 a, const float* pr) { return is_far<KIND, NOFF>(C2, S, a, pr); };
+        use2 = count_atoms(tid, nthr, na, atoms, params, pstride, far2) >= FAR_FEWEST;
+        if (use2) {
+            far_points<KIND, ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C2, far2);
+            for (int i = tid; i < FN; i += nthr) M.group[i] = M.part[0][i];
+        }
+    }
+    for (int child = child0; child < child1; child++) {
+        const int sx = child & 1, sy = (child >> 1) & 1, sz = child >> 2;
+        const int bx = x0 + sx * FB, by = y0 + sy * FB, bz = z0 + sz * FB;
+        if (bx >= B.x_lo + B.nxs || bx + FB <= B.x_lo || by >= B.y_lo + B.nys || by + FB <= B.y_lo || bz >= B.zst_hi ||
+            bz + FB <= B.zst_lo)
+            continue;  // CTA-uniform: no node of this block is stored
+        const FarCube C1 = far_cube(G, bx, by, bz, FB);
+        // an atom of this block alone: not in the group's field
+        auto own = [&](float4 a, const float* pr) { return !(use2 && is_far<KIND, NOFF>(C2, S, a, pr)); };
+        auto far1 = [&](float4 a, const float* pr) { return own(a, pr) && is_far<KIND, NOFF>(C1, S, a, pr); };
+        const int nfar = count_atoms(tid, nthr, na, atoms, params, pstride, far1);
+        const bool use1 = nfar >= FAR_FEWEST, field = use1 || use2;
+        auto near1 = [&](float4 a, const float* pr) {
+            return own(a, pr) && !(use1 && is_far<KIND, NOFF>(C1, S, a, pr));
+        };
+        float4* stage = M.part[1];  // 1024 float4: parts 1 and 2
+        __syncthreads();            // the group's copy, the previous block's stage
+        if (use1) far_points<KIND, ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C1, far1);
+        if (use2) {
+            for (int i = tid; i < FN; i += nthr) M.part[1][i] = far_axis(M.tab.T[sx], M.group, i, 8);
+            __syncthreads();
+            for (int i = tid; i < FN; i += nthr) M.part[2][i] = far_axis(M.tab.T[sy], M.part[1], i, 1);
+            __syncthreads();
+            for (int i = tid; i < FN; i += nthr) {
+                const float4 v = far_axis(M.tab.T[sz], M.part[2], i, 64);
+                const float4 w = use1 ? M.part[0][i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                M.part[0][i] = make_float4(__fadd_rn(v.x, w.x), __fadd_rn(v.y, w.y), __fadd_rn(v.z, w.z),
+                                           __fadd_rn(v.w, w.w));
+            }
+            __syncthreads();
+        }
+        if (field) {  // along x: points (ky, kz) x 16 nodes
+            for (int i = tid; i < FB * FP * FP; i += nthr) {
+                const int x = i & (FB - 1), kk = i >> 4, ky = kk & 7, kz = kk >> 3;
+                float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < FP; k++) s = fma4(M.tab.L[x][k], M.part[0][kz * 64 + k * 8 + ky], s);
+                stage[i] = s;
+            }
+            __syncthreads();
+        }
+        const bool once = na <= FAR_CHUNK;  // the near list holds for every column of this thread
+        int nnear = once ? gather_atoms<KIND, NOFF>(M, tid, nthr, 0, na, atoms, params, pstride, S, near1) : 0;
+        for (int item = tid; item < FB * FB * (FB / ZB); item += nthr) {
+            const int x = item & (FB - 1), y = (item >> 4) & (FB - 1), ic0 = bz + (item >> 8) * ZB;
+            const int ia = bx + x, ib = by + y, xl = ia - B.x_lo, yl = ib - B.y_lo;
+            const bool active = (unsigned)xl < (unsigned)B.nxs && (unsigned)yl < (unsigned)B.nys && ic0 < B.zst_hi &&
+                                ic0 + ZB > B.zst_lo;
+            const f2 zero = bc(0.f);
+            f2 pz[ZP], fx[ZP], fy[ZP], fz[ZP], fe[ZP];
+#pragma unroll
+            for (int p = 0; p < ZP; p++) { fx[p] = zero; fy[p] = zero; fz[p] = zero; fe[p] = zero; }
+            const float px = node_xy(G.p0.x, G.dA.x, G.dB.x, ia, ib);
+            const float py = node_xy(G.p0.y, G.dA.y, G.dB.y, ia, ib);
+            const float pzb = node_xy(G.p0.z, G.dA.z, G.dB.z, ia, ib);
+#pragma unroll
+            for (int p = 0; p < ZP; p++)
+                pz[p] = pk(__fmaf_rn(G.dC.z, (float)(ic0 + 2 * p), pzb), __fmaf_rn(G.dC.z, (float)(ic0 + 2 * p + 1), pzb));
+            if (field && active) {  // along y, then z
+#pragma unroll 1
+                for (int kz = 0; kz < FP; kz++) {
+                    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int k = 0; k < FP; k++) s = fma4(M.tab.L[y][k], stage[(kz * 8 + k) * FB + x], s);
+                    const f2 vx = bc(s.x), vy = bc(s.y), vz = bc(s.z), ve = bc(s.w);
+#pragma unroll
+                    for (int p = 0; p < ZP; p++) {
+                        const float2 l = M.Lz[(item >> 8) * ZP + p][kz];
+                        const f2 w = pk(l.x, l.y);
+                        fx[p] = fma2(w, vx, fx[p]);
+                        fy[p] = fma2(w, vy, fy[p]);
+                        fz[p] = fma2(w, vz, fz[p]);
+                        fe[p] = fma2(w, ve, fe[p]);
+                    }
+                }
+            }
+            for (int c0 = 0; c0 < na; c0 += FAR_CHUNK) {
+                if (!once) nnear = gather_atoms<KIND, NOFF>(M, tid, nthr, c0, na, atoms, params, pstride, S, near1);
+                if (active) {
+#pragma unroll 1
+                    for (int j = 0; j < nnear; j++) {
+                        float q[NOFF > 0 ? NOFF : 1];
+#pragma unroll
+                        for (int k = 0; k < NOFF; k++) q[k] = M.q[k][j];
+                        add_atom<KIND, ON, NOFF, ZP>(M.pos[j], M.prm[j], q, px, py, pz, S, fx, fy, fz, fe);
+                    }
+                }
+            }
+            if (active) store_column<ZP, LAYOUT>(out, B, xl, yl, ic0, fx, fy, fz, fe);
+        }
+    }
+}
+
+template <int NOFF>
+__device__ __forceinline__ void load_far_tab(FarShared<NOFF>& M, const FarTab& tab) {
+    const int nthr = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
+    const float* src = reinterpret_cast<const float*>(&tab);
+    float* dst = reinterpret_cast<float*>(&M.tab);
+    for (int i = tid; i < (int)(sizeof(FarTab) / sizeof(float)); i += nthr) dst[i] = src[i];
+    for (int i = tid; i < FB / 2 * FP; i += nthr)
+        M.Lz[i / FP][i % FP] = make_float2(tab.L[2 * (i / FP)][i % FP], tab.L[2 * (i / FP) + 1][i % FP]);
+    __syncthreads();
+}
+
+// 256 threads, 16 nodes along z each, at 128 registers (two CTAs per SM): 2.24 ms on the 1200-atom 480 x 480
+// x 240 grid (128 threads 2.25, 8 nodes each 2.36; 0.47 ms against 0.71 and 0.44 on 527 atoms, 243 x 138 x
+// 98), 138 us on 38 atoms, 200^3 (128 threads 124).
+constexpr int FAR_THREADS = 256;
+constexpr long long FAR_CTAS = 222;  // CTAs that fill a 148-SM part one and a half times
+
+// A whole grid: one CTA per lattice cell, or per 4, 2 or 1 blocks of a group while the groups alone would
+// leave SMs idle (each CTA then sums the group's field itself: the same values).
+template <int KIND, bool ON, int NOFF>
+__global__ void __launch_bounds__(FAR_THREADS, 2)
+grid_block_kernel(bool group, int split, int na, const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
+                  float4* __restrict__ grid, GridGeom G, TipSites S, const __grid_constant__ FarTab tab) {
+    extern __shared__ __align__(16) unsigned char far_smem[];
+    FarShared<NOFF>& M = *reinterpret_cast<FarShared<NOFF>*>(far_smem);
+    load_far_tab(M, tab);
+    const StoreBox B = {0, G.nx, 0, G.ny, 0, G.nz};
+    const int e = group ? 2 * FB : FB, nb = group ? 8 / split : 1, part = blockIdx.x % split;
+    build_block<KIND, ON, NOFF, GB_ZB, 1>(M, group, part * nb, (part + 1) * nb, na, atoms, params, pstride, grid, G, S,
+                                           B, blockIdx.x / split * e, blockIdx.y * e, blockIdx.z * e);
+}
+
+template <int KIND, bool ON, int NOFF>
+int launch_blocks(int na, const float4* atoms, const float* params, int pstride, float4* out, const GridGeom& G,
+                  const TipSites& S, cudaStream_t st) {
+    static const FarTab tab = make_far_tab();
+    const auto kern = grid_block_kernel<KIND, ON, NOFF>;
+    const size_t smem = sizeof(FarShared<NOFF>);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return set_error(SPM_ERR_CUDA, "spm_grid_build: cannot enable %zu B of shared memory", smem);
+    const bool group = na >= SPM_FAR_GROUP_ATOMS;
+    const int e = group ? 2 * FB : FB;
+    const long long cells = (long long)((G.nx + e - 1) / e) * ((G.ny + e - 1) / e) * ((G.nz + e - 1) / e);
+    int split = 1;
+    while (group && split < 8 && cells * split < FAR_CTAS) split *= 2;
+    kern<<<dim3((G.nx + e - 1) / e * split, (G.ny + e - 1) / e, (G.nz + e - 1) / e), FAR_THREADS, smem, st>>>(
+        group, split, na, atoms, params, pstride, out, G, S, tab);
+    return check_launch("spm_grid_build");
+}
+
 template <int KIND, bool ON>
 int launch_noff(int noff, dim3 grd, dim3 block, cudaStream_t st, int na, const float4* atoms, const float* params,
                 int pstride, float4* out, const GridGeom& G, const TipSites& S) {
+    if (na >= SPM_FAR_MIN_ATOMS) {
+        switch (noff) {
+            case 0: return launch_blocks<KIND, ON, 0>(na, atoms, params, pstride, out, G, S, st);
+            case 1: return launch_blocks<KIND, ON, 1>(na, atoms, params, pstride, out, G, S, st);
+            case 2: return launch_blocks<KIND, ON, 2>(na, atoms, params, pstride, out, G, S, st);
+            case 3: return launch_blocks<KIND, ON, 3>(na, atoms, params, pstride, out, G, S, st);
+            default: return launch_blocks<KIND, ON, 4>(na, atoms, params, pstride, out, G, S, st);
+        }
+    }
     switch (noff) {
         case 0: grid_build_kernel<KIND, ON, 0><<<grd, block, 0, st>>>(na, atoms, params, pstride, out, G, S); break;
         case 1: grid_build_kernel<KIND, ON, 1><<<grd, block, 0, st>>>(na, atoms, params, pstride, out, G, S); break;
@@ -300,6 +746,7 @@ batch_grid_build_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
                         const float* __restrict__ params, int pstride, float4* __restrict__ grid, TipSites S) {
     const long long tile = blockIdx.x;
     const spm_batch_mol* D = mols + SPM_MOL_BY(tile_off, mols, n_mol, tile);
+    if (D->n_atoms >= SPM_FAR_MIN_ATOMS) return;  // built by batch_grid_block_kernel
     const int ty = blockDim.y;
     const int z_lo = D->z_lo, nzs = D->nz_slab;
     const StoreBox B = {D->x_lo, D->nx_slab, D->y_lo, D->ny_slab, z_lo, z_lo + nzs};
@@ -324,6 +771,40 @@ batch_grid_build_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
                                            z_lo + (int)bz * ZB);
 }
 
+// The molecules of SPM_FAR_MIN_ATOMS atoms or more: persistent CTAs over their lattice cells (block_off:
+// prefix of cells over the batch), each cell's nodes inside the molecule's box as grid_block_kernel builds
+// them.
+template <int KIND, bool ON, int NOFF, int LAYOUT>
+__global__ void __launch_bounds__(256, 2)
+batch_grid_block_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const float4* __restrict__ atoms,
+                        const float* __restrict__ params, int pstride, float4* __restrict__ grid, TipSites S,
+                        const __grid_constant__ FarTab tab) {
+    extern __shared__ __align__(16) unsigned char far_smem[];
+    FarShared<NOFF>& M = *reinterpret_cast<FarShared<NOFF>*>(far_smem);
+    load_far_tab(M, tab);
+    const long long total = (long long)mols[n_mol - 1].block_off + far_cells(mols[n_mol - 1]);
+    for (long long c = blockIdx.x; c < total; c += gridDim.x) {
+        const spm_batch_mol* D = mols + SPM_MOL_BY(block_off, mols, n_mol, c);
+        const bool group = D->n_atoms >= SPM_FAR_GROUP_ATOMS;
+        const int e = group ? 2 * FB : FB;
+        const StoreBox B = {D->x_lo, D->nx_slab, D->y_lo, D->ny_slab, D->z_lo, D->z_lo + D->nz_slab};
+        const int cx0 = B.x_lo / e, cy0 = B.y_lo / e, cz0 = B.zst_lo / e;
+        const int ncx = (B.x_lo + B.nxs - 1) / e - cx0 + 1, ncy = (B.y_lo + B.nys - 1) / e - cy0 + 1;
+        const int lc = (int)(c - D->block_off);
+        GridGeom G;
+        G.nx = D->nx; G.ny = D->ny; G.nz = D->nz;
+        G.p0 = ld4f(D->p0);
+        G.dA = ld4f(D->dA);
+        G.dB = ld4f(D->dB);
+        G.dC = ld4f(D->dC);
+        const int ao = D->atom_off;
+        build_block<KIND, ON, NOFF, 8, LAYOUT>(M, group, 0, group ? 8 : 1, D->n_atoms, atoms + ao, params + (size_t)ao * pstride, pstride,
+                                                grid + LAYOUT * D->grid_off, G, S, B, (cx0 + lc % ncx) * e,
+                                                (cy0 + lc / ncx % ncy) * e, (cz0 + lc / ncx / ncy) * e);
+        __syncthreads();  // the next cell reuses the shared memory
+    }
+}
+
 struct BatchLaunch {
     unsigned blocks;
     dim3 block;
@@ -337,37 +818,46 @@ struct BatchLaunch {
     int layout;  // float4 per node: 2 (x-pairs) or 4 (xz-quads)
 };
 
-template <int KIND, bool ON, int NOFF, int LAYOUT>
-void launch_batch_zl(int zb, const BatchLaunch& L, const TipSites& S) {
-    if (zb == 16)
-        batch_grid_build_kernel<KIND, ON, NOFF, 16, LAYOUT><<<L.blocks, L.block, 0, L.st>>>(
-            L.n_mol, L.mols, L.atoms, L.params, L.pstride, L.grid, S);
-    else
-        batch_grid_build_kernel<KIND, ON, NOFF, 8, LAYOUT><<<L.blocks, L.block, 0, L.st>>>(
-            L.n_mol, L.mols, L.atoms, L.params, L.pstride, L.grid, S);
+template <int KIND, bool ON, int NOFF, int ZB, int LAYOUT>
+int launch_batch_z(const BatchLaunch& L, const TipSites& S) {
+    batch_grid_build_kernel<KIND, ON, NOFF, ZB, LAYOUT><<<L.blocks, L.block, 0, L.st>>>(
+        L.n_mol, L.mols, L.atoms, L.params, L.pstride, L.grid, S);
+    static const FarTab tab = make_far_tab();
+    const auto kern = batch_grid_block_kernel<KIND, ON, NOFF, LAYOUT>;
+    const size_t smem = sizeof(FarShared<NOFF>);
+    const int threads = (int)(L.block.x * L.block.y);
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess)
+        return set_error(SPM_ERR_CUDA, "spm_batch_grid_build: cannot prepare the block kernel");
+    kern<<<sms * (per_sm > 0 ? per_sm : 1), L.block, smem, L.st>>>(L.n_mol, L.mols, L.atoms, L.params, L.pstride,
+                                                                   L.grid, S, tab);
+    return check_launch("spm_batch_grid_build");
 }
 
 template <int KIND, bool ON, int NOFF>
-void launch_batch_zb(int zb, const BatchLaunch& L, const TipSites& S) {
-    if (L.layout == 4) launch_batch_zl<KIND, ON, NOFF, 4>(zb, L, S);
-    else launch_batch_zl<KIND, ON, NOFF, 2>(zb, L, S);
+int launch_batch_zb(int zb, const BatchLaunch& L, const TipSites& S) {
+    if (L.layout == 4)
+        return zb == 16 ? launch_batch_z<KIND, ON, NOFF, 16, 4>(L, S) : launch_batch_z<KIND, ON, NOFF, 8, 4>(L, S);
+    return zb == 16 ? launch_batch_z<KIND, ON, NOFF, 16, 2>(L, S) : launch_batch_z<KIND, ON, NOFF, 8, 2>(L, S);
 }
 
 template <int KIND, bool ON>
-void launch_batch_noff(int noff, int zb, const BatchLaunch& L, const TipSites& S) {
+int launch_batch_noff(int noff, int zb, const BatchLaunch& L, const TipSites& S) {
     switch (noff) {
-        case 0: launch_batch_zb<KIND, ON, 0>(zb, L, S); break;
-        case 1: launch_batch_zb<KIND, ON, 1>(zb, L, S); break;
-        case 2: launch_batch_zb<KIND, ON, 2>(zb, L, S); break;
-        case 3: launch_batch_zb<KIND, ON, 3>(zb, L, S); break;
-        default: launch_batch_zb<KIND, ON, 4>(zb, L, S); break;
+        case 0: return launch_batch_zb<KIND, ON, 0>(zb, L, S);
+        case 1: return launch_batch_zb<KIND, ON, 1>(zb, L, S);
+        case 2: return launch_batch_zb<KIND, ON, 2>(zb, L, S);
+        case 3: return launch_batch_zb<KIND, ON, 3>(zb, L, S);
+        default: return launch_batch_zb<KIND, ON, 4>(zb, L, S);
     }
 }
 
 template <int KIND>
-void launch_batch_kind(bool on, int noff, int zb, const BatchLaunch& L, const TipSites& S) {
-    if (on) launch_batch_noff<KIND, true>(noff, zb, L, S);
-    else launch_batch_noff<KIND, false>(noff, zb, L, S);
+int launch_batch_kind(bool on, int noff, int zb, const BatchLaunch& L, const TipSites& S) {
+    return on ? launch_batch_noff<KIND, true>(noff, zb, L, S) : launch_batch_noff<KIND, false>(noff, zb, L, S);
 }
 
 }  // namespace
@@ -405,9 +895,8 @@ extern "C" int spm_batch_grid_build(int kind, int n_mol, const spm_batch_mol* mo
     L.pstride = (kind == SPM_KIND_MORSE) ? 4 : 2;
     L.grid = reinterpret_cast<float4*>(grid);
     L.layout = shape->grid_layout ? 4 : 2;
-    if (kind == SPM_KIND_MORSE) launch_batch_kind<SPM_KIND_MORSE>(on, noff, shape->gb_zb, L, S);
-    else launch_batch_kind<SPM_KIND_LJ>(on, noff, shape->gb_zb, L, S);
-    return check_launch("spm_batch_grid_build");
+    if (kind == SPM_KIND_MORSE) return launch_batch_kind<SPM_KIND_MORSE>(on, noff, shape->gb_zb, L, S);
+    return launch_batch_kind<SPM_KIND_LJ>(on, noff, shape->gb_zb, L, S);
 }
 
 extern "C" int spm_grid_build(int kind, int n_atoms, const float* atoms, const float* params, float* grid,

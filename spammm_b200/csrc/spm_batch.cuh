@@ -11,6 +11,22 @@
 
 namespace spm {
 
+// Atoms from which a force grid is built in blocks with a far field, and in groups of 2^3 blocks
+// (grid_build.cu); the same for a batch's molecules and a single grid.
+constexpr int SPM_FAR_MIN_ATOMS = 32;
+constexpr int SPM_FAR_GROUP_ATOMS = 256;
+constexpr int SPM_FAR_BLOCK = 16;  // nodes per block edge
+
+// Lattice cells (blocks or groups of blocks) that a molecule's box of stored nodes meets; 0 below
+// SPM_FAR_MIN_ATOMS.
+__host__ __device__ inline long long far_cells(const spm_batch_mol& D) {
+    if (D.n_atoms < SPM_FAR_MIN_ATOMS) return 0;
+    const int e = D.n_atoms >= SPM_FAR_GROUP_ATOMS ? 2 * SPM_FAR_BLOCK : SPM_FAR_BLOCK;
+    return ((long long)(D.x_lo + D.nx_slab - 1) / e - D.x_lo / e + 1) *
+           ((long long)(D.y_lo + D.ny_slab - 1) / e - D.y_lo / e + 1) *
+           ((long long)(D.z_lo + D.nz_slab - 1) / e - D.z_lo / e + 1);
+}
+
 template <typename T, T spm_batch_mol::*F>
 __device__ __forceinline__ int find_mol(const spm_batch_mol* __restrict__ mols, int n_mol, long long x) {
     int lo = 0, hi = n_mol - 1;  // mols[0].*F == 0 <= x
