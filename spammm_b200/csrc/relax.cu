@@ -34,6 +34,7 @@ namespace spm {
 namespace {
 
 constexpr int RX_THREADS = 128;
+constexpr int WARPS_PER_SCHEDULER = 1;
 
 // Pixel of this thread under the static schedule (one pixel per lane), or -1.
 __device__ __forceinline__ int pixel_of_thread(int n_scan, int raster_ny) {
@@ -118,7 +119,7 @@ __device__ __forceinline__ PolishSpring pp_spring(const PPFrame& F) {
 // tip frame) z-step: q and fe in, the polished position and the sample there out.
 template <int MODE, typename IDX>
 __device__ __forceinline__ void polish_state(const GridView& G, V3 a, V3 b, V3 c, float4 kk, float4 d0, float surf,
-                                             V3 tip, V3& q, float4& fe) {
+                                             V3 tip, V3& q, float4& fe, TexelCache& cache) {
     PolishSpring S;
     S.a = a; S.b = b; S.c = c;
     S.kk = kk; S.d0 = d0;
@@ -126,7 +127,7 @@ __device__ __forceinline__ void polish_state(const GridView& G, V3 a, V3 b, V3 c
     S.frame = MODE != 0;
     float T[3][3];
     polish_coefs(G, T);
-    newton_polish(FullCellFetch<IDX>{G}, T, S, tip, q, fe);
+    newton_polish(FullCellFetchCached<IDX>{G, cache}, T, S, tip, q, fe);
 }
 
 // One SPM_RELAX_PP iteration (the direct path's bookkeeping: the convergence
@@ -162,12 +163,12 @@ __device__ __forceinline__ bool pp_iter(const GridView& G, const PPFrame& F, V3 
 // polished position, which PP reports.
 template <typename IDX, bool POLISH>
 __device__ __forceinline__ void pp_emit(const GridView& G, const PPFrame& F, V3 tip, V3 pos, float4 fe, int it,
-                                        bool conv, float4* fe_out, float4* pp_out) {
+                                        bool conv, float4* fe_out, float4* pp_out, TexelCache& cache) {
     if (!conv) fe = interp_fe<IDX>(G, pos);  // the position moved after the last sample
     if constexpr (POLISH) {
         float T[3][3];
         polish_coefs(G, T);
-        newton_polish(FullCellFetch<IDX>{G}, T, pp_spring(F), tip, pos, fe);
+        newton_polish(FullCellFetchCached<IDX>{G, cache}, T, pp_spring(F), tip, pos, fe);
     }
     const V3 r = rotmat(mk3(fe.x, fe.y, fe.z), F.a, F.b, F.c);
     *fe_out = make_float4(r.x, r.y, r.z, fe.w);
@@ -241,7 +242,7 @@ relax_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_pa
             bool conv;
             if (pp_iter<IDX, CACHE>(G, F, tip, pos, v, I, fe, it, total_it, conv, T, fnx, fny, fnz)) {
                 const size_t o = (size_t)k * nzs + iz;
-                pp_emit<IDX, POLISH>(G, F, tip, pos, fe, it, conv, FEs + o, disps + o);
+                pp_emit<IDX, POLISH>(G, F, tip, pos, fe, it, conv, FEs + o, disps + o, T);
                 tip = add3(tip, dTip);
                 pos = add3(pos, dTip);
                 v = mk3(0.f, 0.f, 0.f);
@@ -313,13 +314,13 @@ relax_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_pa
             V3 q = pos;  // the output position (polished or not); the next z-step starts from pos
             if (MODE == 0) {
                 float4 fo = fe;
-                if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, fo);
+                if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, fo, T);
                 FEs[o] = fo;
                 const V3 ref = mk3(tip.x + d0.x, tip.y + d0.y, tip.z + d0.z);
                 disps[o] = make_float4(q.x - ref.x, q.y - ref.y, q.z - ref.z, 0.f);
             } else {
                 float4 g = interp_fe<IDX>(G, pos);
-                if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, g);
+                if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, g, T);
                 const V3 r = rotmat(mk3(g.x, g.y, g.z), a, b, c);
                 FEs[o] = make_float4(r.x, r.y, r.z, g.w);
             }
@@ -335,6 +336,11 @@ relax_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_pa
             }
         }
     }
+}
+
+// Raster rows (iy) of a tile of `lanes` pixels: 32 = 4 x 8, 16 = 4 x 4, 8 = 2 x 4, 4 = 2 x 2, 2 = 1 x 2, 1.
+__host__ __device__ __forceinline__ unsigned tile_rows(unsigned lanes) {
+    return lanes == 32 ? 8u : lanes >= 8 ? 4u : lanes >= 2 ? 2u : 1u;
 }
 
 // The dissipation integral fused into the paired relaxation (spm_relax_pair_dissipation): the
@@ -359,14 +365,21 @@ struct DissArgs {
 // where every lane is at its own pixel, z-step and phase and the warp runs the
 // sampling miss path and the per-z-step epilogue for a few lanes at a time
 // (49% of the lanes active per instruction on the 480x480-pixel scan), the
-// lanes of a warp run that code together: 3.81 -> 2.30 ms on that scan.  The
+// lanes of a warp run that code together: 3.81 -> 2.30 ms on that scan.
+//
+// lanes: pixels of a tile, 32 or, for scans that leave the schedulers short of
+// warps, a smaller power of two (tile_lanes; the other lanes idle).  A step
+// costs a warp the cell loads of any of its lanes, and a z-step the steps of its
+// slowest lane: fewer pixels per warp shorten both.  The polish reads its cells
+// through the texel cache of the FIRE loop (480 x 480 x 60 polished 3.03 -> 2.71
+// ms).  The
 // per-lane sequence is relax_kernel's (the same iteration, emit and texel
 // cache), so the results are the same bits.
 template <int MODE, typename IDX, bool POLISH, bool DISS = false>
 __global__ void __launch_bounds__(RX_THREADS)
 relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_params P,
                   float4* __restrict__ FEs, float4* __restrict__ disps, int* __restrict__ iter_count,
-                  unsigned* __restrict__ counter, DissArgs DA = DissArgs{}) {
+                  unsigned* __restrict__ counter, int lanes, DissArgs DA = DissArgs{}) {
     static_assert(!DISS || MODE == 0, "the fused dissipation is for relaxStrokes pairs");
     static_assert(MODE >= 0 && MODE <= 2, "relaxStrokes2D keeps the flattened loop");
     const unsigned lane = threadIdx.x & 31u;
@@ -391,22 +404,23 @@ relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_sc
     const int half = (MODE == 0 && (P.flags & SPM_FLAG_PAIRED)) ? n_scan / 2 : n_scan;
     const int ny = P.raster_ny;
     const int nxr = ny > 0 ? n_scan / ny : 0;
-    const unsigned nty = ny > 0 ? (unsigned)(ny + 7) / 8 : 0u;
-    const unsigned nslots = ny > 0 ? ((unsigned)(nxr + 3) / 4) * nty * 32u : ((unsigned)n_scan + 31u) / 32u * 32u;
+    const unsigned nt = (unsigned)lanes, ty = tile_rows(nt), tx = nt / ty;
+    const unsigned nty = ny > 0 ? ((unsigned)ny + ty - 1u) / ty : 0u;
+    const unsigned ntiles = ny > 0 ? ((unsigned)nxr + tx - 1u) / tx * nty : ((unsigned)n_scan + nt - 1u) / nt;
     while (true) {
-        unsigned base = 0;
-        if (lane == 0) base = atomicAdd(counter, 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= nslots) return;  // warp-uniform
-        const unsigned t = base + lane;
+        unsigned tile = 0;
+        if (lane == 0) tile = atomicAdd(counter, 1u);
+        tile = __shfl_sync(0xffffffffu, tile, 0);
+        if (tile >= ntiles) return;  // warp-uniform
         int k = -1;
-        if (ny > 0) {
-            const unsigned tile = t >> 5, r = t & 31u;
-            const int ix = (int)((tile / nty) * 4 + (r >> 3));
-            const int iy = (int)((tile % nty) * 8 + (r & 7));
-            if (ix < nxr && iy < ny) k = ix * ny + iy;
-        } else if (t < (unsigned)n_scan) {
-            k = (int)t;
+        if (lane < nt) {
+            if (ny > 0) {
+                const int ix = (int)((tile / nty) * tx + lane / ty);
+                const int iy = (int)((tile % nty) * ty + lane % ty);
+                if (ix < nxr && iy < ny) k = ix * ny + iy;
+            } else if (tile * nt + lane < (unsigned)n_scan) {
+                k = (int)(tile * nt + lane);
+            }
         }
         const unsigned members = __ballot_sync(0xffffffffu, k >= 0);
         if (k >= 0) {
@@ -432,7 +446,7 @@ relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_sc
                     while (!pp_iter<IDX, true>(G, F, tip, pos, v, I, fe, it, total_it, conv, T, fnx, fny, fnz)) {
                     }
                     const size_t o = (size_t)k * nzs + iz;
-                    pp_emit<IDX, POLISH>(G, F, tip, pos, fe, it, conv, FEs + o, disps + o);
+                    pp_emit<IDX, POLISH>(G, F, tip, pos, fe, it, conv, FEs + o, disps + o, T);
                 } else {
                     bool done = max_iter <= 0;
                     while (!done) {
@@ -458,13 +472,13 @@ relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_sc
                     V3 q = pos;  // the output position; the next z-step starts from pos
                     if (MODE == 0) {
                         float4 fo = fe;
-                        if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, fo);
+                        if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, fo, T);
                         FEs[o] = fo;
                         const V3 ref = mk3(tip.x + d0.x, tip.y + d0.y, tip.z + d0.z);
                         disps[o] = make_float4(q.x - ref.x, q.y - ref.y, q.z - ref.z, 0.f);
                     } else {
                         float4 g = interp_fe<IDX>(G, pos);
-                        if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, g);
+                        if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, g, T);
                         const V3 r = rotmat(mk3(g.x, g.y, g.z), a, b, c);
                         FEs[o] = make_float4(r.x, r.y, r.z, g.w);
                     }
@@ -557,19 +571,43 @@ spm_scan_params normalized(const spm_scan_params* p, int n_scan) {
     return P;
 }
 
-// Persistent grid size of a counter-scheduled relaxation kernel: as many CTAs as are co-resident
-// (the counter balances the rest).
+// Persistent grid size of a counter-scheduled relaxation kernel: as many CTAs of `threads` as are
+// co-resident, at most one per `warps` work items (the counter balances the rest).
 template <class K>
-int persistent_blocks(K kern, int n_scan, int& blocks) {
+int persistent_blocks(K kern, long long warps, int threads, int& blocks) {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RX_THREADS, 0) != cudaSuccess)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0) != cudaSuccess)
         return set_error(SPM_ERR_CUDA, "relax: cannot query the device occupancy");
-    const int cap = sms * (per_sm > 0 ? per_sm : 1);
-    const int need = (n_scan + RX_THREADS - 1) / RX_THREADS;
-    blocks = need < cap ? need : cap;
+    const long long cap = (long long)sms * (per_sm > 0 ? per_sm : 1), need = (warps * 32 + threads - 1) / threads;
+    blocks = (int)(need < cap ? need : cap);
     return SPM_OK;
+}
+
+// Pixels per warp of a scan of n pixels: 32, halved while that gives fewer than WARPS_PER_SCHEDULER warps
+// for each of the GPU's schedulers.  100 x 100 pixels x 40 z-steps: 32 pixels per warp 893 us, at least one
+// warp per scheduler (16 pixels) 658, two (8) 718, four (4) 980; 24 x 24 x 20: 358 -> 311.
+int tile_lanes(long long n, int& lanes) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return set_error(SPM_ERR_CUDA, "relax: cannot query the device");
+    lanes = 32;
+    while (lanes > 1 && (n + lanes - 1) / lanes < (long long)WARPS_PER_SCHEDULER * 4 * sms) lanes /= 2;
+    return SPM_OK;
+}
+
+// Tile width, CTA size (single warps while tiles are small: they spread evenly over the SMs) and CTAs of
+// relax_tile_kernel.
+template <class K>
+int tile_launch(K kern, int n_scan, int raster_ny, int& lanes, int& threads, int& blocks) {
+    if (int rc = tile_lanes(n_scan, lanes)) return rc;
+    threads = lanes < 32 ? 32 : RX_THREADS;
+    const long long ty = tile_rows((unsigned)lanes), tx = lanes / ty;
+    const long long tiles = raster_ny > 0 ? (n_scan / raster_ny + tx - 1) / tx * ((raster_ny + ty - 1) / ty)
+                                          : (n_scan + lanes - 1) / lanes;
+    return persistent_blocks(kern, tiles, threads, blocks);
 }
 
 template <int MODE, typename IDX, bool POLISH>
@@ -580,14 +618,14 @@ int launch_relax(const GridView& G, const float4* pts, int n_scan, const spm_sca
             return set_error(SPM_ERR_CUDA, "relax: cannot reset the pixel counter");
         if constexpr (MODE <= 2) {  // z-synchronised tiles from the counter
             auto kern = relax_tile_kernel<MODE, IDX, POLISH, false>;
-            int blocks = 0;
-            if (int rc = persistent_blocks(kern, n_scan, blocks)) return rc;
-            kern<<<blocks, RX_THREADS, 0, st>>>(G, pts, n_scan, P, FEs, disps, iter_count, counter, DissArgs{});
+            int lanes = 0, threads = 0, blocks = 0;
+            if (int rc = tile_launch(kern, n_scan, P.raster_ny, lanes, threads, blocks)) return rc;
+            kern<<<blocks, threads, 0, st>>>(G, pts, n_scan, P, FEs, disps, iter_count, counter, lanes, DissArgs{});
             return check_launch("relax");
         }
         auto kern = relax_kernel<MODE, IDX, (MODE <= 2), POLISH>;
         int blocks = 0;
-        if (int rc = persistent_blocks(kern, n_scan, blocks)) return rc;
+        if (int rc = persistent_blocks(kern, (n_scan + 31LL) / 32, RX_THREADS, blocks)) return rc;
         kern<<<blocks, RX_THREADS, 0, st>>>(G, pts, n_scan, P, FEs, disps, iter_count, counter);
         return check_launch("relax");
     }
@@ -692,7 +730,7 @@ __global__ void __launch_bounds__(MINB == 5 ? 128 : 256, MINB)
 batch_relax_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, unsigned n_slots, int th_log2,
                    const float* __restrict__ grid, const float4* __restrict__ pts, spm_scan_params P,
                    float4* __restrict__ FEs, float4* __restrict__ PPs, int* __restrict__ iter_count,
-                   unsigned* __restrict__ counter) {
+                   unsigned* __restrict__ counter, int) {
     const float dz = P.tipC[3];
     int m = 0, k = 0;
     bool have = next_batch_pixel(counter, n_slots, mols, n_mol, th_log2, m, k);
@@ -1046,24 +1084,27 @@ static_assert(sizeof(TailEntry) == 48, "tail entries are 48 bytes");
 // draw counter, then the tail list from byte 16.
 constexpr long long TAIL_OFF = 16;
 
+// The prefix pass at MINB = 5 takes four 128-thread CTAs per SM (128 registers): it keeps the texel cache
+// and the Newton step's two Jacobians, and spilled 136 bytes per thread at five (64-molecule fitting step
+// 23.9 -> 23.1 ms).
 template <int MINB, bool CACHE, int LAYOUT>
-__global__ void __launch_bounds__(MINB == 5 ? 128 : 256, MINB)
+__global__ void __launch_bounds__(MINB == 5 ? 128 : 256, MINB == 5 ? 4 : MINB)
 batch_relax_prefix_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, unsigned n_slots, int th_log2,
                           const float* __restrict__ grid, const float4* __restrict__ pts, spm_scan_params P,
                           float4* __restrict__ FEs, float4* __restrict__ PPs, int* __restrict__ iter_count,
-                          unsigned* __restrict__ ws) {
+                          unsigned* __restrict__ ws, int lanes) {
     const float dz = P.tipC[3];
     const unsigned lane = threadIdx.x & 31u;
     TailEntry* tail = reinterpret_cast<TailEntry*>(reinterpret_cast<char*>(ws) + TAIL_OFF);
     while (true) {
         unsigned base = 0;
-        if (lane == 0) base = atomicAdd(ws, 32u);
+        if (lane == 0) base = atomicAdd(ws, (unsigned)lanes);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= n_slots) return;  // warp-uniform
         const int m = SPM_MOL_BY(slot_off, mols, n_mol, (long long)base);
         const spm_batch_mol* D = mols + m;
         int k;
-        const bool valid = slot_pixel(D, base + lane - (unsigned)D->slot_off, th_log2, k);
+        const bool valid = slot_pixel(D, base + lane - (unsigned)D->slot_off, th_log2, k) && lane < (unsigned)lanes;
         const unsigned members = __ballot_sync(0xffffffffu, valid);
         if (valid) {
             const AxisView G = axis_view<LAYOUT>(D, grid);
@@ -1158,18 +1199,18 @@ __global__ void __launch_bounds__(MINB == 5 ? 128 : 256, MINB)
 batch_relax_sync_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, unsigned n_slots, int th_log2,
                         const float* __restrict__ grid, const float4* __restrict__ pts, spm_scan_params P,
                         float4* __restrict__ FEs, float4* __restrict__ PPs, int* __restrict__ iter_count,
-                        unsigned* __restrict__ counter) {
+                        unsigned* __restrict__ counter, int lanes) {
     const float dz = P.tipC[3];
     const unsigned lane = threadIdx.x & 31u;
     while (true) {
         unsigned base = 0;
-        if (lane == 0) base = atomicAdd(counter, 32u);
+        if (lane == 0) base = atomicAdd(counter, (unsigned)lanes);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= n_slots) return;  // warp-uniform
         const int m = SPM_MOL_BY(slot_off, mols, n_mol, (long long)base);
         const spm_batch_mol* D = mols + m;
         int k;
-        const bool valid = slot_pixel(D, base + lane - (unsigned)D->slot_off, th_log2, k);
+        const bool valid = slot_pixel(D, base + lane - (unsigned)D->slot_off, th_log2, k) && lane < (unsigned)lanes;
         const unsigned members = __ballot_sync(0xffffffffu, valid);
         if (valid) relax_tile_stroke<CACHE, LAYOUT, POLISH>(D, grid, pts, P, FEs, PPs, iter_count, k, dz, members);
         __syncwarp();  // the whole warp draws the next tile
@@ -1379,7 +1420,7 @@ __global__ void __launch_bounds__(STAGE_WARPS * 32, 4)
 batch_relax_staged_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, unsigned n_slots, int th_log2,
                           const float* __restrict__ grid, const float4* __restrict__ pts, spm_scan_params P,
                           float4* __restrict__ FEs, float4* __restrict__ PPs, int* __restrict__ iter_count,
-                          unsigned* __restrict__ counter) {
+                          unsigned* __restrict__ counter, int) {
     __shared__ __align__(128) ulonglong2 s_box[STAGE_WARPS][2 * STAGE_CAP];
     __shared__ __align__(8) unsigned long long s_bar[STAGE_WARPS];
     const float dz = P.tipC[3];
@@ -1514,7 +1555,12 @@ extern "C" int spm_batch_relax(int n_mol, const spm_batch_mol* mols, long long n
         return set_error(SPM_ERR_CUDA, "spm_batch_relax: cannot query the device occupancy");
     if (per_sm < 1) per_sm = 1;
     if (shape->rx_ctas_per_sm > 0 && shape->rx_ctas_per_sm < per_sm) per_sm = shape->rx_ctas_per_sm;
-    const long long need = (n_slots + thr - 1) / thr;
+    // fewer slots per draw while the batch leaves the schedulers short of warps (not the lane-by-lane schedule
+    // and the staged variant)
+    int lanes = 32;
+    if (sync == 1 && shape->rx_regs != 5)
+        if (int rc = tile_lanes(n_slots, lanes)) return rc;
+    const long long need = (n_slots * (32 / lanes) + thr - 1) / thr;
     const long long cap = (long long)sms * per_sm;
     const unsigned blocks = (unsigned)(need < cap ? need : cap);
     cudaStream_t st = as_stream(stream);
@@ -1526,7 +1572,7 @@ extern "C" int spm_batch_relax(int n_mol, const spm_batch_mol* mols, long long n
     kern<<<blocks, thr, 0, st>>>(n_mol, mols, (unsigned)n_slots, th_log2, grid,
                                                reinterpret_cast<const float4*>(points), *p,
                                                reinterpret_cast<float4*>(FEs), reinterpret_cast<float4*>(PPs),
-                                               iter_count, ctr);
+                                               iter_count, ctr, lanes);
     if (two_pass) {
         int rc = check_launch("spm_batch_relax (prefix pass)");
         if (rc) return rc;
@@ -1650,12 +1696,12 @@ extern "C" int spm_relax_pair_dissipation(const float* grid, int nx, int ny, int
     const bool pol = (P.flags & SPM_FLAG_POLISH) != 0;
     auto kern = big ? (pol ? relax_tile_kernel<0, size_t, true, true> : relax_tile_kernel<0, size_t, false, true>)
                     : (pol ? relax_tile_kernel<0, unsigned, true, true> : relax_tile_kernel<0, unsigned, false, true>);
-    int blocks = 0;
-    if (int rc2 = persistent_blocks(kern, n_scan, blocks)) return rc2;
+    int lanes = 0, threads = 0, blocks = 0;
+    if (int rc2 = tile_launch(kern, n_scan, P.raster_ny, lanes, threads, blocks)) return rc2;
     if (cudaMemsetAsync(ctr, 0, sizeof(unsigned), st) != cudaSuccess)
         return set_error(SPM_ERR_CUDA, "spm_relax_pair_dissipation: cannot reset the pixel counter");
-    kern<<<blocks, RX_THREADS, 0, st>>>(G, reinterpret_cast<const float4*>(points), n_scan, P,
-                                        reinterpret_cast<float4*>(FEs), reinterpret_cast<float4*>(disps), iter_count,
-                                        ctr, DA);
+    kern<<<blocks, threads, 0, st>>>(G, reinterpret_cast<const float4*>(points), n_scan, P,
+                                     reinterpret_cast<float4*>(FEs), reinterpret_cast<float4*>(disps), iter_count, ctr,
+                                     lanes, DA);
     return check_launch("spm_relax_pair_dissipation");
 }

@@ -303,6 +303,28 @@ __device__ __forceinline__ float4 blend_cached(const TexelCache& T, float ax, fl
     return r;
 }
 
+// The cell with texel-coordinate floors (fx, fy, fz) of a full grid into the cache; false (cache
+// unchanged) outside the sampler's range.
+template <typename IDX>
+__device__ __forceinline__ bool load_cell_full(const GridView& G, float fx, float fy, float fz, TexelCache& T) {
+    int x0, x1, y0, y1, z0, z1;
+    bool ok = tex_index(fx, G.nx, (float)G.nx, x0, x1);
+    ok = tex_index(fy, G.ny, (float)G.ny, y0, y1) && ok;
+    ok = tex_index(fz, G.nz, (float)G.nz, z0, z1) && ok;
+    if (!ok) return false;
+    const IDX r00 = ((IDX)z0 * G.ny + y0) * G.nx, r10 = ((IDX)z0 * G.ny + y1) * G.nx;
+    const IDX r01 = ((IDX)z1 * G.ny + y0) * G.nx, r11 = ((IDX)z1 * G.ny + y1) * G.nx;
+    const ulonglong2* g = reinterpret_cast<const ulonglong2*>(G.g);
+    T.f000 = __ldg(g + r00 + x0); T.f100 = __ldg(g + r00 + x1);
+    T.f010 = __ldg(g + r10 + x0); T.f110 = __ldg(g + r10 + x1);
+    T.f001 = __ldg(g + r01 + x0); T.f101 = __ldg(g + r01 + x1);
+    T.f011 = __ldg(g + r11 + x0); T.f111 = __ldg(g + r11 + x1);
+    T.kx = fx;
+    T.ky = fy;
+    T.kz = fz;
+    return true;
+}
+
 // interp_fe on a full (nz,ny,nx) grid with any sampling transform, with a
 // TexelCache: the same texels and lerps, so the same sample; the eight
 // texels are loaded only when the cell (the floors of the three texel
@@ -317,25 +339,9 @@ __device__ __forceinline__ float4 interp_fe_cached_full(const GridView& G, float
     const float ax = tex_coord(u, fnx, fx);
     const float ay = tex_coord(v, fny, fy);
     const float az = tex_coord(w, fnz, fz);
-    if (!(fx == T.kx && fy == T.ky && fz == T.kz)) {
-        int x0, x1, y0, y1, z0, z1;
-        bool ok = tex_index(fx, G.nx, fnx, x0, x1);
-        ok = tex_index(fy, G.ny, fny, y0, y1) && ok;
-        ok = tex_index(fz, G.nz, fnz, z0, z1) && ok;
-        if (!ok) {
-            float nan = __int_as_float(0x7fc00000);
-            return make_float4(nan, nan, nan, nan);
-        }
-        const IDX r00 = ((IDX)z0 * G.ny + y0) * G.nx, r10 = ((IDX)z0 * G.ny + y1) * G.nx;
-        const IDX r01 = ((IDX)z1 * G.ny + y0) * G.nx, r11 = ((IDX)z1 * G.ny + y1) * G.nx;
-        const ulonglong2* g = reinterpret_cast<const ulonglong2*>(G.g);
-        T.f000 = __ldg(g + r00 + x0); T.f100 = __ldg(g + r00 + x1);
-        T.f010 = __ldg(g + r10 + x0); T.f110 = __ldg(g + r10 + x1);
-        T.f001 = __ldg(g + r01 + x0); T.f101 = __ldg(g + r01 + x1);
-        T.f011 = __ldg(g + r11 + x0); T.f111 = __ldg(g + r11 + x1);
-        T.kx = fx;
-        T.ky = fy;
-        T.kz = fz;
+    if (!(fx == T.kx && fy == T.ky && fz == T.kz) && !load_cell_full<IDX>(G, fx, fy, fz, T)) {
+        float nan = __int_as_float(0x7fc00000);
+        return make_float4(nan, nan, nan, nan);
     }
     return blend_cached(T, ax, ay, az);
 }
@@ -605,6 +611,31 @@ struct FullCellFetch {
         t[2] = __ldg(G.g + r10 + x0); t[3] = __ldg(G.g + r10 + x1);
         t[4] = __ldg(G.g + r01 + x0); t[5] = __ldg(G.g + r01 + x1);
         t[6] = __ldg(G.g + r11 + x0); t[7] = __ldg(G.g + r11 + x1);
+        return true;
+    }
+};
+
+// FullCellFetch through the lane's TexelCache: the cell FIRE ended in, or the previous evaluation's, needs
+// no loads.  The same texels either way.
+template <typename IDX>
+struct FullCellFetchCached {
+    const GridView& G;
+    TexelCache& T;
+    __device__ __forceinline__ bool operator()(V3 p, float& ax, float& ay, float& az, float4 (&t)[8]) const {
+        const float u = __fmaf_rn(p.x, G.dA.x, __fmaf_rn(p.y, G.dA.y, __fmaf_rn(p.z, G.dA.z, G.dA.w)));
+        const float v = __fmaf_rn(p.x, G.dB.x, __fmaf_rn(p.y, G.dB.y, __fmaf_rn(p.z, G.dB.z, G.dB.w)));
+        const float w = __fmaf_rn(p.x, G.dC.x, __fmaf_rn(p.y, G.dC.y, __fmaf_rn(p.z, G.dC.z, G.dC.w)));
+        float fx, fy, fz;
+        ax = tex_coord(u, (float)G.nx, fx);
+        ay = tex_coord(v, (float)G.ny, fy);
+        az = tex_coord(w, (float)G.nz, fz);
+        if (!(fx == T.kx && fy == T.ky && fz == T.kz) && !load_cell_full<IDX>(G, fx, fy, fz, T)) return false;
+        const ulonglong2 c[8] = {T.f000, T.f100, T.f010, T.f110, T.f001, T.f101, T.f011, T.f111};
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            upk(c[i].x, t[i].x, t[i].y);
+            upk(c[i].y, t[i].z, t[i].w);
+        }
         return true;
     }
 };
