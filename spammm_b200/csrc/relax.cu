@@ -25,6 +25,7 @@
 // This translation unit is compiled with -fmad=false: the only fused
 // multiply-adds are the explicit __fmaf_rn calls shared with the CPU oracle.
 #include <climits>
+#include <type_traits>
 #include "spm_internal.cuh"
 #include "spm_fire.cuh"
 #include "spm_batch.cuh"
@@ -117,7 +118,7 @@ __device__ __forceinline__ PolishSpring pp_spring(const PPFrame& F) {
 
 // The polished output of a relaxStrokes (MODE 0: plain spring) or relaxStrokesTilted (MODE 1:
 // tip frame) z-step: q and fe in, the polished position and the sample there out.
-template <int MODE, typename IDX>
+template <int MODE, typename IDX, bool PLAIN>
 __device__ __forceinline__ void polish_state(const GridView& G, V3 a, V3 b, V3 c, float4 kk, float4 d0, float surf,
                                              V3 tip, V3& q, float4& fe, TexelCache& cache) {
     PolishSpring S;
@@ -125,16 +126,37 @@ __device__ __forceinline__ void polish_state(const GridView& G, V3 a, V3 b, V3 c
     S.kk = kk; S.d0 = d0;
     S.surf = surf;
     S.frame = MODE != 0;
+    if (PLAIN) {  // no rotation, diagonal T
+        S.ident = true;
+        if (MODE == 0) S.surf = 0.f;
+    }
     float T[3][3];
     polish_coefs(G, T);
-    newton_polish(FullCellFetchCached<IDX>{G, cache}, T, S, tip, q, fe);
+    newton_polish(FullCellFetchCached<IDX, PLAIN>{G, cache}, T, S, tip, q, fe);
+}
+
+// Total force of the tilted modes: the sample, the spring in the tip frame a, b, c, the surface bias
+// along c.  PLAIN: the frame is x, y, z and there is no radial bond -- the same values, up to the sign of a
+// zero.
+template <bool PLAIN>
+__device__ __forceinline__ V3 tilted_force(float4 fe, V3 d, V3 a, V3 b, V3 c, float4 kk, float4 d0, float surf) {
+    if (PLAIN) {
+        const V3 ft = tip_spring(d, kk, d0);
+        return mk3(fe.x + ft.x, fe.y + ft.y, __fadd_rn(surf, fe.z + ft.z));
+    }
+    const V3 ft = rotmatT(tip_force(rotmat(d, a, b, c), kk, d0), a, b, c);
+    V3 f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
+    f.x = __fmaf_rn(c.x, surf, f.x);
+    f.y = __fmaf_rn(c.y, surf, f.y);
+    f.z = __fmaf_rn(c.z, surf, f.z);
+    return f;
 }
 
 // One SPM_RELAX_PP iteration (the direct path's bookkeeping: the convergence
 // test comes before the update).  Returns true when the z-step is finished;
 // conv tells whether it converged.  CACHE: sample through the texel cache T
-// (fnx, fny, fnz the dimensions as floats).
-template <typename IDX, bool CACHE>
+// (fnx, fny, fnz the dimensions as floats).  PLAIN: see relax_tile_kernel.
+template <typename IDX, bool CACHE, bool PLAIN>
 __device__ __forceinline__ bool pp_iter(const GridView& G, const PPFrame& F, V3 tip, V3& pos, V3& v, Integrator& I,
                                         float4& fe, int& it, int& total_it, bool& conv, TexelCache& T, float fnx,
                                         float fny, float fnz) {
@@ -142,18 +164,14 @@ __device__ __forceinline__ bool pp_iter(const GridView& G, const PPFrame& F, V3 
     if (it >= F.max_iter) return true;
     ++it;
     ++total_it;
-    if constexpr (CACHE) fe = interp_fe_cached_full<IDX>(G, fnx, fny, fnz, pos, T);
+    if constexpr (CACHE) fe = interp_fe_cached_full<IDX, PLAIN>(G, fnx, fny, fnz, pos, T);
     else fe = interp_fe<IDX>(G, pos);
-    const V3 ft = rotmatT(tip_force(rotmat(sub3(pos, tip), F.a, F.b, F.c), F.kk, F.d0), F.a, F.b, F.c);
-    V3 f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
-    f.x = __fmaf_rn(F.c.x, F.surf, f.x);
-    f.y = __fmaf_rn(F.c.y, F.surf, f.y);
-    f.z = __fmaf_rn(F.c.z, F.surf, f.z);
+    const V3 f = tilted_force<PLAIN>(fe, sub3(pos, tip), F.a, F.b, F.c, F.kk, F.d0, F.surf);
     if (dot3(f, f) < F.f2conv) {
         conv = true;
         return true;
     }
-    md_step(f, v, pos, I, F.fire);
+    md_step(f, v, pos, I, PLAIN || F.fire);
     return it >= F.max_iter;
 }
 
@@ -161,16 +179,18 @@ __device__ __forceinline__ bool pp_iter(const GridView& G, const PPFrame& F, V3 
 // position and PP = (pos, +iterations if converged and finite, else -iterations).
 // POLISH: the state is Newton-polished first (newton_polish); FE is then the sample at the
 // polished position, which PP reports.
-template <typename IDX, bool POLISH>
+template <typename IDX, bool POLISH, bool PLAIN>
 __device__ __forceinline__ void pp_emit(const GridView& G, const PPFrame& F, V3 tip, V3 pos, float4 fe, int it,
                                         bool conv, float4* fe_out, float4* pp_out, TexelCache& cache) {
     if (!conv) fe = interp_fe<IDX>(G, pos);  // the position moved after the last sample
     if constexpr (POLISH) {
         float T[3][3];
         polish_coefs(G, T);
-        newton_polish(FullCellFetchCached<IDX>{G, cache}, T, pp_spring(F), tip, pos, fe);
+        PolishSpring S = pp_spring(F);
+        S.ident = PLAIN;
+        newton_polish(FullCellFetchCached<IDX, PLAIN>{G, cache}, T, S, tip, pos, fe);
     }
-    const V3 r = rotmat(mk3(fe.x, fe.y, fe.z), F.a, F.b, F.c);
+    const V3 r = PLAIN ? mk3(fe.x, fe.y, fe.z) : rotmat(mk3(fe.x, fe.y, fe.z), F.a, F.b, F.c);
     *fe_out = make_float4(r.x, r.y, r.z, fe.w);
     const bool finite = isfinite(fe.x) && isfinite(fe.y) && isfinite(fe.z) && isfinite(fe.w) && isfinite(pos.x) &&
                         isfinite(pos.y) && isfinite(pos.z);
@@ -240,9 +260,9 @@ relax_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_pa
     while (k >= 0) {
         if (MODE == 2) {
             bool conv;
-            if (pp_iter<IDX, CACHE>(G, F, tip, pos, v, I, fe, it, total_it, conv, T, fnx, fny, fnz)) {
+            if (pp_iter<IDX, CACHE, false>(G, F, tip, pos, v, I, fe, it, total_it, conv, T, fnx, fny, fnz)) {
                 const size_t o = (size_t)k * nzs + iz;
-                pp_emit<IDX, POLISH>(G, F, tip, pos, fe, it, conv, FEs + o, disps + o, T);
+                pp_emit<IDX, POLISH, false>(G, F, tip, pos, fe, it, conv, FEs + o, disps + o, T);
                 tip = add3(tip, dTip);
                 pos = add3(pos, dTip);
                 v = mk3(0.f, 0.f, 0.f);
@@ -290,18 +310,14 @@ relax_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_pa
         }
         bool done = max_iter <= 0;
         if (!done) {
-            if constexpr (CACHE) fe = interp_fe_cached_full<IDX>(G, fnx, fny, fnz, pos, T);
+            if constexpr (CACHE) fe = interp_fe_cached_full<IDX, false>(G, fnx, fny, fnz, pos, T);
             else fe = interp_fe<IDX>(G, pos);
             V3 f;
             if (MODE == 0) {
                 const V3 ft = tip_force(sub3(pos, tip), kk, d0);
                 f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
             } else {
-                const V3 ft = rotmatT(tip_force(rotmat(sub3(pos, tip), a, b, c), kk, d0), a, b, c);
-                f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
-                f.x = __fmaf_rn(c.x, surf, f.x);
-                f.y = __fmaf_rn(c.y, surf, f.y);
-                f.z = __fmaf_rn(c.z, surf, f.z);
+                f = tilted_force<false>(fe, sub3(pos, tip), a, b, c, kk, d0, surf);
             }
             md_step(f, v, pos, I, fire);
             ++it;
@@ -314,13 +330,13 @@ relax_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_pa
             V3 q = pos;  // the output position (polished or not); the next z-step starts from pos
             if (MODE == 0) {
                 float4 fo = fe;
-                if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, fo, T);
+                if constexpr (POLISH) polish_state<MODE, IDX, false>(G, a, b, c, kk, d0, surf, tip, q, fo, T);
                 FEs[o] = fo;
                 const V3 ref = mk3(tip.x + d0.x, tip.y + d0.y, tip.z + d0.z);
                 disps[o] = make_float4(q.x - ref.x, q.y - ref.y, q.z - ref.z, 0.f);
             } else {
                 float4 g = interp_fe<IDX>(G, pos);
-                if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, g, T);
+                if constexpr (POLISH) polish_state<MODE, IDX, false>(G, a, b, c, kk, d0, surf, tip, q, g, T);
                 const V3 r = rotmat(mk3(g.x, g.y, g.z), a, b, c);
                 FEs[o] = make_float4(r.x, r.y, r.z, g.w);
             }
@@ -375,7 +391,13 @@ struct DissArgs {
 // ms).  The
 // per-lane sequence is relax_kernel's (the same iteration, emit and texel
 // cache), so the results are the same bits.
-template <int MODE, typename IDX, bool POLISH, bool DISS = false>
+//
+// PLAIN (plain_scan): FIRE on an axis-aligned grid without a radial bond, the tilted modes with the frame x,
+// y, z -- the usual scan.  The transform's and the rotations' zero and unit terms and the per-step tests of
+// the flags are left out: the loop is bound by its instructions (157 per step, 3.7 cycles each with one warp
+// per scheduler), the same values up to the sign of a zero.  480 x 480 x 60: 2.11 -> 1.97 ms, with polished
+// PP bookkeeping 3.04 -> 2.52; 100 x 100 x 40: 648 -> 573 us.
+template <int MODE, typename IDX, bool POLISH, bool PLAIN, bool DISS = false>
 __global__ void __launch_bounds__(RX_THREADS)
 relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_params P,
                   float4* __restrict__ FEs, float4* __restrict__ disps, int* __restrict__ iter_count,
@@ -443,26 +465,22 @@ relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_sc
                 int it = 0;
                 if (MODE == 2) {
                     bool conv;
-                    while (!pp_iter<IDX, true>(G, F, tip, pos, v, I, fe, it, total_it, conv, T, fnx, fny, fnz)) {
+                    while (!pp_iter<IDX, true, PLAIN>(G, F, tip, pos, v, I, fe, it, total_it, conv, T, fnx, fny, fnz)) {
                     }
                     const size_t o = (size_t)k * nzs + iz;
-                    pp_emit<IDX, POLISH>(G, F, tip, pos, fe, it, conv, FEs + o, disps + o, T);
+                    pp_emit<IDX, POLISH, PLAIN>(G, F, tip, pos, fe, it, conv, FEs + o, disps + o, T);
                 } else {
                     bool done = max_iter <= 0;
                     while (!done) {
-                        fe = interp_fe_cached_full<IDX>(G, fnx, fny, fnz, pos, T);
+                        fe = interp_fe_cached_full<IDX, PLAIN>(G, fnx, fny, fnz, pos, T);
                         V3 f;
                         if (MODE == 0) {
-                            const V3 ft = tip_force(sub3(pos, tip), kk, d0);
+                            const V3 ft = PLAIN ? tip_spring(sub3(pos, tip), kk, d0) : tip_force(sub3(pos, tip), kk, d0);
                             f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
                         } else {
-                            const V3 ft = rotmatT(tip_force(rotmat(sub3(pos, tip), a, b, c), kk, d0), a, b, c);
-                            f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
-                            f.x = __fmaf_rn(c.x, surf, f.x);
-                            f.y = __fmaf_rn(c.y, surf, f.y);
-                            f.z = __fmaf_rn(c.z, surf, f.z);
+                            f = tilted_force<PLAIN>(fe, sub3(pos, tip), a, b, c, kk, d0, surf);
                         }
-                        md_step(f, v, pos, I, fire);
+                        md_step(f, v, pos, I, PLAIN || fire);
                         ++it;
                         ++total_it;
                         done = (dot3(f, f) < P.f2conv) || (it >= max_iter);
@@ -472,14 +490,14 @@ relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_sc
                     V3 q = pos;  // the output position; the next z-step starts from pos
                     if (MODE == 0) {
                         float4 fo = fe;
-                        if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, fo, T);
+                        if constexpr (POLISH) polish_state<MODE, IDX, PLAIN>(G, a, b, c, kk, d0, surf, tip, q, fo, T);
                         FEs[o] = fo;
                         const V3 ref = mk3(tip.x + d0.x, tip.y + d0.y, tip.z + d0.z);
                         disps[o] = make_float4(q.x - ref.x, q.y - ref.y, q.z - ref.z, 0.f);
                     } else {
                         float4 g = interp_fe<IDX>(G, pos);
-                        if constexpr (POLISH) polish_state<MODE, IDX>(G, a, b, c, kk, d0, surf, tip, q, g, T);
-                        const V3 r = rotmat(mk3(g.x, g.y, g.z), a, b, c);
+                        if constexpr (POLISH) polish_state<MODE, IDX, PLAIN>(G, a, b, c, kk, d0, surf, tip, q, g, T);
+                        const V3 r = PLAIN ? mk3(g.x, g.y, g.z) : rotmat(mk3(g.x, g.y, g.z), a, b, c);
                         FEs[o] = make_float4(r.x, r.y, r.z, g.w);
                     }
                 }
@@ -585,6 +603,15 @@ int persistent_blocks(K kern, long long warps, int threads, int& blocks) {
     return SPM_OK;
 }
 
+// The scans relax_tile_kernel's PLAIN form covers.
+bool plain_scan(int mode, const spm_scan_params& P) {
+    const bool axis = P.dinvA[1] == 0.f && P.dinvA[2] == 0.f && P.dinvB[0] == 0.f && P.dinvB[2] == 0.f &&
+                      P.dinvC[0] == 0.f && P.dinvC[1] == 0.f;
+    const bool frame = P.tipA[0] == 1.f && P.tipA[1] == 0.f && P.tipA[2] == 0.f && P.tipB[0] == 0.f &&
+                       P.tipB[1] == 1.f && P.tipB[2] == 0.f && P.tipC[0] == 0.f && P.tipC[1] == 0.f && P.tipC[2] == 1.f;
+    return axis && (mode == SPM_RELAX_STROKES || frame) && P.stiffness[3] == 0.f && (P.flags & SPM_FLAG_FIRE);
+}
+
 // Pixels per warp of a scan of n pixels: 32, halved while that gives fewer than WARPS_PER_SCHEDULER warps
 // for each of the GPU's schedulers.  100 x 100 pixels x 40 z-steps: 32 pixels per warp 893 us, at least one
 // warp per scheduler (16 pixels) 658, two (8) 718, four (4) 980; 24 x 24 x 20: 358 -> 311.
@@ -618,6 +645,8 @@ int launch_relax(const GridView& G, const float4* pts, int n_scan, const spm_sca
             return set_error(SPM_ERR_CUDA, "relax: cannot reset the pixel counter");
         if constexpr (MODE <= 2) {  // z-synchronised tiles from the counter
             auto kern = relax_tile_kernel<MODE, IDX, POLISH, false>;
+            if constexpr (std::is_same<IDX, unsigned>::value)
+                if (plain_scan(MODE, P)) kern = relax_tile_kernel<MODE, IDX, POLISH, true>;
             int lanes = 0, threads = 0, blocks = 0;
             if (int rc = tile_launch(kern, n_scan, P.raster_ny, lanes, threads, blocks)) return rc;
             kern<<<blocks, threads, 0, st>>>(G, pts, n_scan, P, FEs, disps, iter_count, counter, lanes, DissArgs{});
@@ -682,7 +711,8 @@ __device__ __forceinline__ float4 sample_z(const AxisView& G, V3 p, TexelCache& 
     else return interp_fe_cell<IDX, LAYOUT>(G, p);
 }
 
-template <typename IDX, bool CACHE, int LAYOUT>
+// PLAIN: FIRE without a radial bond (the tests left out of the loop: 64-molecule forward 27.2 -> 26.3 ms).
+template <typename IDX, bool CACHE, int LAYOUT, bool PLAIN = false>
 __device__ __forceinline__ bool pp_iter_z(const AxisView& G, TexelCache& T, const spm_scan_params& P, V3 tip,
                                           V3& pos, V3& v, float& dt, float& damp, float4& fe, int& it, int& total_it,
                                           bool& conv) {
@@ -692,7 +722,8 @@ __device__ __forceinline__ bool pp_iter_z(const AxisView& G, TexelCache& T, cons
     ++total_it;
     fe = sample_z<IDX, CACHE, LAYOUT>(G, pos, T);
     if (fe.w != fe.w) return true;  // outside the slab (or a NaN grid): not converged
-    const V3 ft = tip_force(sub3(pos, tip), ld4(P.stiffness), ld4(P.dpos0));
+    const V3 ft = PLAIN ? tip_spring(sub3(pos, tip), ld4(P.stiffness), ld4(P.dpos0))
+                        : tip_force(sub3(pos, tip), ld4(P.stiffness), ld4(P.dpos0));
     V3 f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
     f.z = __fadd_rn(f.z, P.surfFF[0]);
     if (dot3(f, f) < P.f2conv) {
@@ -701,7 +732,7 @@ __device__ __forceinline__ bool pp_iter_z(const AxisView& G, TexelCache& T, cons
     }
     // the stroke's integrator constants straight from the launch parameters (dtmin = dtmax * 0.1)
     md_step_c(f, v, pos, dt, damp, __fmul_rn(P.relax_params[0], 0.1f), P.relax_params[0], P.relax_params[1],
-              (P.flags & SPM_FLAG_FIRE) != 0);
+              PLAIN || (P.flags & SPM_FLAG_FIRE) != 0);
     return it >= P.max_iter;
 }
 
@@ -986,8 +1017,14 @@ __device__ __forceinline__ bool stroke_zstep(const AxisView& G, TexelCache& T, c
     }
     L.total_it += it;
     if (!newton_done) {
-        while (!pp_iter_z<unsigned, CACHE, LAYOUT>(G, T, P, L.tip, pos, L.v, L.dt, L.damp, fe, it, L.total_it,
-                                                   conv)) {
+        if (P.stiffness[3] == 0.f && (P.flags & SPM_FLAG_FIRE)) {
+            while (!pp_iter_z<unsigned, CACHE, LAYOUT, true>(G, T, P, L.tip, pos, L.v, L.dt, L.damp, fe, it, L.total_it,
+                                                             conv)) {
+            }
+        } else {
+            while (!pp_iter_z<unsigned, CACHE, LAYOUT>(G, T, P, L.tip, pos, L.v, L.dt, L.damp, fe, it, L.total_it,
+                                                       conv)) {
+            }
         }
         if (!conv) fe = sample_z<unsigned, CACHE, LAYOUT>(G, pos, T);  // the position moved after the last sample
     }
@@ -1694,8 +1731,12 @@ extern "C" int spm_relax_pair_dissipation(const float* grid, int nx, int ny, int
         return set_error(SPM_ERR_CUDA, "spm_relax_pair_dissipation: cannot reset the pair counters");
     const bool big = (long long)nx * ny * nz >= (1LL << 32);
     const bool pol = (P.flags & SPM_FLAG_POLISH) != 0;
-    auto kern = big ? (pol ? relax_tile_kernel<0, size_t, true, true> : relax_tile_kernel<0, size_t, false, true>)
-                    : (pol ? relax_tile_kernel<0, unsigned, true, true> : relax_tile_kernel<0, unsigned, false, true>);
+    auto kern = big ? (pol ? relax_tile_kernel<0, size_t, true, false, true>
+                           : relax_tile_kernel<0, size_t, false, false, true>)
+                : plain_scan(0, P) ? (pol ? relax_tile_kernel<0, unsigned, true, true, true>
+                                          : relax_tile_kernel<0, unsigned, false, true, true>)
+                                   : (pol ? relax_tile_kernel<0, unsigned, true, false, true>
+                                          : relax_tile_kernel<0, unsigned, false, false, true>);
     int lanes = 0, threads = 0, blocks = 0;
     if (int rc2 = tile_launch(kern, n_scan, P.raster_ny, lanes, threads, blocks)) return rc2;
     if (cudaMemsetAsync(ctr, 0, sizeof(unsigned), st) != cudaSuccess)

@@ -32,12 +32,16 @@ __device__ __forceinline__ V3 rotmatT(V3 v, V3 a, V3 b, V3 c) {
               __fmaf_rn(c.z, v.z, __fmaf_rn(b.z, v.y, __fmul_rn(a.z, v.x)))};
 }
 
+// tip_force without the radial bond (k.w == 0).
+__device__ __forceinline__ V3 tip_spring(V3 d, float4 k, float4 d0) {
+    return V3{__fmul_rn(d.x - d0.x, k.x), __fmul_rn(d.y - d0.y, k.y), __fmul_rn(d.z - d0.z, k.z)};
+}
+
 // Harmonic 3D spring + radial bond: (d - d0.xyz)*k.xyz + d*(k.w*(r - d0.w)/r).
 // With k.w == 0 the radial term is exactly +-0 and is skipped (only the sign of
 // an all-zero component can differ from adding it; the oracle does the same).
 __device__ __forceinline__ V3 tip_force(V3 d, float4 k, float4 d0) {
-    if (k.w == 0.f)
-        return V3{__fmul_rn(d.x - d0.x, k.x), __fmul_rn(d.y - d0.y, k.y), __fmul_rn(d.z - d0.z, k.z)};
+    if (k.w == 0.f) return tip_spring(d, k, d0);
     float r = __fsqrt_rn(dot3(d, d));
     r = fmaxf(r, 1e-10f);
     float s = __fdiv_rn(__fmul_rn(k.w, r - d0.w), r);
@@ -303,6 +307,17 @@ __device__ __forceinline__ float4 blend_cached(const TexelCache& T, float ax, fl
     return r;
 }
 
+// Normalized texture coordinates of p.  AXIS: dinvA, dinvB, dinvC are multiples of x, y, z (their zero terms
+// are exact: the same values, up to the sign of a zero).
+template <bool AXIS>
+__device__ __forceinline__ V3 tex_uvw(const GridView& G, V3 p) {
+    if (AXIS)
+        return mk3(__fmaf_rn(p.x, G.dA.x, G.dA.w), __fmaf_rn(p.y, G.dB.y, G.dB.w), __fmaf_rn(p.z, G.dC.z, G.dC.w));
+    return mk3(__fmaf_rn(p.x, G.dA.x, __fmaf_rn(p.y, G.dA.y, __fmaf_rn(p.z, G.dA.z, G.dA.w))),
+               __fmaf_rn(p.x, G.dB.x, __fmaf_rn(p.y, G.dB.y, __fmaf_rn(p.z, G.dB.z, G.dB.w))),
+               __fmaf_rn(p.x, G.dC.x, __fmaf_rn(p.y, G.dC.y, __fmaf_rn(p.z, G.dC.z, G.dC.w))));
+}
+
 // The cell with texel-coordinate floors (fx, fy, fz) of a full grid into the cache; false (cache
 // unchanged) outside the sampler's range.
 template <typename IDX>
@@ -329,12 +344,11 @@ __device__ __forceinline__ bool load_cell_full(const GridView& G, float fx, floa
 // TexelCache: the same texels and lerps, so the same sample; the eight
 // texels are loaded only when the cell (the floors of the three texel
 // coordinates) changes.  fnx, fny, fnz: the dimensions as floats.
-template <typename IDX>
+template <typename IDX, bool AXIS>
 __device__ __forceinline__ float4 interp_fe_cached_full(const GridView& G, float fnx, float fny, float fnz, V3 p,
                                                         TexelCache& T) {
-    const float u = __fmaf_rn(p.x, G.dA.x, __fmaf_rn(p.y, G.dA.y, __fmaf_rn(p.z, G.dA.z, G.dA.w)));
-    const float v = __fmaf_rn(p.x, G.dB.x, __fmaf_rn(p.y, G.dB.y, __fmaf_rn(p.z, G.dB.z, G.dB.w)));
-    const float w = __fmaf_rn(p.x, G.dC.x, __fmaf_rn(p.y, G.dC.y, __fmaf_rn(p.z, G.dC.z, G.dC.w)));
+    const V3 t = tex_uvw<AXIS>(G, p);
+    const float u = t.x, v = t.y, w = t.z;
     float fx, fy, fz;
     const float ax = tex_coord(u, fnx, fx);
     const float ay = tex_coord(v, fny, fy);
@@ -617,18 +631,16 @@ struct FullCellFetch {
 
 // FullCellFetch through the lane's TexelCache: the cell FIRE ended in, or the previous evaluation's, needs
 // no loads.  The same texels either way.
-template <typename IDX>
+template <typename IDX, bool AXIS>
 struct FullCellFetchCached {
     const GridView& G;
     TexelCache& T;
     __device__ __forceinline__ bool operator()(V3 p, float& ax, float& ay, float& az, float4 (&t)[8]) const {
-        const float u = __fmaf_rn(p.x, G.dA.x, __fmaf_rn(p.y, G.dA.y, __fmaf_rn(p.z, G.dA.z, G.dA.w)));
-        const float v = __fmaf_rn(p.x, G.dB.x, __fmaf_rn(p.y, G.dB.y, __fmaf_rn(p.z, G.dB.z, G.dB.w)));
-        const float w = __fmaf_rn(p.x, G.dC.x, __fmaf_rn(p.y, G.dC.y, __fmaf_rn(p.z, G.dC.z, G.dC.w)));
+        const V3 uvw = tex_uvw<AXIS>(G, p);
         float fx, fy, fz;
-        ax = tex_coord(u, (float)G.nx, fx);
-        ay = tex_coord(v, (float)G.ny, fy);
-        az = tex_coord(w, (float)G.nz, fz);
+        ax = tex_coord(uvw.x, (float)G.nx, fx);
+        ay = tex_coord(uvw.y, (float)G.ny, fy);
+        az = tex_coord(uvw.z, (float)G.nz, fz);
         if (!(fx == T.kx && fy == T.ky && fz == T.kz) && !load_cell_full<IDX>(G, fx, fy, fz, T)) return false;
         const ulonglong2 c[8] = {T.f000, T.f100, T.f010, T.f110, T.f001, T.f101, T.f011, T.f111};
 #pragma unroll
