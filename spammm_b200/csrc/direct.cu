@@ -26,6 +26,7 @@ namespace spm {
 namespace {
 
 constexpr int DX_THREADS = 128;
+constexpr int BOUND_ATOMS = 256;
 constexpr float R2SAFE = 1e-4f;
 constexpr float COULOMB_CONST = 14.3996448915f;
 constexpr float LOG2E = 1.4426950408889634f;
@@ -163,10 +164,54 @@ __device__ __noinline__ double group_force2_f64(V3 p, V3 tip, int na, int sub, u
     return fx * fx + fy * fy + fz * fz;
 }
 
-// Groups of LPP lanes, one pixel per group (DX_THREADS / LPP pixels per CTA, in raster order); the
+// Bound of |F32 - F64| of the total force at p, summed over the group: what the FP32 evaluation above can be
+// off from group_force2_f64, from its roundings.  Per atom, with x the exponent of the Morse factor e:
+// differences, r^2, rsqrt.approx and r = r^2 rsqrt err by at most 8e-7 of r, so e errs by (8e-7 + 2^-23)
+// |x| ln 2 < 1.5e-6 |x|, and the force 2 K E0 e (e - 1), whose difference cancels near the minimum, by that
+// times e (1 + e) plus 2e-6 for its own products; a charge site's force by 2e-6 and by 4e-7 (|dz| + |qz|) / r
+// for the rounded offset; the sum of na terms adds na 2^-24 of their magnitudes.  The spring: 4e-7 of the
+// lengths times their stiffnesses (rotations, root, products) and of the force itself.
+template <int NS, int LPP>
+__device__ __noinline__ float group_force_bound(V3 p, V3 tip, int na, int sub, unsigned gmask, const float4* s_pos,
+                                                const float4* s_m, const float* s_q, const Sites& S, float4 kk,
+                                                float4 d0, float surf) {
+    float err = 0.f, mag = 0.f;
+    for (int j = sub; j < na; j += LPP) {
+        const float4 a = s_pos[j];
+        const float4 m = s_m[j];
+        const float dx = p.x - a.x, dy = p.y - a.y, dz = p.z - a.z;
+        const float dxy2 = fmaf(dx, dx, fmaf(dy, dy, R2SAFE));
+        const float r2 = fmaf(dz, dz, dxy2);
+        const float r = r2 * fast_rsqrt(r2);
+        const float e = fast_ex2(fmaf(m.x, r, m.y));
+        const float b = fabsf(m.w * e) * (1.f + e);
+        err = fmaf(b, fmaf(1.5e-6f, fmaf(fabsf(m.x), r, fabsf(m.y)), 2e-6f), err);
+        mag += b;
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            const float dzk = dz + S.qz[k];
+            const float rsk = fast_rsqrt(fmaf(dzk, dzk, dxy2));
+            const float f = fabsf(s_q[k * na + j]) * rsk * rsk;
+            err = fmaf(f, fmaf(4e-7f, (fabsf(dz) + fabsf(S.qz[k])) * rsk, 2e-6f), err);
+            mag += f;
+        }
+    }
+    err = group_sum<LPP>(err, gmask);
+    mag = group_sum<LPP>(mag, gmask);
+    const V3 d = sub3(p, tip);
+    const float len = sqrtf(dot3(d, d)), l0 = fabsf(d0.x) + fabsf(d0.y) + fabsf(d0.z);
+    const float k3 = fmaxf(fabsf(kk.x), fmaxf(fabsf(kk.y), fabsf(kk.z)));
+    const float spring = k3 * (len + l0) + fabsf(kk.w) * (len + 0.25f * fabsf(len - fabsf(d0.w))) + fabsf(surf);
+    return err + 6e-8f * (float)(na + 8) * mag + 4e-7f * spring;
+}
+
+// Groups of LPP lanes, one pixel per group (blockDim / LPP pixels per CTA, in raster order); the
 // whole molecule staged in shared memory; each group runs its pixel's (z-step, FIRE step) sequence
 // with the stroke state held identically by every lane of the group.  Convergence is tested before
-// the update, and an FP32 "converged" is confirmed in FP64.
+// the update, and an FP32 "converged" is confirmed in FP64 -- unless the FP32 force is below the threshold by
+// more than its error bound, where FP64 cannot decide otherwise (most confirmations of molecules; beyond
+// BOUND_ATOMS atoms the bound of the sum's rounding nears the threshold and is not tried).  38 atoms, 100 x
+// 100 pixels x 40 z-steps, at 16 lanes per pixel: 1686 -> 1405 us.  ident: the tip frame is x, y, z (the rotations change no value).
 template <int NS, int LPP>
 __global__ void __launch_bounds__(DX_THREADS)
 relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __restrict__ cMs,
@@ -180,7 +225,7 @@ relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __re
     __syncthreads();
     const int lane = threadIdx.x & 31, sub = lane & (LPP - 1);
     const unsigned gmask = (LPP == 32) ? 0xffffffffu : (((1u << LPP) - 1u) << (lane & ~(LPP - 1)));
-    const int k = blockIdx.x * (DX_THREADS / LPP) + threadIdx.x / LPP;
+    const int k = blockIdx.x * (blockDim.x / LPP) + threadIdx.x / LPP;
     if (k >= n_scan) return;  // the whole group
 
     const float4 kk = make_float4(P.stiffness[0], P.stiffness[1], P.stiffness[2], P.stiffness[3]);
@@ -190,6 +235,8 @@ relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __re
     const V3 c = mk3(P.tipC[0], P.tipC[1], P.tipC[2]);
     const V3 dTip = mk3(c.x * P.tipC[3], c.y * P.tipC[3], c.z * P.tipC[3]);
     const float surf = P.surfFF[0];
+    const bool ident = a.x == 1.f && a.y == 0.f && a.z == 0.f && b.x == 0.f && b.y == 1.f && b.z == 0.f &&
+                       c.x == 0.f && c.y == 0.f && c.z == 1.f;
     const float4 p4 = pts[k];
     V3 tip = mk3(p4.x, p4.y, p4.z);
     V3 pos = add3(tip, rotmatT(mk3(d0.x, d0.y, d0.z), a, b, c));
@@ -210,14 +257,29 @@ relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __re
         if (it < P.max_iter) {
             ++it;
             fe = group_pair_sum<NS, LPP>(pos, na, sub, gmask, s_pos, s_m, s_q, S.qz);
-            const V3 ft = rotmatT(tip_force(rotmat(sub3(pos, tip), a, b, c), kk, d0), a, b, c);
+            const V3 d = sub3(pos, tip);
+            const V3 ft = ident ? tip_force(d, kk, d0) : rotmatT(tip_force(rotmat(d, a, b, c), kk, d0), a, b, c);
             V3 f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
-            f.x = fmaf(c.x, surf, f.x);
-            f.y = fmaf(c.y, surf, f.y);
-            f.z = fmaf(c.z, surf, f.z);
-            if (dot3(f, f) < P.f2conv &&
-                group_force2_f64<LPP>(pos, tip, na, sub, gmask, atoms, cMs, S, a, b, c, kk, d0, surf) <
-                    (double)P.f2conv) {
+            if (ident) {
+                f.z += surf;
+            } else {
+                f.x = fmaf(c.x, surf, f.x);
+                f.y = fmaf(c.y, surf, f.y);
+                f.z = fmaf(c.z, surf, f.z);
+            }
+            const float f2 = dot3(f, f);
+            bool below = false;
+            if (f2 < P.f2conv) {
+                if (na <= BOUND_ATOMS) {
+                    const float far = sqrtf(f2) + group_force_bound<NS, LPP>(pos, tip, na, sub, gmask, s_pos, s_m, s_q,
+                                                                             S, kk, d0, surf);
+                    below = far * far < 0.999f * P.f2conv;
+                }
+                below = below ||
+                        group_force2_f64<LPP>(pos, tip, na, sub, gmask, atoms, cMs, S, a, b, c, kk, d0,
+                                              surf) < (double)P.f2conv;
+            }
+            if (below) {
                 done = conv = true;
             } else {
                 md_step(f, v, pos, I, true);
@@ -541,11 +603,13 @@ Sites make_sites(const float* Qs, const float* QZs, bool compact, int* ns) {
     return S;
 }
 
-// Lanes per pixel: about four atoms per lane, at least 4 and at most 32 lanes, more while the scan
-// leaves the GPU short of warps (fewer than ~8 warps per SM of a 148-SM part).
+// Lanes per pixel: about eight atoms per lane, at least 4 and at most 32 lanes, more while the scan
+// leaves the GPU short of warps (fewer than ~8 warps per SM of a 148-SM part).  38 atoms, 100 x 100 pixels x 40
+// z-steps: four atoms per lane (16 lanes) 1405 us, eight (8 lanes) 1193, sixteen (4 lanes, two warps per
+// scheduler) 1850; with 64 x 50 pixels half as many warps cost 638 us against 466.
 int direct_lpp(int na, int n_scan) {
     int lpp = 4;
-    while (lpp < 32 && lpp * 4 < na) lpp *= 2;
+    while (lpp < 32 && lpp * 8 < na) lpp *= 2;
     while (lpp < 32 && (long long)n_scan * lpp < 148LL * 8 * 32) lpp *= 2;
     return lpp;
 }
@@ -562,9 +626,11 @@ int launch_direct(int na, const float* atoms, const float* cMs, const float* poi
         if (e != cudaSuccess) return set_error(SPM_ERR_CUDA, "spm_relax_direct_morse: smem %zu B: %s", smem,
                                                cudaGetErrorString(e));
     }
-    const int per_cta = DX_THREADS / lpp;
+    // two-warp CTAs spread a scan of a few thousand warps evenly over the SMs; a large molecule is staged
+    // for four warps at a time
+    const int threads = smem <= 8 * 1024 ? 64 : DX_THREADS, per_cta = threads / lpp;
     const int blocks = (n_scan + per_cta - 1) / per_cta;
-    kern<<<blocks, DX_THREADS, smem, st>>>(na, reinterpret_cast<const float4*>(atoms),
+    kern<<<blocks, threads, smem, st>>>(na, reinterpret_cast<const float4*>(atoms),
                                            reinterpret_cast<const float4*>(cMs),
                                            reinterpret_cast<const float4*>(points), n_scan, P, S,
                                            reinterpret_cast<float4*>(FEs), reinterpret_cast<float4*>(PPs));
