@@ -345,6 +345,21 @@ int spm_adjoint_grid_params(int kind, int n_atoms, const float* atoms, const flo
                             void* scratch, void* stream);
 long long spm_adjoint_grid_scratch_bytes(int n_atoms, long long n_state);
 
+/* The same gradients node by node: the states' w*ubar are summed onto the
+ * nx*ny*nz grid nodes (64-bit fixed point, scale 2^42 / max|ubar|: exact, at
+ * most 2^20 states per node), each touched node then contracted once per atom
+ * (FP64 sums, fixed order) instead of once per state and corner.  Results as
+ * spm_adjoint_grid_params up to rounding.  1 <= n_atoms, n_state; scratch >=
+ * spm_adjoint_grid_nodes_scratch_bytes (32 bytes per grid node; only the box of
+ * touched nodes is used), 16-byte aligned, its content arbitrary. */
+int spm_adjoint_grid_params_nodes(int kind, int n_atoms, const float* atoms, const float* params,
+                                  const float* p0, const float* dA, const float* dB, const float* dC,
+                                  const float* Qs, const float* QZs, int nx, int ny, int nz,
+                                  const spm_scan_params* p, const float* PPs, const float* ubar,
+                                  const float* dk, long long n_state, double* grad, double* dk_sum,
+                                  void* scratch, void* stream);
+long long spm_adjoint_grid_nodes_scratch_bytes(int n_atoms, long long n_state, int nx, int ny, int nz);
+
 /* ------------------------------------------------------------------------
  * Batched grid path: many molecules of uneven atom count, grid size and scan
  * window, each stage ONE launch over the whole batch (no counterpart in the

@@ -164,6 +164,9 @@ _SIGNATURES = {
     "spm_adjoint_grid_params": (_i, [_i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _P, _vp, _vp,
                                      _vp, _ll, _vp, _vp, _vp, _vp]),
     "spm_adjoint_grid_scratch_bytes": (_ll, [_i, _ll]),
+    "spm_adjoint_grid_params_nodes": (_i, [_i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _P, _vp, _vp, _vp,
+                                           _ll, _vp, _vp, _vp, _vp]),
+    "spm_adjoint_grid_nodes_scratch_bytes": (_ll, [_i, _ll, _i, _i, _i]),
     "spm_batch_default_shape": (BatchShape, []),
     "spm_batch_prepare": (_i, [ctypes.POINTER(BatchMol), _i, _BS, _LLP]),
     "spm_batch_grid_build": (_i, [_i, _i, _vp, _ll, _BS, _vp, _vp, _vp, _vp, _vp, _vp]),

@@ -26,6 +26,8 @@
 //                              state-major gather: no scatter onto the grid, no
 //                              atomics), FP64 accumulation, fixed-order CTA
 //                              tree, then a fixed-order fold over chunks.
+//   grid_nodes_*_kernel        node-major form of the gather for larger scans: w * ubar
+//                              summed onto the grid's nodes, each node once per atom
 // Batched (spm_batch_*, many molecules per launch), node-major instead:
 //   batch_ubar_max_kernel      per-molecule max |ubar| (fixed-point scale)
 //   batch_scatter_kernel       w * ubar onto each state's 8 corner nodes of an
@@ -1024,6 +1026,222 @@ batch_scatter_tile_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, uns
     }
 }
 
+// ---- node-major adjoint of one grid ------------------------------------------
+// spm_adjoint_grid_params_nodes: the states' w*ubar are summed onto the grid's nodes first (64-bit fixed point
+// as the batch's scatter: exact, in any order), then every touched node is evaluated once per atom with
+// pair_grad and FP64 sums.  The state-major gather evaluates it once per (state, corner): on a 0.1 A raster of
+// 100 x 100 pixels x 40 z-steps 3.2 million corners fall on 0.44 million nodes, and the kernel was bound by
+// its evaluations and conversions to FP64: the call with 38 atoms takes 826 -> 233 us, with 120 atoms on 128 x
+// 128 x 40 states 3917 -> 491, on 24 x 24 x 20 states 108 either way.
+// Only the box of touched nodes is cleared and read.
+constexpr int GN_THREADS = 256;
+constexpr int GN_CTAS = 592;  // four per SM of a 148-SM part; fixed, so that the sums' order is
+
+struct NodesHead {
+    unsigned umax;  // max |ubar| (float bits) of the states that touch the grid; infinity's if one is not finite
+    int box[6];     // max of (nx-1-x, x+1, ny-1-y, y+1, nz-1-z, z+1) over their corners (all zero: none)
+    int pad;
+};
+
+struct NodesBox {
+    int x0, y0, z0, nx, ny, nz;
+    __device__ __forceinline__ NodesBox(const NodesHead* H, const GridView& G) {
+        x0 = G.nx - 1 - H->box[0]; nx = H->box[1] > 0 ? H->box[1] - x0 : 0;
+        y0 = G.ny - 1 - H->box[2]; ny = H->box[3] > 0 ? H->box[3] - y0 : 0;
+        z0 = G.nz - 1 - H->box[4]; nz = H->box[5] > 0 ? H->box[5] - z0 : 0;
+    }
+    __device__ __forceinline__ long long total() const { return (long long)nx * ny * nz; }
+    // grid node index of box node i, and its coordinates
+    __device__ __forceinline__ size_t node(const GridView& G, long long i, int& x, int& y, int& z) const {
+        const long long r = i / nx;
+        x = x0 + (int)(i - r * nx);
+        y = y0 + (int)(r % ny);
+        z = z0 + (int)(r / ny);
+        return ((size_t)z * G.ny + y) * G.nx + x;
+    }
+};
+
+__device__ __forceinline__ bool has_weight(float4 u) { return !(u.x == 0.f && u.y == 0.f && u.z == 0.f && u.w == 0.f); }
+
+__global__ void __launch_bounds__(GN_THREADS)
+grid_nodes_box_kernel(GridView G, long long n_state, const float4* __restrict__ PPs, const float4* __restrict__ ubar,
+                      NodesHead* __restrict__ H) {
+    __shared__ int s_v[7];
+    if (threadIdx.x < 7) s_v[threadIdx.x] = 0;
+    __syncthreads();
+    int v[7] = {0, 0, 0, 0, 0, 0, 0};
+    for (long long st = (long long)blockIdx.x * GN_THREADS + threadIdx.x; st < n_state; st += (long long)gridDim.x * GN_THREADS) {
+        const float4 u = __ldg(ubar + st);
+        if (!has_weight(u)) continue;
+        const float4 pp = __ldg(PPs + st);
+        const Corners C = corners_of<false>(G, mk3(pp.x, pp.y, pp.z));
+        if (!C.ok) continue;
+        // a finite non-negative float's bits order as an int; one that is not finite is above them all
+        const bool fin = isfinite(u.x) && isfinite(u.y) && isfinite(u.z) && isfinite(u.w);
+        v[0] = max(v[0], fin ? __float_as_int(fmaxf(fmaxf(fabsf(u.x), fabsf(u.y)), fmaxf(fabsf(u.z), fabsf(u.w))))
+                             : 0x7f800000);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            v[1] = max(v[1], G.nx - 1 - C.x[k]); v[2] = max(v[2], C.x[k] + 1);
+            v[3] = max(v[3], G.ny - 1 - C.y[k]); v[4] = max(v[4], C.y[k] + 1);
+            v[5] = max(v[5], G.nz - 1 - C.z[k]); v[6] = max(v[6], C.z[k] + 1);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+        const int w = __reduce_max_sync(0xffffffffu, v[k]);
+        if ((threadIdx.x & 31) == 0 && w > 0) atomicMax(s_v + k, w);
+    }
+    __syncthreads();
+    if (threadIdx.x < 7 && s_v[threadIdx.x] > 0) atomicMax(reinterpret_cast<int*>(H) + threadIdx.x, s_v[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(GN_THREADS)
+grid_nodes_clear_kernel(GridView G, const NodesHead* __restrict__ H, ulonglong2* __restrict__ q) {
+    const NodesBox B(H, G);
+    const long long rows = (long long)B.ny * B.nz;
+    for (long long r = (long long)blockIdx.x * (GN_THREADS / 32) + (threadIdx.x >> 5); r < rows;
+         r += (long long)gridDim.x * (GN_THREADS / 32)) {
+        ulonglong2* row = q + 2 * (((size_t)(B.z0 + r / B.ny) * G.ny + (B.y0 + r % B.ny)) * G.nx + B.x0);
+        for (int i = threadIdx.x & 31; i < 2 * B.nx; i += 32) row[i] = make_ulonglong2(0ull, 0ull);
+    }
+}
+
+// Thread per state.  Consecutive lanes are consecutive z-steps of a stroke: a lane whose cell sits on the next
+// lane's (same column, one layer above) takes over that lane's upper-layer sums, as batch_scatter_kernel does.
+__global__ void __launch_bounds__(GN_THREADS)
+grid_nodes_scatter_kernel(GridView G, int nz_steps, long long n_state, const float4* __restrict__ PPs,
+                          const float4* __restrict__ ubar, const NodesHead* __restrict__ H,
+                          unsigned long long* __restrict__ q) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const long long st = (long long)blockIdx.x * GN_THREADS + threadIdx.x;
+    float4 ub = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (st < n_state) ub = __ldg(ubar + st);
+    bool valid = has_weight(ub);
+    Corners C = {{0, 0}, {0, 0}, {0, 0}, 0.f, 0.f, 0.f, false};
+    if (valid) {
+        const float4 pp = __ldg(PPs + st);
+        C = corners_of<false>(G, mk3(pp.x, pp.y, pp.z));
+        valid = C.ok;
+    }
+    const double scale = pow2(42 - scale_exp(H->umax));
+    const long long stroke = st / nz_steps;
+    auto above = [&](bool v, long long s, int x, int y, int z1) {  // that lane's lower layer is (s, x, y, z1)'s upper
+        return valid && v && s == stroke && x == C.x[0] && y == C.y[0] && z1 == C.z[0];
+    };
+    const bool take = lane < 31 & above(__shfl_down_sync(FULL, valid, 1), __shfl_down_sync(FULL, stroke, 1),
+                                        __shfl_down_sync(FULL, C.x[0], 1), __shfl_down_sync(FULL, C.y[0], 1),
+                                        __shfl_down_sync(FULL, C.z[1], 1));
+    const bool given = __shfl_up_sync(FULL, take, 1) && lane > 0;
+    const float u4[4] = {ub.x, ub.y, ub.z, ub.w};
+    float w[8];
+    size_t node[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+        const int i = c & 1, j = (c >> 1) & 1, k = c >> 2;
+        w[c] = valid ? (i ? C.ax : 1.f - C.ax) * (j ? C.ay : 1.f - C.ay) * (k ? C.az : 1.f - C.az) : 0.f;
+        node[c] = ((size_t)C.z[k] * G.ny + C.y[j]) * G.nx + C.x[i];
+    }
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) {
+        if (__all_sync(FULL, u4[ch] == 0.f)) continue;
+        long long v[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) v[c] = valid ? __double2ll_rn((double)(w[c] * u4[ch]) * scale) : 0ll;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const long long up = __shfl_down_sync(FULL, v[4 + c], 1);
+            if (take) v[c] += up;
+        }
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+            if (valid && !(c >= 4 && given) && v[c] != 0) atomicAdd(q + node[c] * 4 + ch, (unsigned long long)v[c]);
+    }
+}
+
+// CTA c takes the box's 256-node runs c, c + GN_CTAS, ...: their non-zero nodes are compacted into shared
+// memory, thread t owns atom a0 + t % nslot and every P-th staged node; one partial row per (atom, CTA).
+template <int KIND>
+__global__ void __launch_bounds__(GN_THREADS, 3)
+grid_nodes_atoms_kernel(int na, const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
+                        Sites S, NodeGeom NG, GridView G, const NodesHead* __restrict__ H,
+                        const ulonglong2* __restrict__ q, double* __restrict__ partial) {
+    __shared__ float4 s_p[GN_THREADS], s_g[GN_THREADS];
+    __shared__ int s_w[GN_THREADS / 32];
+    __shared__ double red[6][GN_THREADS];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const NodesBox B(H, G);
+    const long long total = B.total();
+    const double inv = pow2(scale_exp(H->umax) - 42);
+    for (int a0 = 0; a0 < na; a0 += GN_THREADS) {
+        const int nslot = min(na - a0, GN_THREADS), P = GN_THREADS / nslot, ph = t / nslot;
+        const bool act = ph < P;
+        const int a = a0 + (act ? t % nslot : 0);
+        const float4 at = __ldg(atoms + a);
+        const float* pr = params + (size_t)a * pstride;
+        const float p1 = __ldg(pr + 0), p2 = __ldg(pr + 1), p3 = (pstride > 2) ? __ldg(pr + 2) : 0.f;
+        // a ubar that is not finite has no fixed-point sum: every gradient is NaN, as the gather's sums would be
+        const double a0_ = H->umax >= 0x7f800000u ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
+        double acc[6] = {a0_, a0_, a0_, a0_, a0_, a0_};
+        for (long long i0 = (long long)blockIdx.x * GN_THREADS; i0 < total; i0 += (long long)GN_CTAS * GN_THREADS) {
+            const long long i = i0 + t;
+            int x = 0, y = 0, z = 0;
+            ulonglong2 lo = make_ulonglong2(0ull, 0ull), hi = lo;
+            if (i < total) {
+                const size_t n = B.node(G, i, x, y, z);
+                lo = __ldg(q + 2 * n);
+                hi = __ldg(q + 2 * n + 1);
+            }
+            const bool nz = (lo.x | lo.y | hi.x | hi.y) != 0ull;
+            const unsigned m = __ballot_sync(0xffffffffu, nz);
+            __syncthreads();  // the previous run's nodes are read
+            if (lane == 0) s_w[warp] = __popc(m);
+            __syncthreads();
+            int at_ = __popc(m & ((1u << lane) - 1u)), n = 0;
+#pragma unroll
+            for (int w = 0; w < GN_THREADS / 32; w++) {
+                if (w < warp) at_ += s_w[w];
+                n += s_w[w];
+            }
+            if (nz) {
+                s_p[at_] = make_float4(NG.p0.x + NG.dA.x * x + NG.dB.x * y + NG.dC.x * z,
+                                       NG.p0.y + NG.dA.y * x + NG.dB.y * y + NG.dC.y * z,
+                                       NG.p0.z + NG.dA.z * x + NG.dB.z * y + NG.dC.z * z, 0.f);
+                s_g[at_] = make_float4((float)((double)(long long)lo.x * inv), (float)((double)(long long)lo.y * inv),
+                                       (float)((double)(long long)hi.x * inv), (float)((double)(long long)hi.y * inv));
+            }
+            __syncthreads();
+            if (act)
+                for (int j = ph; j < n; j += P) {
+                    const float4 p = s_p[j], g = s_g[j];
+                    pair_grad<KIND>(mk3(p.x, p.y, p.z), at, p1, p2, p3, S, mk3(g.x, g.y, g.z), g.w, acc);
+                }
+        }
+#pragma unroll
+        for (int c = 0; c < 6; c++) red[c][t] = act ? acc[c] : 0.0;
+        __syncthreads();
+        for (int k = t; k < nslot * 6; k += GN_THREADS) {
+            const int sl = k / 6, c = k % 6;
+            double v = 0.0;
+            for (int p = 0; p < P; p++) v += red[c][sl + p * nslot];
+            partial[((size_t)(a0 + sl) * GN_CTAS + blockIdx.x) * 6 + c] = v;
+        }
+        __syncthreads();
+    }
+}
+
+// Scratch of spm_adjoint_grid_params_nodes: header, (atom, CTA) partials, dk row sums, the node sums.
+struct NodesScratch {
+    long long part, dk, q, total;
+    NodesScratch(int n_atoms, long long n_state, long long nodes) {
+        part = 64;
+        dk = part + (long long)n_atoms * GN_CTAS * 48;
+        q = (dk + n_rowblocks(n_state) * 32 + 15) / 16 * 16;
+        total = q + nodes * 32;
+    }
+};
+
 constexpr int NM_THREADS = 256;
 constexpr int NM_PER_THREAD = 2;
 constexpr int NM_STAGE = NM_THREADS * NM_PER_THREAD;  // nodes examined per staging pass
@@ -1931,4 +2149,63 @@ extern "C" int spm_adjoint_grid_params(int kind, int n_atoms, const float* atoms
         return set_error(SPM_ERR_CUDA, "spm_adjoint_grid_params: memset failed");
     }
     return check_launch("spm_adjoint_grid_params");
+}
+
+extern "C" long long spm_adjoint_grid_nodes_scratch_bytes(int n_atoms, long long n_state, int nx, int ny, int nz) {
+    using namespace spm;
+    long long nodes = 0;
+    if (n_atoms < 0 || n_state < 0 || nx <= 0 || ny <= 0 || nz <= 0 || !mul_ok((long long)nx * ny, nz, &nodes) ||
+        nodes > (1LL << 56))
+        return 0;
+    return NodesScratch(n_atoms, n_state, nodes).total;
+}
+
+extern "C" int spm_adjoint_grid_params_nodes(int kind, int n_atoms, const float* atoms, const float* params,
+                                             const float* p0, const float* dA, const float* dB, const float* dC,
+                                             const float* Qs, const float* QZs, int nx, int ny, int nz,
+                                             const spm_scan_params* p, const float* PPs, const float* ubar,
+                                             const float* dk, long long n_state, double* grad, double* dk_sum,
+                                             void* scratch, void* stream) {
+    using namespace spm;
+    clear_error();
+    SPM_REQUIRE(kind == SPM_KIND_LJ || kind == SPM_KIND_MORSE, "spm_adjoint_grid_params_nodes: kind=%d", kind);
+    SPM_REQUIRE(n_atoms >= 1 && n_atoms <= 65535, "spm_adjoint_grid_params_nodes: n_atoms=%d outside [1,65535]", n_atoms);
+    SPM_REQUIRE(p && p0 && dA && dB && dC && Qs && QZs && grad && dk_sum && scratch && atoms && params && PPs && ubar && dk,
+                "spm_adjoint_grid_params_nodes: null pointer");
+    SPM_REQUIRE(n_state >= 1 && nx > 0 && ny > 0 && nz > 0 && p->nz > 0, "spm_adjoint_grid_params_nodes: bad sizes");
+    SPM_REQUIRE(aligned16(PPs) && aligned16(ubar) && aligned16(dk) && aligned16(atoms) && aligned16(scratch),
+                "spm_adjoint_grid_params_nodes: buffers not 16-byte aligned");
+    const long long blocks = (n_state + GN_THREADS - 1) / GN_THREADS, rb = n_rowblocks(n_state);
+    SPM_REQUIRE(blocks < (1LL << 31) && spm_adjoint_grid_nodes_scratch_bytes(n_atoms, n_state, nx, ny, nz) > 0,
+                "spm_adjoint_grid_params_nodes: too many states or nodes");
+    Sites S = {};
+    for (int k = 0; k < 4; k++) { S.qs[k] = Qs[k] * COULOMB_CONST; S.qz[k] = QZs[k]; }
+    NodeGeom NG;
+    NG.p0 = make_float4(p0[0], p0[1], p0[2], p0[3]);
+    NG.dA = make_float4(dA[0], dA[1], dA[2], dA[3]);
+    NG.dB = make_float4(dB[0], dB[1], dB[2], dB[3]);
+    NG.dC = make_float4(dC[0], dC[1], dC[2], dC[3]);
+    const NodesScratch L(n_atoms, n_state, (long long)nx * ny * nz);
+    char* base = static_cast<char*>(scratch);
+    NodesHead* H = reinterpret_cast<NodesHead*>(base);
+    double* part = reinterpret_cast<double*>(base + L.part);
+    double* dkpart = reinterpret_cast<double*>(base + L.dk);
+    unsigned long long* q = reinterpret_cast<unsigned long long*>(base + L.q);
+    const float4 *pp4 = reinterpret_cast<const float4*>(PPs), *ub4 = reinterpret_cast<const float4*>(ubar);
+    const float4* a4 = reinterpret_cast<const float4*>(atoms);
+    const int pstride = kind == SPM_KIND_MORSE ? 4 : 2;
+    const GridView G = view_of(nullptr, nx, ny, nz, p);
+    cudaStream_t st = as_stream(stream);
+    if (cudaMemsetAsync(H, 0, sizeof(NodesHead), st) != cudaSuccess)
+        return set_error(SPM_ERR_CUDA, "spm_adjoint_grid_params_nodes: memset failed");
+    grid_nodes_box_kernel<<<(unsigned)(blocks < GN_CTAS ? blocks : GN_CTAS), GN_THREADS, 0, st>>>(G, n_state, pp4, ub4, H);
+    grid_nodes_clear_kernel<<<GN_CTAS, GN_THREADS, 0, st>>>(G, H, reinterpret_cast<ulonglong2*>(q));
+    grid_nodes_scatter_kernel<<<(unsigned)blocks, GN_THREADS, 0, st>>>(G, p->nz, n_state, pp4, ub4, H, q);
+    const auto kern = kind == SPM_KIND_MORSE ? grid_nodes_atoms_kernel<SPM_KIND_MORSE> : grid_nodes_atoms_kernel<SPM_KIND_LJ>;
+    kern<<<GN_CTAS, GN_THREADS, 0, st>>>(n_atoms, a4, params, pstride, S, NG, G, H,
+                                         reinterpret_cast<const ulonglong2*>(q), part);
+    fold_chunks_kernel<<<dim3((unsigned)n_atoms, 6), 256, 0, st>>>(part, GN_CTAS, 6, grad);
+    sum_rows_kernel<<<(unsigned)rb, 256, 0, st>>>(reinterpret_cast<const float4*>(dk), n_state, dkpart);
+    fold_chunks_kernel<<<dim3(1, 4), 256, 0, st>>>(dkpart, (int)rb, 4, dk_sum);
+    return check_launch("spm_adjoint_grid_params_nodes");
 }

@@ -170,6 +170,13 @@ def adjoint_grid_state(grid, params, points, PPs, dL_dFEs):
     return ubar, dk, diag
 
 
+# adjoint_grid_params takes the node-major form from so many (state, atom) pairs on -- 4.4e5 pairs take 108 us
+# either way, 1.2e6 128 us against the gather's 147, 1.5e7 233 against 826 -- on grids whose node sums take up
+# to 2 GB
+NODES_MIN_PAIRS = 1 << 20
+NODES_MAX_GRID = 1 << 26
+
+
 def adjoint_grid_params(kind, atoms, params_atoms, p0, dA, dB, dC, Qs, QZs, grid, scan_params, PPs, ubar, dk):
     """Atom and spring gradients of the grid path -> grad (na,6) f64 (x,y,z,P1,P2,Q), dk (4,) f64."""
     nx, ny, nz = _grid_dims(grid)
@@ -182,9 +189,17 @@ def adjoint_grid_params(kind, atoms, params_atoms, p0, dA, dB, dC, Qs, QZs, grid
     na, n_state = int(atoms.shape[0]), int(PPs.shape[0])
     grad = torch.empty((na, 6), dtype=F64, device=atoms.device)
     dk_sum = torch.empty((4,), dtype=F64, device=atoms.device)
+    hv = [hostvec(v) for v in (p0, dA, dB, dC, Qs, QZs)]
+    if na and n_state * na >= NODES_MIN_PAIRS and scan_params.nz and nx * ny * nz <= NODES_MAX_GRID:
+        nbytes = int(lib().spm_adjoint_grid_nodes_scratch_bytes(na, n_state, nx, ny, nz))
+        scratch = torch.empty(((nbytes + 15) // 16, 2), dtype=F64, device=atoms.device)
+        rc = lib().spm_adjoint_grid_params_nodes(int(kind), na, ptr(atoms), ptr(prm), *[hptr(h) for h in hv], nx, ny, nz,
+                                                 ctypes.byref(scan_params), ptr(PPs), ptr(ubar), ptr(dk), n_state,
+                                                 ptr(grad), ptr(dk_sum), ptr(scratch), stream_ptr())
+        check(rc, "spm_adjoint_grid_params_nodes")
+        return grad, dk_sum
     nbytes = int(lib().spm_adjoint_grid_scratch_bytes(na, n_state))
     scratch = torch.empty((max(nbytes, 8) + 7) // 8, dtype=F64, device=atoms.device)
-    hv = [hostvec(v) for v in (p0, dA, dB, dC, Qs, QZs)]
     rc = lib().spm_adjoint_grid_params(int(kind), na, ptr(atoms) if na else None, ptr(prm) if na else None,
                                        *[hptr(h) for h in hv], ptr(grid), nx, ny, nz, ctypes.byref(scan_params),
                                        ptr(PPs), ptr(ubar), ptr(dk), n_state, ptr(grad), ptr(dk_sum), ptr(scratch),
