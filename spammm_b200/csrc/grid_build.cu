@@ -310,6 +310,7 @@ grid_build_kernel(int na, const float4* __restrict__ atoms, const float* __restr
 constexpr int FB = SPM_FAR_BLOCK;
 constexpr int FP = 8;
 constexpr int FN = FP * FP * FP;
+constexpr int FAR_REF = 3 * 64 + 3 * 8 + 3;  // the point whose value is interpolated as a constant
 constexpr int FAR_CHUNK = 256;       // atoms gathered at a time
 constexpr float FAR_RATIO = 9.f;
 constexpr float FAR_KH = 1.5f;
@@ -574,12 +575,21 @@ __device__ __forceinline__ void build_block(FarShared<NOFF>& M, bool group, int 
             }
             __syncthreads();
         }
+        // the interpolation acts on the differences from one point's value, which is added last: its rounding
+        // is relative to the field's variation over the block, not to the field (error of the FE samples of 100 x
+        // 100 x 40 polished states over a 38-atom molecule, six seeds: 8.6e-7 -> 8.3e-7; 8.0e-7 with direct sums)
+        float4 ref = make_float4(0.f, 0.f, 0.f, 0.f);
         if (field) {  // along x: points (ky, kz) x 16 nodes
+            ref = M.part[0][FAR_REF];
             for (int i = tid; i < FB * FP * FP; i += nthr) {
                 const int x = i & (FB - 1), kk = i >> 4, ky = kk & 7, kz = kk >> 3;
                 float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int k = 0; k < FP; k++) s = fma4(M.tab.L[x][k], M.part[0][kz * 64 + k * 8 + ky], s);
+                for (int k = 0; k < FP; k++) {
+                    const float4 v = M.part[0][kz * 64 + k * 8 + ky];
+                    s = fma4(M.tab.L[x][k], make_float4(__fsub_rn(v.x, ref.x), __fsub_rn(v.y, ref.y),
+                                                        __fsub_rn(v.z, ref.z), __fsub_rn(v.w, ref.w)), s);
+                }
                 stage[i] = s;
             }
             __syncthreads();
@@ -617,6 +627,14 @@ __device__ __forceinline__ void build_block(FarShared<NOFF>& M, bool group, int 
                         fz[p] = fma2(w, vz, fz[p]);
                         fe[p] = fma2(w, ve, fe[p]);
                     }
+                }
+                const f2 rx = bc(ref.x), ry = bc(ref.y), rz = bc(ref.z), re = bc(ref.w);
+#pragma unroll
+                for (int p = 0; p < ZP; p++) {
+                    fx[p] = add2(fx[p], rx);
+                    fy[p] = add2(fy[p], ry);
+                    fz[p] = add2(fz[p], rz);
+                    fe[p] = add2(fe[p], re);
                 }
             }
             for (int c0 = 0; c0 < na; c0 += FAR_CHUNK) {
