@@ -34,16 +34,6 @@ UNIT = "px·z/s"
 # non-zero tip-charge site (the on-node charge's Coulomb law included, although the kernel shares its rsqrt)
 FLOPS_PAIR = {0: 26, 1: 28}
 FLOPS_SITE = 23
-# work the grid-build kernel executes per (node, atom) pair (csrc/grid_build.cu, build_tile's packed
-# f32x2 loop; two nodes per instruction): FP32-pipe lane instructions and flops (FMA = 2), besides one
-# MUFU rsqrt (and one ex2 for Morse).  Pair law with the on-node charge merged (ON): LJ 15 instructions /
-# 23 flops, Morse 16 / 23; without charges: LJ 13 / 20, Morse 13 / 19; each off-node charge site adds
-# 8 / 13 (+1 MUFU).
-EXEC_PAIR = {(0, True): (15, 23), (0, False): (13, 20), (1, True): (16, 23), (1, False): (13, 19)}
-EXEC_SITE = (8, 13)
-# DRAM bytes of one grid_build_kernel launch on the 1200-atom / 480x480x240 workload, from the ncu
-# capture in profiles/grid_build_plain_large.md (dram__bytes_read.sum + dram__bytes_write.sum)
-GRID_BUILD_DRAM_BYTES = 6017024 + 826515456
 
 
 def parse():
@@ -403,46 +393,33 @@ def run_ours(args, rank, world, local_rank):
     peaks = measured_peaks()
     fp32_peak = gpu.fp32_peak_flops(1 << 15)
     ns = int(np.count_nonzero(cfg.tipQs))
-    on = bool(cfg.tipQs[0] != 0 and cfg.tipQZs[0] == 0)  # the kernel merges an on-node site into the pair law
-    n_off = ns - (1 if on else 0)
-    inst_pair = EXEC_PAIR[(cfg.kind, on)][0] + EXEC_SITE[0] * n_off
-    xflops_pair = EXEC_PAIR[(cfg.kind, on)][1] + EXEC_SITE[1] * n_off
-    flops = cfg.pairs * (FLOPS_PAIR[cfg.kind] + FLOPS_SITE * ns)
+    flops = cfg.pairs * (FLOPS_PAIR[cfg.kind] + FLOPS_SITE * ns)  # of the direct sum the build stands for
     ach_fp32 = flops / (stage[0] * 1e-3)
-    # FP32-pipe issue: lane instructions per second against the pipe's peak (the FFMA probe's FLOP/s / 2);
-    # reported as FMA-equivalent TFLOP/s (2 flops per lane instruction) against the probe's peak
-    ach_pipe = cfg.pairs * inst_pair * 2 / (stage[0] * 1e-3)
-    ach_exec = cfg.pairs * xflops_pair / (stage[0] * 1e-3)
     hbm_peak = float(peaks.get("hbm_gbs", 6650.0))
     slab_nodes = nx * ny * (int(np.ceil((cfg.dz * cfg.nz + 2.0) / cfg.step)) + 2)
     relax_bytes = cfg.pxz * 32 + slab_nodes * 16
     ach_relax = relax_bytes / (stage[1] * 1e-3) / 1e9
     df_bytes = cfg.pxz * (16 + 4)
-    names = ["grid_build_kernel", "relax_tile_kernel<0>", "df_amp_dir_kernel"]
+    grid_bytes = nx * ny * cfg.ngrid[2] * 16
+    ach_grid = grid_bytes / (stage[0] * 1e-3) / 1e9
+    names = ["grid_block_kernel", "relax_tile_kernel<0>", "df_amp_z_kernel"]
     dom = int(np.argmax(stage))
-    if dom == 0:
-        roof = {"kernel": names[0], "bound": "fp32 pipe issue", "achieved": ach_pipe / 1e12,
-                "peak": fp32_peak / 1e12, "unit": "TFLOP/s", "frac": ach_pipe / fp32_peak,
-                "traffic": GRID_BUILD_DRAM_BYTES if cfg.name == "plain_large" else None,
-                "traffic_note": "ncu dram__bytes_read.sum + write.sum of one launch (profiles/grid_build_plain_large.md); "
-                                "the grid it writes is 884.7 MB",
-                "peak_source": "measured live: FFMA-chain probe (spm_fp32_peak_probe) on this GPU",
-                "algorithmic": f"{cfg.pairs:.3e} (node,atom) pairs x {inst_pair} FP32 lane instructions as "
-                               f"executed (FMA-equivalent: x2 flops)",
-                "executed_flops": {"per_pair": xflops_pair, "tflops": ach_exec / 1e12, "frac": ach_exec / fp32_peak,
-                                   "note": "FMA = 2, mul/add = 1: the kernel's 15 lane instructions per pair hold "
-                                           "8 FMAs and 7 mul/add"},
-                "laws_counted_in_full": {"per_pair": FLOPS_PAIR[cfg.kind] + FLOPS_SITE * ns,
-                                      "tflops": ach_fp32 / 1e12, "frac": ach_fp32 / fp32_peak,
-                                      "note": "counts the on-node Coulomb law in full; the kernel shares its "
-                                              "rsqrt and radial factor with the pair law, so this exceeds 1"}}
-    else:
-        roof = {"kernel": names[dom], "bound": "hbm", "achieved": ach_relax if dom == 1 else
-                df_bytes / (stage[2] * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s", "traffic": None,
-                "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if "hbm_gbs" in peaks else "fallback"}
-        roof["frac"] = roof["achieved"] / hbm_peak
+    ach = (ach_grid, ach_relax, df_bytes / (stage[2] * 1e-3) / 1e9)[dom]
+    roof = {"kernel": names[dom], "bound": "hbm", "achieved": ach, "peak": hbm_peak, "unit": "GB/s",
+            "frac": ach / hbm_peak, "traffic": None,
+            "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if "hbm_gbs" in peaks else "fallback",
+            "note": ("the grid's bytes, which the build cannot do without; its time goes to FP32 work (near pair "
+                     "sums, the far field at each block's points, the interpolation)",
+                     "the outputs and the sampled slab; the kernel is bound by issue and the FIRE chain",
+                     "volume in, df out")[dom]}
     out.update(stage_ms={"grid_build": stage[0], "relax": stage[1], "df": stage[2]},
-               stage_roofline={"grid_build_pipe_frac": ach_pipe / fp32_peak, "fp32_peak_tflops": fp32_peak / 1e12,
+               stage_roofline={"fp32_peak_tflops": fp32_peak / 1e12,
+                               "grid_build": {"alg_gbs": ach_grid, "alg_hbm_frac": ach_grid / hbm_peak,
+                                              "direct_sum_tflops": ach_fp32 / 1e12,
+                                              "direct_sum_frac": ach_fp32 / fp32_peak,
+                                              "note": "direct_sum: every (node, atom) pair's laws counted in full "
+                                                      "over the build's time; the far field leaves most of those "
+                                                      "pairs out, so this exceeds 1"},
                                "relax": {"bound": "issue / FIRE dependency chain (latency)",
                                          "fire_steps_per_s": steps_total / (stage[1] * 1e-3),
                                          "alg_gbs": ach_relax, "alg_bytes": relax_bytes,
@@ -809,7 +786,7 @@ def run_batched(args, dev_index):
         "px_z_per_s": b.total_states / (ms * 1e-3), "slab_gb": b.grid_float4 * 16 / 1e9,
         "iters_per_state": float(b.iter_count.double().sum()) / b.total_states,
         "converged_frac": float((b.PPs[:, 3] > 0).float().mean()), "clocks": clocks,
-        "gpu_launches_per_step": 3, "grid_layout": "xz-quads" if b.shape.grid_layout else "x-pairs",
+        "gpu_launches_per_step": 4, "grid_layout": "xz-quads" if b.shape.grid_layout else "x-pairs",
         "layout_note": layout_note}
     del gf, b
     torch.cuda.empty_cache()
