@@ -298,8 +298,8 @@ grid_build_kernel(int na, const float4* __restrict__ atoms, const float* __restr
 // nodes a probe reaches (|E| < 0.5 eV), relative to their norm, direct sum -> blocks: 1200 LJ atoms on an
 // ionic slab 1.98e-6 -> 1.89e-6 (energy 2.9e-6 -> 1.7e-6), 57 Morse atoms with offset charges 7.7e-7 -> 7.7e-7.
 //
-// Time, direct sum -> blocks: 1200 atoms on 480 x 480 x 240 nodes 32.0 -> 2.24 ms, 57 Morse atoms with two
-// offset charges on 187 x 203 x 149 442 -> 186 us, 38 atoms on 200^3 211 -> 138 us.  What is left is the near
+// Time, direct sum -> blocks: 1200 atoms on 480 x 480 x 240 nodes 32.0 -> 2.28 ms, 57 Morse atoms with two
+// offset charges on 187 x 203 x 149 426 -> 181 us, 38 atoms on 200^3 187 -> 124 us.  What is left is the near
 // sums (FP32 issue), the far sums and the interpolation in about equal parts.  Below SPM_FAR_MIN_ATOMS most
 // atoms are near most blocks and the interpolation does not pay.
 //
@@ -603,7 +603,7 @@ __device__ __forceinline__ void load_far_tab(FarShared<NOFF>& M, const FarTab& t
 
 // 256 threads, 16 nodes along z each, at 128 registers (two CTAs per SM): 2.24 ms on the 1200-atom 480 x 480
 // x 240 grid (128 threads 2.25, 8 nodes each 2.36; 0.47 ms against 0.71 and 0.44 on 527 atoms, 243 x 138 x
-// 98), 138 us on 38 atoms, 200^3 (128 threads 124).
+// 98); on 38 atoms, 200^3, 128 threads took 10% less.  The differences from one point cost 2% since.
 constexpr int FAR_THREADS = 256;
 constexpr long long FAR_CTAS = 222;  // CTAs that fill a 148-SM part one and a half times
 

@@ -606,31 +606,8 @@ __device__ __forceinline__ void newton_polish(const Fetch& fetch, const float (&
     newton_core(fetch, T, S, tip, q, fe, g2, evals);
 }
 
-// Cell fetcher of a full (nz,ny,nx) grid with any sampling transform (interp_fe's addressing).
-template <typename IDX>
-struct FullCellFetch {
-    const GridView& G;
-    __device__ __forceinline__ bool operator()(V3 p, float& ax, float& ay, float& az, float4 (&t)[8]) const {
-        const float u = __fmaf_rn(p.x, G.dA.x, __fmaf_rn(p.y, G.dA.y, __fmaf_rn(p.z, G.dA.z, G.dA.w)));
-        const float v = __fmaf_rn(p.x, G.dB.x, __fmaf_rn(p.y, G.dB.y, __fmaf_rn(p.z, G.dB.z, G.dB.w)));
-        const float w = __fmaf_rn(p.x, G.dC.x, __fmaf_rn(p.y, G.dC.y, __fmaf_rn(p.z, G.dC.z, G.dC.w)));
-        int x0, x1, y0, y1, z0, z1;
-        bool ok = tex_axis(u, G.nx, x0, x1, ax);
-        ok = tex_axis(v, G.ny, y0, y1, ay) && ok;
-        ok = tex_axis(w, G.nz, z0, z1, az) && ok;
-        if (!ok) return false;
-        const IDX r00 = ((IDX)z0 * G.ny + y0) * G.nx, r10 = ((IDX)z0 * G.ny + y1) * G.nx;
-        const IDX r01 = ((IDX)z1 * G.ny + y0) * G.nx, r11 = ((IDX)z1 * G.ny + y1) * G.nx;
-        t[0] = __ldg(G.g + r00 + x0); t[1] = __ldg(G.g + r00 + x1);
-        t[2] = __ldg(G.g + r10 + x0); t[3] = __ldg(G.g + r10 + x1);
-        t[4] = __ldg(G.g + r01 + x0); t[5] = __ldg(G.g + r01 + x1);
-        t[6] = __ldg(G.g + r11 + x0); t[7] = __ldg(G.g + r11 + x1);
-        return true;
-    }
-};
-
-// FullCellFetch through the lane's TexelCache: the cell FIRE ended in, or the previous evaluation's, needs
-// no loads.  The same texels either way.
+// Cell fetcher of a full (nz,ny,nx) grid with any sampling transform, through the lane's TexelCache: the
+// cell FIRE ended in, or the previous evaluation's, needs no loads.
 template <typename IDX, bool AXIS>
 struct FullCellFetchCached {
     const GridView& G;
