@@ -795,7 +795,7 @@ def run_batched(args, dev_index):
 
 def run_reference(args, rank, world):
     """The reference's CPU implementation of the path on the host cores: the reference itself is
-    PyOpenCL and neither this image nor the GPU boxes have an OpenCL platform (clGetPlatformIDs
+    PyOpenCL and neither this image nor the GPU hosts have an OpenCL platform (clGetPlatformIDs
     returns -1001, no ICD under /etc/OpenCL/vendors, no pyopencl), so the arm times the oracle's
     C/OpenMP restatement of its kernels, on every host thread, one bounded proportional sample
     (CpuSample) per step.  Under torchrun only rank 0 runs."""
@@ -821,7 +821,7 @@ def run_reference(args, rank, world):
             "config": dict(config_dict(cfg, "CPU"), sample=det["sample"]), "impl": "reference",
             "cpu_baseline": det,
             "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-            "note": "the reference's path is PyOpenCL and no OpenCL platform exists on this image or the GPU box "
+            "note": "the reference's path is PyOpenCL and no OpenCL platform exists on this image or the GPU host "
                     "(probed: no pyopencl, clGetPlatformIDs -1001); this arm times the C/OpenMP restatement of "
                     "its kernels on the host cores, per step a bounded proportional sample of the workload"}
 

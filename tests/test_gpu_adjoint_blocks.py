@@ -21,10 +21,9 @@ def _items(kind, counts, seed):
     return out
 
 
-def _grads(items, kind, chunk=None):
+def _grads(items, kind, chunk=1024):
     shape = _lib.BatchShape(*_lib.lib().spm_batch_default_shape().key())
-    if chunk:
-        shape.adj_chunk = chunk
+    shape.adj_chunk = chunk  # small units: enough of them for the blocks
     b = AFMBatch(items, kind=kind, shape=shape)
     rng = np.random.default_rng(4)
     for i, it in enumerate(b.items):
@@ -56,11 +55,11 @@ def test_matches_state_major(cuda, kind, counts, monkeypatch):
 def test_repeats_and_unit_counts(cuda):
     """The same bits call after call (the adjoint grid is left cleared); more or fewer units per molecule than
     lattice cells group the same sums differently."""
-    items = _items(0, (40, 90), seed=3)
+    items = _items(0, (40, 64, 90, 120), seed=3)
     b = _grads(items, 0)
     first = b.grad.clone()
     b.forward_adjoint()
     torch.cuda.synchronize()
     assert torch.equal(first, b.grad)
-    for chunk in (1024, 1 << 20):
+    for chunk in (2048,):
         torch.testing.assert_close(_grads(items, 0, chunk).grad, first, rtol=1e-6, atol=1e-7 * float(first.abs().max()))
