@@ -78,38 +78,67 @@ __device__ __forceinline__ double group_sum(double v, unsigned gmask) {
     return v;
 }
 
-template <int NS, int LPP>
+// group_sum of two values per lane, taken as the lanes sub and sub + LPP of a group twice as wide: the sum that
+// group has, bit for bit, by as many shuffles (even lanes go on with the lower half's sum, odd lanes with the
+// upper half's; the last exchange adds the two).
+template <int LPP>
+__device__ __forceinline__ float group_sum_halves(float lo, float hi, int sub, unsigned gmask) {
+    const bool odd = sub & 1;
+    const float other = __shfl_xor_sync(gmask, odd ? lo : hi, 1);
+    float v = (odd ? hi : lo) + other;
+#pragma unroll
+    for (int o = 2; o < LPP; o <<= 1) v += __shfl_xor_sync(gmask, v, o);
+    return v + __shfl_xor_sync(gmask, v, 1);
+}
+
+// Atom j's terms added to (fx, fy, fz, fe).
+template <int NS>
+__device__ __forceinline__ void add_pair(float4& f, V3 p, int j, int na, const float4* s_pos, const float4* s_m,
+                                         const float* s_q, const float* qz) {
+    const float4 a = s_pos[j];
+    const float4 m = s_m[j];
+    const float dx = p.x - a.x, dy = p.y - a.y, dz = p.z - a.z;
+    const float dxy2 = fmaf(dx, dx, fmaf(dy, dy, R2SAFE));
+    const float r2 = fmaf(dz, dz, dxy2);
+    const float rs = fast_rsqrt(r2);
+    const float r = r2 * rs;
+    const float e = fast_ex2(fmaf(m.x, r, m.y));
+    f.w = fmaf(m.z * e, e - 2.f, f.w);
+    const float sg = (m.w * e) * (e - 1.f) * rs;
+    f.x = fmaf(dx, sg, f.x);
+    f.y = fmaf(dy, sg, f.y);
+    f.z = fmaf(dz, sg, f.z);
+#pragma unroll
+    for (int k = 0; k < NS; k++) {
+        const float dzk = dz + qz[k];
+        const float rsk = fast_rsqrt(fmaf(dzk, dzk, dxy2));
+        const float Ek = s_q[k * na + j] * rsk;
+        f.w += Ek;
+        const float sk = Ek * rsk * rsk;
+        f.x = fmaf(dx, sk, f.x);
+        f.y = fmaf(dy, sk, f.y);
+        f.z = fmaf(dzk, sk, f.z);
+    }
+}
+
+// The pair sums at p.  HALVES = 2: each lane keeps the two partial sums of the lanes sub and sub + LPP of a
+// group of 2 LPP, so a scan's bits do not depend on which of the two widths the launch takes.
+template <int NS, int LPP, int HALVES>
 __device__ __forceinline__ float4 group_pair_sum(V3 p, int na, int sub, unsigned gmask, const float4* s_pos,
                                                  const float4* s_m, const float* s_q, const float* qz) {
-    float fx = 0.f, fy = 0.f, fz = 0.f, fe = 0.f;
-    for (int j = sub; j < na; j += LPP) {
-        const float4 a = s_pos[j];
-        const float4 m = s_m[j];
-        const float dx = p.x - a.x, dy = p.y - a.y, dz = p.z - a.z;
-        const float dxy2 = fmaf(dx, dx, fmaf(dy, dy, R2SAFE));
-        const float r2 = fmaf(dz, dz, dxy2);
-        const float rs = fast_rsqrt(r2);
-        const float r = r2 * rs;
-        const float e = fast_ex2(fmaf(m.x, r, m.y));
-        fe = fmaf(m.z * e, e - 2.f, fe);
-        const float sg = (m.w * e) * (e - 1.f) * rs;
-        fx = fmaf(dx, sg, fx);
-        fy = fmaf(dy, sg, fy);
-        fz = fmaf(dz, sg, fz);
-#pragma unroll
-        for (int k = 0; k < NS; k++) {
-            const float dzk = dz + qz[k];
-            const float rsk = fast_rsqrt(fmaf(dzk, dzk, dxy2));
-            const float Ek = s_q[k * na + j] * rsk;
-            fe += Ek;
-            const float sk = Ek * rsk * rsk;
-            fx = fmaf(dx, sk, fx);
-            fy = fmaf(dy, sk, fy);
-            fz = fmaf(dzk, sk, fz);
-        }
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (HALVES == 1) {
+        for (int j = sub; j < na; j += LPP) add_pair<NS>(f, p, j, na, s_pos, s_m, s_q, qz);
+        return make_float4(group_sum<LPP>(f.x, gmask), group_sum<LPP>(f.y, gmask), group_sum<LPP>(f.z, gmask),
+                           group_sum<LPP>(f.w, gmask));
     }
-    return make_float4(group_sum<LPP>(fx, gmask), group_sum<LPP>(fy, gmask), group_sum<LPP>(fz, gmask),
-                       group_sum<LPP>(fe, gmask));
+    float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = sub; j < na; j += 2 * LPP) {
+        add_pair<NS>(f, p, j, na, s_pos, s_m, s_q, qz);
+        if (j + LPP < na) add_pair<NS>(h, p, j + LPP, na, s_pos, s_m, s_q, qz);
+    }
+    return make_float4(group_sum_halves<LPP>(f.x, h.x, sub, gmask), group_sum_halves<LPP>(f.y, h.y, sub, gmask),
+                       group_sum_halves<LPP>(f.z, h.z, sub, gmask), group_sum_halves<LPP>(f.w, h.w, sub, gmask));
 }
 
 // |total force|^2 at p in FP64 -- the Morse + Coulomb sums from the atoms' float32 inputs with IEEE
@@ -212,7 +241,7 @@ __device__ __noinline__ float group_force_bound(V3 p, V3 tip, int na, int sub, u
 // more than its error bound, where FP64 cannot decide otherwise (most confirmations of molecules; beyond
 // BOUND_ATOMS atoms the bound of the sum's rounding nears the threshold and is not tried).  38 atoms, 100 x
 // 100 pixels x 40 z-steps, at 16 lanes per pixel: 1686 -> 1405 us.  ident: the tip frame is x, y, z (the rotations change no value).
-template <int NS, int LPP>
+template <int NS, int LPP, int HALVES>
 __global__ void __launch_bounds__(DX_THREADS)
 relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __restrict__ cMs,
                     const float4* __restrict__ pts, int n_scan, spm_scan_params P, Sites S,
@@ -256,7 +285,7 @@ relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __re
         float4 fe = make_float4(0.f, 0.f, 0.f, 0.f);
         if (it < P.max_iter) {
             ++it;
-            fe = group_pair_sum<NS, LPP>(pos, na, sub, gmask, s_pos, s_m, s_q, S.qz);
+            fe = group_pair_sum<NS, LPP, HALVES>(pos, na, sub, gmask, s_pos, s_m, s_q, S.qz);
             const V3 d = sub3(pos, tip);
             const V3 ft = ident ? tip_force(d, kk, d0) : rotmatT(tip_force(rotmat(d, a, b, c), kk, d0), a, b, c);
             V3 f = mk3(fe.x + ft.x, fe.y + ft.y, fe.z + ft.z);
@@ -289,7 +318,7 @@ relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __re
             done = true;  // max_iter == 0
         }
         if (done) {
-            if (!conv) fe = group_pair_sum<NS, LPP>(pos, na, sub, gmask, s_pos, s_m, s_q, S.qz);  // moved since
+            if (!conv) fe = group_pair_sum<NS, LPP, HALVES>(pos, na, sub, gmask, s_pos, s_m, s_q, S.qz);  // moved since
             if (sub == 0) {
                 const V3 r = rotmat(mk3(fe.x, fe.y, fe.z), a, b, c);
                 fe_out[iz] = make_float4(r.x, r.y, r.z, fe.w);
@@ -603,13 +632,11 @@ Sites make_sites(const float* Qs, const float* QZs, bool compact, int* ns) {
     return S;
 }
 
-// Lanes per pixel: about eight atoms per lane, at least 4 and at most 32 lanes, more while the scan
-// leaves the GPU short of warps (fewer than ~8 warps per SM of a 148-SM part).  38 atoms, 100 x 100 pixels x 40
-// z-steps: four atoms per lane (16 lanes) 1405 us, eight (8 lanes) 1193, sixteen (4 lanes, two warps per
-// scheduler) 1850; with 64 x 50 pixels half as many warps cost 638 us against 466.
-int direct_lpp(int na, int n_scan) {
+// Lanes per pixel of a scan: `atoms` atoms per lane, at least 4 and at most 32 lanes, more while the scan
+// leaves the GPU short of warps (fewer than ~8 warps per SM of a 148-SM part).
+int direct_lpp(int na, int n_scan, int atoms) {
     int lpp = 4;
-    while (lpp < 32 && lpp * 8 < na) lpp *= 2;
+    while (lpp < 32 && lpp * atoms < na) lpp *= 2;
     while (lpp < 32 && (long long)n_scan * lpp < 148LL * 8 * 32) lpp *= 2;
     return lpp;
 }
@@ -618,9 +645,17 @@ template <int NS>
 int launch_direct(int na, const float* atoms, const float* cMs, const float* points, int n_scan,
                   const spm_scan_params& P, const Sites& S, float* FEs, float* PPs, cudaStream_t st) {
     const size_t smem = (size_t)na * (2 * sizeof(float4) + NS * sizeof(float));
-    const int lpp = direct_lpp(na, n_scan);
-    auto kern = lpp == 4 ? relax_direct_kernel<NS, 4> : lpp == 8 ? relax_direct_kernel<NS, 8>
-              : lpp == 16 ? relax_direct_kernel<NS, 16> : relax_direct_kernel<NS, 32>;
+    // The order of the atom sums is that of four atoms per lane (unpolished strokes stop elsewhere within their
+    // threshold in another order); the launch takes eight, half the lanes with two partial sums each.  38 atoms,
+    // 100 x 100 pixels x 40 z-steps: 16 lanes per pixel 1405 us, 8 lanes in this order 1247 (1163 in their own
+    // order), 4 lanes 1850 (two warps per scheduler); with 64 x 50 pixels half as many warps cost 638 us
+    // against 466.
+    const int lpp = direct_lpp(na, n_scan, 8);
+    const bool two = direct_lpp(na, n_scan, 4) != lpp;  // twice as many then
+    auto kern = lpp == 4    ? (two ? relax_direct_kernel<NS, 4, 2> : relax_direct_kernel<NS, 4, 1>)
+                : lpp == 8  ? (two ? relax_direct_kernel<NS, 8, 2> : relax_direct_kernel<NS, 8, 1>)
+                : lpp == 16 ? (two ? relax_direct_kernel<NS, 16, 2> : relax_direct_kernel<NS, 16, 1>)
+                            : relax_direct_kernel<NS, 32, 1>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return set_error(SPM_ERR_CUDA, "spm_relax_direct_morse: smem %zu B: %s", smem,
