@@ -41,7 +41,6 @@
 #include "spm_internal.cuh"
 #include "spm_fire.cuh"
 #include "spm_batch.cuh"
-#include "spm_far.cuh"
 
 namespace spm {
 namespace {
@@ -1303,35 +1302,6 @@ struct AtomC {
     float q;         // Q
 };
 
-template <int KIND>
-__device__ __forceinline__ AtomC node_atom(const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
-                                           const NodeSites& S, int ga) {
-    const float4 at = __ldg(atoms + ga);
-    const float* pr = params + (size_t)ga * pstride;
-    const float p1 = __ldg(pr + 0), p2 = __ldg(pr + 1), p3 = (pstride > 2) ? __ldg(pr + 2) : 0.f;
-    AtomC C;
-    C.x = bc(at.x);
-    C.y = bc(at.y);
-    C.z = bc(at.z);
-    C.q = at.w;
-    C.qw = bc(at.w * S.qon);
-    C.qw3 = bc(3.f * (at.w * S.qon));
-    if (KIND == SPM_KIND_LJ) {  // p1 = c6, p2 = c12
-        C.c0 = bc(12.f * p2);
-        C.c1 = bc(-6.f * p1);
-        C.c2 = bc(168.f * p2);
-        C.c3 = bc(-48.f * p1);
-        C.c4 = bc(0.f);
-    } else {  // p1 = R0, p2 = E0, p3 = K
-        C.c0 = bc(p3 * LOG2E);
-        C.c1 = bc(-p3 * p1 * LOG2E);
-        C.c2 = bc(-2.f * p3 * p2);
-        C.c3 = bc(2.f * p3 * p3 * p2);
-        C.c4 = bc(-2.f * p3);
-    }
-    return C;
-}
-
 // Derivatives of the pair laws of the grid build (LJ / Morse + point-charge
 // Coulomb, R2SAFE-softened, as pair_grad) at two nodes per call, contracted
 // with the nodes' adjoint vectors g = (gx,gy,gz,gw):
@@ -1452,10 +1422,6 @@ __device__ __forceinline__ bool nm_try_wait(unsigned bar, unsigned parity) {
     return ok != 0;
 }
 
-// Molecules whose adjoint goes through blocks with a far field.
-constexpr int BLK_MAX_ATOMS = 256;
-__device__ __forceinline__ bool in_blocks(int na) { return na >= SPM_FAR_MIN_ATOMS && na <= BLK_MAX_ATOMS; }
-
 // CTA per node unit (molecule, `chunk` consecutive slab nodes).  Non-zero
 // adjoint-grid nodes are compacted into shared memory (one float array per
 // component, so nodes 2i and 2i+1 load as one packed pair); thread t owns atom
@@ -1482,7 +1448,7 @@ batch_adjoint_nodes_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, in
                            const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
                            NodeSites S, unsigned long long* __restrict__ gq, const int* __restrict__ box,
                            const unsigned* __restrict__ umax, double* __restrict__ partial,
-                           unsigned* __restrict__ status, bool blocks) {
+                           unsigned* __restrict__ status) {
     static_assert(!BULK || ILP == 1, "bulk-copy staging with one node pair per step");
     constexpr int APT = ILP == 3 ? 2 : 1;  // atoms per thread
     extern __shared__ __align__(16) unsigned char nm_smem[];
@@ -1506,7 +1472,6 @@ batch_adjoint_nodes_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, in
     const long long unit = blockIdx.x;
     const int m = SPM_MOL_BY(unit_off, mols, n_mol, unit);
     const spm_batch_mol* D = mols + m;
-    if (blocks && in_blocks(D->n_atoms)) return;  // batch_adjoint_blocks_kernel's molecule
     const long long lc = unit - D->unit_off;
     // slab pitches (stored columns, rows) and the stored box's corner in the full grid
     const int nx = D->nx_slab, ny = D->ny_slab, x_lo = D->x_lo, y_lo = D->y_lo, z_lo = D->z_lo;
@@ -1534,7 +1499,32 @@ batch_adjoint_nodes_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, in
     };
     // ILP = 3: the second atom's FP64 sums (red2[c][t]), after the shared arrays
     double(*red2)[NM_THREADS] = reinterpret_cast<double(*)[NM_THREADS]>(nm_smem + (NM_SMEM + 15) / 16 * 16);
-    auto atom_consts = [&](int ga) { return node_atom<KIND>(atoms, params, pstride, S, ga); };
+    auto atom_consts = [&](int ga) {
+        const float4 at = __ldg(atoms + ga);
+        const float* pr = params + (size_t)ga * pstride;
+        const float p1 = __ldg(pr + 0), p2 = __ldg(pr + 1), p3 = (pstride > 2) ? __ldg(pr + 2) : 0.f;
+        AtomC C;
+        C.x = bc(at.x);
+        C.y = bc(at.y);
+        C.z = bc(at.z);
+        C.q = at.w;
+        C.qw = bc(at.w * S.qon);
+        C.qw3 = bc(3.f * (at.w * S.qon));
+        if (KIND == SPM_KIND_LJ) {  // p1 = c6, p2 = c12
+            C.c0 = bc(12.f * p2);
+            C.c1 = bc(-6.f * p1);
+            C.c2 = bc(168.f * p2);
+            C.c3 = bc(-48.f * p1);
+            C.c4 = bc(0.f);
+        } else {  // p1 = R0, p2 = E0, p3 = K
+            C.c0 = bc(p3 * LOG2E);
+            C.c1 = bc(-p3 * p1 * LOG2E);
+            C.c2 = bc(-2.f * p3 * p2);
+            C.c3 = bc(2.f * p3 * p3 * p2);
+            C.c4 = bc(-2.f * p3);
+        }
+        return C;
+    };
     for (int a0 = 0, nag = 0; a0 < na; a0 += nag) {
         // atom group: nslot thread slots x P phases <= 256 threads, APT atoms per slot (slot s takes atoms
         // a0 + s and a0 + nslot + s).  The remaining atoms go in one group when that keeps >= 85% of the
@@ -1838,293 +1828,6 @@ batch_adjoint_nodes_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, in
     }
 }
 
-// The adjoint of a force grid built in blocks (grid_build.cu): a block's adjoint nodes act on its near atoms
-// node by node, and on its far atoms through the block's 8^3 Chebyshev points -- the transpose of the
-// interpolation sums the nodes' adjoint vectors onto the points (along x, y, z in turn), and the pair
-// derivatives are evaluated at 512 points instead of up to 4096 nodes.
-// Bound: the FP32 pair terms (near atoms take 3/4 of them).  64 molecules of 10..120 atoms: 7.6 ms for
-// batch_adjoint_nodes_kernel, 5.7 + 0.4 ms for the small ones in the nodes kernel (fitting step 23.3 -> 21.7 ms).
-//
-// ADJ_FAR: the position derivatives carry one more power of 1/r than the build's field, so its ratio of 9
-// would leave a larger error than the node sums' rounding: rms of the x column against IEEE pair terms summed
-// in 64 bits 1.6e-7 node by node, 2.1e-7 at a ratio of 9 (20.7 ms per step), 1.8e-7 at 12, 1.6e-7 at 13
-// (22.3 ms); over four batches the columns move by -20% to +10% at 12, either way at rounding level.
-//
-// The slab's lattice cells are dealt round-robin to the molecule's node units, so a CTA writes the same
-// (unit, atom) partial rows as batch_adjoint_nodes_kernel, in a fixed order.  Both passes over a block read
-// its nodes from global memory (the second from L2), and nodes are zeroed as they are staged for the near
-// atoms.  Two CTAs per SM at 128 registers: three at 80 spill 364 B (fitting step 0.8 ms longer).
-constexpr float ADJ_FAR = 12.f;
-constexpr int ADJ_FAR_ROWS = 40;  // fewer non-zero rows of 16 nodes than this: 512 points save nothing
-struct BlkShared {
-    float n[7][NM_BUF];            // staged nodes or points: x, y, z, gx, gy, gz, gw
-    float4 a[FB * FB * FP];        // sums along x, then y in place; the phases' FP64 sums afterwards
-    double acc[6][BLK_MAX_ATOMS];  // the unit's sums per atom
-    int far[BLK_MAX_ATOMS], near[BLK_MAX_ATOMS];
-    float L[FB][FP], c[FP];
-    int warp[3][NM_THREADS / 32];  // two staging passes' counts, the far atoms'
-};
-static_assert(sizeof(float4) * FB * FB * FP >= 6 * NM_THREADS * sizeof(double), "the phase sums fit");
-
-template <int KIND, bool ON, bool PAR>
-__global__ void __launch_bounds__(NM_THREADS, 2)
-batch_adjoint_blocks_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, int chunk,
-                            const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
-                            NodeSites S, unsigned long long* __restrict__ gq, const int* __restrict__ box,
-                            const unsigned* __restrict__ umax, double* __restrict__ partial,
-                            const __grid_constant__ FarTab tab) {
-    extern __shared__ __align__(16) unsigned char nm_smem[];
-    BlkShared& M = *reinterpret_cast<BlkShared*>(nm_smem);
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int m = SPM_MOL_BY(unit_off, mols, n_mol, (long long)blockIdx.x);
-    const spm_batch_mol* D = mols + m;
-    const int na = D->n_atoms, ao = D->atom_off;
-    if (!in_blocks(na)) return;
-    const int nx = D->nx_slab, ny = D->ny_slab, nz = D->nz_slab, x_lo = D->x_lo, y_lo = D->y_lo, z_lo = D->z_lo;
-    const long long slab = (long long)nx * ny * nz;
-    const int units = (int)((slab + chunk - 1) / chunk), lc = (int)(blockIdx.x - D->unit_off);
-    NodeGeom NG;
-    NG.p0 = ld4f(D->p0);
-    NG.dA = ld4f(D->dA);
-    NG.dB = ld4f(D->dB);
-    NG.dC = ld4f(D->dC);
-    const double inv = pow2(scale_exp(__ldg(umax + m)) - 42);
-    ulonglong2* q2 = reinterpret_cast<ulonglong2*>(gq + (size_t)D->grid_off * 4);
-    const int ylo = ny - 1 - box[4 * m], yhi = box[4 * m + 1] - 1;  // touched rows and layers (empty: yhi < 0)
-    const int zlo = nz - 1 - box[4 * m + 2], zhi = box[4 * m + 3] - 1;
-    if (t < FB * FP) M.L[t / FP][t % FP] = tab.L[t / FP][t % FP];
-    if (t < FP) M.c[t] = tab.c[t];
-#pragma unroll
-    for (int c = 0; c < 6; c++) M.acc[c][t] = 0.0;
-
-    // adds the L staged nodes' derivatives for the listed atoms (n > 0) to the unit's sums
-    auto compute = [&](int L, const int* list, int n) {
-        if (t == 0 && (L & 1)) {  // pad to whole pairs: a distant node of zero weight adds +-0
-#pragma unroll
-            for (int c = 0; c < 7; c++) M.n[c][L] = c < 3 ? 1e4f : 0.f;
-        }
-        __syncthreads();
-        const int P = NM_THREADS / n, ph = t / n;
-        double sum[6] = {0, 0, 0, 0, 0, 0};
-        if (ph < P) {
-            const AtomC C = node_atom<KIND>(atoms, params, pstride, S, ao + list[t % n]);
-            const f2 zero = bc(0.f);
-            f2 a32[6] = {zero, zero, zero, zero, zero, zero};
-            const int Lp = (L + 1) >> 1, step = 2 * P;
-            const float* sp = &M.n[0][2 * ph];
-            int left = ph < Lp ? (Lp - ph + P - 1) / P : 0;
-            while (left > 0) {
-                const int nb = min(NM_FLUSH / 2, left);
-#pragma unroll 4
-                for (int k = 0; k < nb; k++, sp += step)
-                    pair_adj2<KIND, ON, PAR>(lds2(sp), lds2(sp + NM_BUF), lds2(sp + 2 * NM_BUF), lds2(sp + 3 * NM_BUF),
-                                             lds2(sp + 4 * NM_BUF), lds2(sp + 5 * NM_BUF), lds2(sp + 6 * NM_BUF), C, S,
-                                             a32);
-                left -= nb;
-                fold_sums<PAR>(a32, sum, 1);
-            }
-        }
-        double(*red)[NM_THREADS] = reinterpret_cast<double(*)[NM_THREADS]>(M.a);
-#pragma unroll
-        for (int c = 0; c < 6; c++) red[c][t] = sum[c];
-        __syncthreads();
-        for (int k = t; k < 6 * n; k += NM_THREADS) {
-            const int c = k / n, sl = k - c * n;
-            double v = 0.0;
-            for (int p = 0; p < P; p++) v += red[c][sl + p * n];
-            M.acc[c][list[sl]] += v;
-        }
-        __syncthreads();  // the staged nodes and the phase sums are reused
-    };
-    const int cx0 = x_lo / FB, cy0 = y_lo / FB, cz0 = z_lo / FB;
-    const int ncx = (x_lo + nx - 1) / FB - cx0 + 1, ncy = (y_lo + ny - 1) / FB - cy0 + 1;
-    const int cells = ncx * ncy * ((z_lo + nz - 1) / FB - cz0 + 1);
-    for (int cell = lc; cell < cells; cell += units) {
-        // the block's first node, as a slab index (may be negative at the box's lower edges)
-        const int bx = (cx0 + cell % ncx) * FB - x_lo, by = (cy0 + cell / ncx % ncy) * FB - y_lo;
-        const int bz = (cz0 + cell / ncx / ncy) * FB - z_lo;
-        if (yhi < 0 || by > yhi || by + FB <= ylo || bz > zhi || bz + FB <= zlo) continue;  // CTA-uniform
-        // near and far atoms, in atom order
-        const FarCube C = far_cube(NG, bx + x_lo, by + y_lo, bz + z_lo, FB, ADJ_FAR);
-        bool far = false;
-        if (t < na) {
-            const float4 a = __ldg(atoms + ao + t);
-            const float dx = C.x - a.x, dy = C.y - a.y, dz = C.z - a.z, dxy2 = fmaf(dy, dy, dx * dx);
-            far = fmaf(dz, dz, dxy2) >= C.lim2;
-            for (int k = 0; k < S.noff; k++) {
-                const float dk = dz + S.qz[k];
-                far = far && fmaf(dk, dk, dxy2) >= C.lim2;
-            }
-            if (KIND == SPM_KIND_MORSE)
-                far = far && fabsf(__ldg(params + (size_t)(ao + t) * pstride + 2)) * C.h <= FAR_KH;
-        }
-        int nf = __syncthreads_count(far);
-        if (nf < FAR_FEWEST) {
-            far = false;
-            nf = 0;
-        }
-        int nn = na - nf;
-        const unsigned fm = __ballot_sync(0xffffffffu, far);
-        if (lane == 0) M.warp[2][warp] = __popc(fm);
-        __syncthreads();
-        if (t < na) {
-            int f = __popc(fm & ((1u << lane) - 1u));  // far atoms before this one
-            for (int w = 0; w < warp; w++) f += M.warp[2][w];
-            if (far) M.far[f] = t;
-            else M.near[t - f] = t;
-        }
-        if (nf > 0) {
-            // along x: thread t = the row (y, z) of the block
-            const int yl = by + (t & 15), zl = bz + (t >> 4);
-            const bool row = (unsigned)yl < (unsigned)ny && (unsigned)zl < (unsigned)nz;
-            float4 o[FP];
-#pragma unroll
-            for (int k = 0; k < FP; k++) o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            bool any = false;
-            if (row) {
-                const ulonglong2* r = q2 + 2 * (((long long)zl * ny + yl) * nx + bx);
-#pragma unroll 4
-                for (int x = 0; x < FB; x++) {
-                    if ((unsigned)(bx + x) >= (unsigned)nx) continue;
-                    const ulonglong2 lo = r[2 * x], hi = r[2 * x + 1];
-                    if ((lo.x | lo.y | hi.x | hi.y) == 0ull) continue;
-                    any = true;
-                    const float4 g = make_float4((float)((double)(long long)lo.x * inv), (float)((double)(long long)lo.y * inv),
-                                                 (float)((double)(long long)hi.x * inv), (float)((double)(long long)hi.y * inv));
-#pragma unroll
-                    for (int k = 0; k < FP; k++) {
-                        const float w = M.L[x][k];
-                        o[k] = make_float4(fmaf(w, g.x, o[k].x), fmaf(w, g.y, o[k].y), fmaf(w, g.z, o[k].z),
-                                           fmaf(w, g.w, o[k].w));
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < FP; k++) M.a[k * FB * FB + t] = o[k];  // (kx, z, y)
-            const int rows = __syncthreads_count(any);
-            if (rows == 0) continue;  // nothing to do in this block
-            if (rows < ADJ_FAR_ROWS) {
-                if (t < na) M.near[t] = t;  // read after a staging pass' barrier
-                nn = na;
-            } else {
-                float* af = reinterpret_cast<float*>(M.a);
-                // along y, in place: one (kx, z, channel) column of 16 y per item, its 8 sums into the first slots
-                for (int i = t; i < FP * FB * 4; i += NM_THREADS) {
-                    float* col = af + (size_t)(i >> 2) * FB * 4 + (i & 3);
-                    float v[FB];
-#pragma unroll
-                    for (int y = 0; y < FB; y++) v[y] = col[4 * y];
-#pragma unroll
-                    for (int k = 0; k < FP; k++) {
-                        float w = 0.f;
-#pragma unroll
-                        for (int y = 0; y < FB; y++) w = fmaf(M.L[y][k], v[y], w);
-                        col[4 * k] = w;
-                    }
-                }
-                __syncthreads();
-                // along z: thread t = (kx, ky, channel); the points staged as nodes (kz*64 + kx*8 + ky)
-                {
-                    const int ch = t & 3, ky = (t >> 2) & 7, kx = t >> 5;
-                    float v[FB];
-#pragma unroll
-                    for (int z = 0; z < FB; z++) v[z] = af[((size_t)(kx * FB + z) * FB + ky) * 4 + ch];
-#pragma unroll
-                    for (int k = 0; k < FP; k++) {
-                        float w = 0.f;
-#pragma unroll
-                        for (int z = 0; z < FB; z++) w = fmaf(M.L[z][k], v[z], w);
-                        M.n[3 + ch][k * 64 + kx * 8 + ky] = w;
-                    }
-                }
-                for (int i = t; i < FN; i += NM_THREADS) {
-                    const float ux = C.half * M.c[(i >> 3) & 7], uy = C.half * M.c[i & 7], uz = C.half * M.c[i >> 6];
-                    M.n[0][i] = fmaf(NG.dB.x, uy, fmaf(NG.dA.x, ux, C.x));
-                    M.n[1][i] = fmaf(NG.dB.y, uy, fmaf(NG.dA.y, ux, C.y));
-                    M.n[2][i] = fmaf(NG.dC.z, uz, fmaf(NG.dB.z, uy, fmaf(NG.dA.z, ux, C.z)));
-                }
-                compute(FN, M.far, nf);  // begins with a barrier
-            }
-        }
-        // the nodes, NM_STAGE at a time: compacted for the near atoms and zeroed
-        int staged = 0;
-        for (int b0 = 0, pass = 0; b0 <= FB * FB * FB; b0 += NM_STAGE, pass++) {
-            if (b0 < FB * FB * FB) {
-                ulonglong2 lo[NM_PER_THREAD], hi[NM_PER_THREAD];
-                bool nzr[NM_PER_THREAD];
-                int cnt = 0;
-#pragma unroll
-                for (int r = 0; r < NM_PER_THREAD; r++) {
-                    const int i = b0 + r * NM_THREADS + t, xl = bx + (i & 15), yl = by + ((i >> 4) & 15), zl = bz + (i >> 8);
-                    lo[r] = make_ulonglong2(0ull, 0ull);
-                    hi[r] = lo[r];
-                    if ((unsigned)xl < (unsigned)nx && (unsigned)yl < (unsigned)ny && (unsigned)zl < (unsigned)nz) {
-                        ulonglong2* qn = q2 + 2 * (((long long)zl * ny + yl) * nx + xl);
-                        lo[r] = qn[0];
-                        hi[r] = qn[1];
-                        if ((lo[r].x | lo[r].y | hi[r].x | hi[r].y) != 0ull) {
-                            qn[0] = make_ulonglong2(0ull, 0ull);
-                            qn[1] = make_ulonglong2(0ull, 0ull);
-                        }
-                    }
-                    nzr[r] = (lo[r].x | lo[r].y | hi[r].x | hi[r].y) != 0ull;
-                    cnt += nzr[r] ? 1 : 0;
-                }
-                int x = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= o) x += y;
-                }
-                int* ws = M.warp[pass & 1];  // alternating: no barrier needed before the next pass writes
-                if (lane == 31) ws[warp] = x;
-                __syncthreads();
-                int off = staged + x - cnt, L = 0;
-#pragma unroll
-                for (int w = 0; w < NM_THREADS / 32; w++) {
-                    const int c = ws[w];
-                    if (w < warp) off += c;
-                    L += c;
-                }
-#pragma unroll
-                for (int r = 0; r < NM_PER_THREAD; r++) {
-                    if (!nzr[r]) continue;
-                    const int i = b0 + r * NM_THREADS + t;
-                    const int ix = bx + x_lo + (i & 15), iy = by + y_lo + ((i >> 4) & 15), iz = bz + z_lo + (i >> 8);
-                    M.n[0][off] = NG.p0.x + NG.dA.x * ix + NG.dB.x * iy + NG.dC.x * iz;
-                    M.n[1][off] = NG.p0.y + NG.dA.y * ix + NG.dB.y * iy + NG.dC.y * iz;
-                    M.n[2][off] = NG.p0.z + NG.dA.z * ix + NG.dB.z * iy + NG.dC.z * iz;
-                    M.n[3][off] = (float)((double)(long long)lo[r].x * inv);
-                    M.n[4][off] = (float)((double)(long long)lo[r].y * inv);
-                    M.n[5][off] = (float)((double)(long long)hi[r].x * inv);
-                    M.n[6][off] = (float)((double)(long long)hi[r].y * inv);
-                    off++;
-                }
-                staged = nn > 0 ? staged + L : 0;
-            }
-            // < 2 * NM_STAGE staged: a pass adds at most NM_STAGE
-            if (staged >= NM_STAGE || (b0 == FB * FB * FB && staged > 0)) {
-                compute(staged, M.near, nn);
-                staged = 0;
-            }
-        }
-        __syncthreads();  // the lists and counts are rewritten for the next block
-    }
-    __syncthreads();
-    for (int k = t; k < 6 * na; k += NM_THREADS) {
-        const int a = k / 6, c = k - 6 * a;
-        const double v = M.acc[c][a];
-        partial[((size_t)D->row_off + (size_t)lc * na + a) * 6 + c] = (KIND == SPM_KIND_LJ && PAR && c == 3) ? -v : v;
-    }
-}
-
-template <bool PAR>
-auto blocks_kernel(int kind, bool on) {
-    if (kind == SPM_KIND_MORSE)
-        return on ? batch_adjoint_blocks_kernel<SPM_KIND_MORSE, true, PAR> : batch_adjoint_blocks_kernel<SPM_KIND_MORSE, false, PAR>;
-    return on ? batch_adjoint_blocks_kernel<SPM_KIND_LJ, true, PAR> : batch_adjoint_blocks_kernel<SPM_KIND_LJ, false, PAR>;
-}
-
 // grad[ga*6 + c] = sum over the molecule's node units, fixed order.  When the
 // node kernel ran before it (mark != null), block 0 marks the adjoint grid clear.
 __global__ void __launch_bounds__(256)
@@ -2339,27 +2042,12 @@ extern "C" int spm_batch_adjoint_params(int kind, int n_mol, const spm_batch_mol
             const bool on = S.qon != 0.f;
             const auto kern = node_kernel(kind, on, (adj_flags & SPM_ADJ_PAIR_PARAMS) != 0, shape->adj_ilp,
                                           shape->adj_stage);
-            // blocks with a far field for the molecules in_blocks names (not the tuner's node-kernel variants)
-            // and only from two units per resident CTA on: two molecules of up to 60 atoms took 1.02 ms per fitting
-            // step with blocks against 0.85 node by node, a batch of 16 5.81 against 6.23
-            const bool blocks = shape->adj_ilp == 1 && shape->adj_stage == 0 && n_units >= 4 * 148;
             // status: the second word of the marker slot (bit 0: a bulk copy's wait ran out)
             unsigned* status = reinterpret_cast<unsigned*>(mark + 1);
             const size_t nm_bytes = shape->adj_stage ? NM_SMEM_BULK : shape->adj_ilp == 3 ? NM_SMEM_2ATOM : NM_SMEM;
             kern<<<(unsigned)n_units, NM_THREADS, nm_bytes, st>>>(
                 n_mol, mols, chunk, reinterpret_cast<const float4*>(atoms), params, pstride, S, gq, box, umax, part,
-                status, blocks);
-            if (blocks) {
-                static const FarTab tab = make_far_tab();
-                const bool par = (adj_flags & SPM_ADJ_PAIR_PARAMS) != 0;
-                const auto bk = par ? blocks_kernel<true>(kind, on) : blocks_kernel<false>(kind, on);
-                if (cudaFuncSetAttribute(bk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlkShared)) !=
-                    cudaSuccess)
-                    return set_error(SPM_ERR_CUDA, "spm_batch_adjoint_params: cannot set shared memory size");
-                bk<<<(unsigned)n_units, NM_THREADS, sizeof(BlkShared), st>>>(
-                    n_mol, mols, chunk, reinterpret_cast<const float4*>(atoms), params, pstride, S, gq, box, umax, part,
-                    tab);
-            }
+                status);
             nodes_ran = true;
         }
         batch_fold_rows_kernel<<<dim3((unsigned)n_atoms, 6), 256, 0, st>>>(n_mol, mols, chunk, part, grad,

@@ -1,6 +1,5 @@
 // spm_far.cuh -- blocks of grid nodes with a far field: the Chebyshev points and interpolation weights of a
-// block, and the test that an atom is far from it.  Shared by the force-grid build (grid_build.cu, where the
-// reasons for the constants stand) and its adjoint (adjoint_grid.cu).
+// block, and the test that an atom is far from it (the reasons for the constants stand in grid_build.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <cmath>
@@ -56,7 +55,7 @@ __device__ __forceinline__ float len3(float x, float y, float z) {
 
 // Geom: p0, dA, dB, dC of the grid.
 template <class Geom>
-__device__ __forceinline__ FarCube far_cube(const Geom& G, int x, int y, int z, int n, float ratio = FAR_RATIO) {
+__device__ __forceinline__ FarCube far_cube(const Geom& G, int x, int y, int z, int n) {
     FarCube C;
     C.half = 0.5f * (float)(n - 1);
     const float cx = (float)x + C.half, cy = (float)y + C.half, cz = (float)z + C.half;
@@ -71,7 +70,7 @@ __device__ __forceinline__ FarCube far_cube(const Geom& G, int x, int y, int z, 
                                                  __fmaf_rn(sc, G.dC.z, __fmaf_rn(sb, G.dB.z, G.dA.z)))));
     }
     C.h = __fmul_rn(e, C.half);
-    C.lim2 = __fmul_rn(__fmul_rn(ratio, C.h), __fmul_rn(ratio, C.h));
+    C.lim2 = __fmul_rn(__fmul_rn(FAR_RATIO, C.h), __fmul_rn(FAR_RATIO, C.h));
     return C;
 }
 
