@@ -19,10 +19,10 @@
 //     non-zero offset get their own rsqrt.
 // Transcendentals use MUFU approximations (rsqrt.approx, ex2.approx).
 //
-// That direct sum is for systems of few atoms.  From SPM_FAR_MIN_ATOMS atoms on the
+// That direct sum is for molecules.  From SPM_FAR_MIN_ATOMS atoms on (slabs) the
 // nodes are built in blocks of 16^3, each atom at a block's nodes only when it is
 // near the block; the smooth field of the distant atoms is evaluated at 8^3
-// Chebyshev points of the block and interpolated (build_block below).
+// Chebyshev points of the block and interpolated (build_cell below).
 #include "spm_internal.cuh"
 #include "spm_batch.cuh"
 #include "spm_f32x2.cuh"
@@ -298,15 +298,14 @@ grid_build_kernel(int na, const float4* __restrict__ atoms, const float* __restr
 // nodes a probe reaches (|E| < 0.5 eV), relative to their norm, direct sum -> blocks: 1200 LJ atoms on an
 // ionic slab 1.98e-6 -> 1.89e-6 (energy 2.9e-6 -> 1.7e-6), 57 Morse atoms with offset charges 7.7e-7 -> 7.7e-7.
 //
-// Time, direct sum -> blocks: 1200 atoms on 480 x 480 x 240 nodes 32.0 -> 2.28 ms, 57 Morse atoms with two
-// offset charges on 187 x 203 x 149 426 -> 181 us, 38 atoms on 200^3 187 -> 124 us.  What is left is the near
-// sums (FP32 issue), the far sums and the interpolation in about equal parts.  Below SPM_FAR_MIN_ATOMS most
-// atoms are near most blocks and the interpolation does not pay.
+// The blocks come in groups of 2^3 whose common far atoms (FAR_RATIO group half-edges
+// away) are summed once at the group's Chebyshev points; a block takes that field at
+// its own points by interpolation and adds the atoms that are far for it alone.
 //
-// Systems of SPM_FAR_GROUP_ATOMS atoms or more take the blocks in groups of 2^3 whose
-// common far atoms (FAR_RATIO group half-edges away) are summed once at the
-// group's Chebyshev points; a block takes that field at its own points by
-// interpolation and adds the atoms that are far for it alone.
+// SPM_FAR_MIN_ATOMS: molecules keep the direct sum's order and bits.  Unpolished FIRE strokes stop where their
+// force falls below the threshold, so a grid that differs in its last bits moves their images by 1e-4 (64
+// molecules of 10 to 120 atoms), and with few atoms most are near most blocks: 38 atoms on 200^3 nodes take
+// 187 us directly and 124 in blocks, 256 1223 against 461, 1200 on 480 x 480 x 240 32.0 ms against 2.28.
 constexpr int FAR_REF = 3 * 64 + 3 * 8 + 3;  // the point whose value is interpolated as a constant
 constexpr int FAR_CHUNK = 256;       // atoms gathered at a time
 
@@ -460,25 +459,21 @@ __device__ __forceinline__ float4 far_axis(const float (*W)[FP], const float4* i
     return s;
 }
 
-// Blocks [child0, child1) of one lattice cell (x0, y0, z0: its first node; group: a cell of 2^3 blocks, else
-// one), nodes inside the box B stored as build_tile does.  ZB: nodes along z per thread in the near sums, 8 or 16.
+// Blocks [child0, child1) of the 2^3 of one lattice cell (x0, y0, z0: its first node), nodes inside the box B
+// stored as build_tile does.  ZB: nodes along z per thread in the near sums, 8 or 16.
 template <int KIND, bool ON, int NOFF, int ZB, int LAYOUT>
-__device__ __forceinline__ void build_block(FarShared<NOFF>& M, bool group, int child0, int child1, int na, const float4* __restrict__ atoms,
-                                            const float* __restrict__ params, int pstride, float4* __restrict__ out,
-                                            const GridGeom& G, const TipSites& S, const StoreBox& B, int x0, int y0,
-                                            int z0) {
+__device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int child1, int na,
+                                           const float4* __restrict__ atoms, const float* __restrict__ params,
+                                           int pstride, float4* __restrict__ out, const GridGeom& G, const TipSites& S,
+                                           const StoreBox& B, int x0, int y0, int z0) {
     constexpr int ZP = ZB / 2;
     const int nthr = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
-    FarCube C2 = {};
-    bool use2 = false;
-    if (group) {
-        C2 = far_cube(G, x0, y0, z0, 2 * FB);
-        auto far2 = [&](float4 a, const float* pr) { return is_far<KIND, NOFF>(C2, S, a, pr); };
-        use2 = count_atoms(tid, nthr, na, atoms, params, pstride, far2) >= FAR_FEWEST;
-        if (use2) {
-            far_points<KIND, ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C2, far2);
-            for (int i = tid; i < FN; i += nthr) M.group[i] = M.part[0][i];
-        }
+    const FarCube C2 = far_cube(G, x0, y0, z0, SPM_FAR_CELL);
+    auto far2 = [&](float4 a, const float* pr) { return is_far<KIND, NOFF>(C2, S, a, pr); };
+    const bool use2 = count_atoms(tid, nthr, na, atoms, params, pstride, far2) >= FAR_FEWEST;
+    if (use2) {
+        far_points<KIND, ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C2, far2);
+        for (int i = tid; i < FN; i += nthr) M.group[i] = M.part[0][i];
     }
     for (int child = child0; child < child1; child++) {
         const int sx = child & 1, sy = (child >> 1) & 1, sz = child >> 2;
@@ -530,8 +525,6 @@ __device__ __forceinline__ void build_block(FarShared<NOFF>& M, bool group, int 
             }
             __syncthreads();
         }
-        const bool once = na <= FAR_CHUNK;  // the near list holds for every column of this thread
-        int nnear = once ? gather_atoms<KIND, NOFF>(M, tid, nthr, 0, na, atoms, params, pstride, S, near1) : 0;
         for (int item = tid; item < FB * FB * (FB / ZB); item += nthr) {
             const int x = item & (FB - 1), y = (item >> 4) & (FB - 1), ic0 = bz + (item >> 8) * ZB;
             const int ia = bx + x, ib = by + y, xl = ia - B.x_lo, yl = ib - B.y_lo;
@@ -574,7 +567,7 @@ __device__ __forceinline__ void build_block(FarShared<NOFF>& M, bool group, int 
                 }
             }
             for (int c0 = 0; c0 < na; c0 += FAR_CHUNK) {
-                if (!once) nnear = gather_atoms<KIND, NOFF>(M, tid, nthr, c0, na, atoms, params, pstride, S, near1);
+                const int nnear = gather_atoms<KIND, NOFF>(M, tid, nthr, c0, na, atoms, params, pstride, S, near1);
                 if (active) {
 #pragma unroll 1
                     for (int j = 0; j < nnear; j++) {
@@ -603,7 +596,7 @@ __device__ __forceinline__ void load_far_tab(FarShared<NOFF>& M, const FarTab& t
 
 // 256 threads, 16 nodes along z each, at 128 registers (two CTAs per SM): 2.24 ms on the 1200-atom 480 x 480
 // x 240 grid (128 threads 2.25, 8 nodes each 2.36; 0.47 ms against 0.71 and 0.44 on 527 atoms, 243 x 138 x
-// 98); on 38 atoms, 200^3, 128 threads took 10% less.  The differences from one point cost 2% since.
+// 98).  The differences from one point cost 2% since.
 constexpr int FAR_THREADS = 256;
 constexpr long long FAR_CTAS = 222;  // CTAs that fill a 148-SM part one and a half times
 
@@ -611,15 +604,15 @@ constexpr long long FAR_CTAS = 222;  // CTAs that fill a 148-SM part one and a h
 // leave SMs idle (each CTA then sums the group's field itself: the same values).
 template <int KIND, bool ON, int NOFF>
 __global__ void __launch_bounds__(FAR_THREADS, 2)
-grid_block_kernel(bool group, int split, int na, const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
+grid_block_kernel(int split, int na, const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
                   float4* __restrict__ grid, GridGeom G, TipSites S, const __grid_constant__ FarTab tab) {
     extern __shared__ __align__(16) unsigned char far_smem[];
     FarShared<NOFF>& M = *reinterpret_cast<FarShared<NOFF>*>(far_smem);
     load_far_tab(M, tab);
     const StoreBox B = {0, G.nx, 0, G.ny, 0, G.nz};
-    const int e = group ? 2 * FB : FB, nb = group ? 8 / split : 1, part = blockIdx.x % split;
-    build_block<KIND, ON, NOFF, GB_ZB, 1>(M, group, part * nb, (part + 1) * nb, na, atoms, params, pstride, grid, G, S,
-                                           B, blockIdx.x / split * e, blockIdx.y * e, blockIdx.z * e);
+    const int e = SPM_FAR_CELL, nb = 8 / split, part = blockIdx.x % split;
+    build_cell<KIND, ON, NOFF, GB_ZB, 1>(M, part * nb, (part + 1) * nb, na, atoms, params, pstride, grid, G, S, B,
+                                         blockIdx.x / split * e, blockIdx.y * e, blockIdx.z * e);
 }
 
 template <int KIND, bool ON, int NOFF>
@@ -630,13 +623,12 @@ int launch_blocks(int na, const float4* atoms, const float* params, int pstride,
     const size_t smem = sizeof(FarShared<NOFF>);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return set_error(SPM_ERR_CUDA, "spm_grid_build: cannot enable %zu B of shared memory", smem);
-    const bool group = na >= SPM_FAR_GROUP_ATOMS;
-    const int e = group ? 2 * FB : FB;
+    const int e = SPM_FAR_CELL;
     const long long cells = (long long)((G.nx + e - 1) / e) * ((G.ny + e - 1) / e) * ((G.nz + e - 1) / e);
     int split = 1;
-    while (group && split < 8 && cells * split < FAR_CTAS) split *= 2;
+    while (split < 8 && cells * split < FAR_CTAS) split *= 2;
     kern<<<dim3((G.nx + e - 1) / e * split, (G.ny + e - 1) / e, (G.nz + e - 1) / e), FAR_THREADS, smem, st>>>(
-        group, split, na, atoms, params, pstride, out, G, S, tab);
+        split, na, atoms, params, pstride, out, G, S, tab);
     return check_launch("spm_grid_build");
 }
 
@@ -739,8 +731,7 @@ batch_grid_block_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
     const long long total = (long long)mols[n_mol - 1].block_off + far_cells(mols[n_mol - 1]);
     for (long long c = blockIdx.x; c < total; c += gridDim.x) {
         const spm_batch_mol* D = mols + SPM_MOL_BY(block_off, mols, n_mol, c);
-        const bool group = D->n_atoms >= SPM_FAR_GROUP_ATOMS;
-        const int e = group ? 2 * FB : FB;
+        const int e = SPM_FAR_CELL;
         const StoreBox B = {D->x_lo, D->nx_slab, D->y_lo, D->ny_slab, D->z_lo, D->z_lo + D->nz_slab};
         const int cx0 = B.x_lo / e, cy0 = B.y_lo / e, cz0 = B.zst_lo / e;
         const int ncx = (B.x_lo + B.nxs - 1) / e - cx0 + 1, ncy = (B.y_lo + B.nys - 1) / e - cy0 + 1;
@@ -752,9 +743,9 @@ batch_grid_block_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
         G.dB = ld4f(D->dB);
         G.dC = ld4f(D->dC);
         const int ao = D->atom_off;
-        build_block<KIND, ON, NOFF, 8, LAYOUT>(M, group, 0, group ? 8 : 1, D->n_atoms, atoms + ao, params + (size_t)ao * pstride, pstride,
-                                                grid + LAYOUT * D->grid_off, G, S, B, (cx0 + lc % ncx) * e,
-                                                (cy0 + lc / ncx % ncy) * e, (cz0 + lc / ncx / ncy) * e);
+        build_cell<KIND, ON, NOFF, 8, LAYOUT>(M, 0, 8, D->n_atoms, atoms + ao, params + (size_t)ao * pstride, pstride,
+                                              grid + LAYOUT * D->grid_off, G, S, B, (cx0 + lc % ncx) * e,
+                                              (cy0 + lc / ncx % ncy) * e, (cz0 + lc / ncx / ncy) * e);
         __syncthreads();  // the next cell reuses the shared memory
     }
 }

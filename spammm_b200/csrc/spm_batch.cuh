@@ -11,17 +11,16 @@
 
 namespace spm {
 
-// Atoms from which a force grid is built in blocks with a far field, and in groups of 2^3 blocks
-// (grid_build.cu); the same for a batch's molecules and a single grid.
-constexpr int SPM_FAR_MIN_ATOMS = 32;
-constexpr int SPM_FAR_GROUP_ATOMS = 256;
-constexpr int SPM_FAR_BLOCK = 16;  // nodes per block edge
+// Atoms from which a force grid is built in blocks with a far field (grid_build.cu); the same for a batch's
+// molecules and a single grid.
+constexpr int SPM_FAR_MIN_ATOMS = 256;
+constexpr int SPM_FAR_BLOCK = 16;                // nodes per block edge
+constexpr int SPM_FAR_CELL = 2 * SPM_FAR_BLOCK;  // lattice cells: groups of 2^3 blocks
 
-// Lattice cells (blocks or groups of blocks) that a molecule's box of stored nodes meets; 0 below
-// SPM_FAR_MIN_ATOMS.
+// Lattice cells that a molecule's box of stored nodes meets; 0 below SPM_FAR_MIN_ATOMS.
 __host__ __device__ inline long long far_cells(const spm_batch_mol& D) {
     if (D.n_atoms < SPM_FAR_MIN_ATOMS) return 0;
-    const int e = D.n_atoms >= SPM_FAR_GROUP_ATOMS ? 2 * SPM_FAR_BLOCK : SPM_FAR_BLOCK;
+    const int e = SPM_FAR_CELL;
     return ((long long)(D.x_lo + D.nx_slab - 1) / e - D.x_lo / e + 1) *
            ((long long)(D.y_lo + D.ny_slab - 1) / e - D.y_lo / e + 1) *
            ((long long)(D.z_lo + D.nz_slab - 1) / e - D.z_lo / e + 1);

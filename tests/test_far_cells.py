@@ -24,11 +24,10 @@ def test_block_prefix_covers_each_box(nas):
     for j in range(plan.n):
         D = plan.mols[j]
         assert D.block_off == at
-        if D.n_atoms < 32:
+        if D.n_atoms < 256:
             continue
-        e = 32 if D.n_atoms >= 256 else 16
         cells = 1
         for lo, n in ((D.x_lo, D.nx_slab), (D.y_lo, D.ny_slab), (D.z_lo, D.nz_slab)):
-            cells *= len({i // e for i in range(lo, lo + n)})
+            cells *= len({i // 32 for i in range(lo, lo + n)})
         at += cells
     assert ctypes.sizeof(_lib.BatchMol) % 8 == 0

@@ -1,5 +1,5 @@
-"""Force grids of 32 atoms or more: blocks of 16^3 nodes whose distant atoms are interpolated from 8^3
-Chebyshev points (build_block, grid_build.cu), against the FP64 pair sums.
+"""Force grids of 256 atoms or more: blocks of 16^3 nodes whose distant atoms are interpolated from 8^3
+Chebyshev points (build_cell, grid_build.cu), against the FP64 pair sums.
 
 Bound per channel: 1e-5 S (S the sum of the atoms' contribution magnitudes) + the float32 node-coordinate
 term of test_gpu_scale.py.  A pair term errs by up to 2e-6 (rsqrt.approx to the 13th power) or, for Morse,
@@ -57,9 +57,25 @@ def _check(kind, atoms, prm, n, p0, dA, dB, dC, sites):
 @pytest.mark.parametrize("na", [31, 32, 33, 255, 256, 257, 600])
 @pytest.mark.parametrize("sites", [ON, OFF, BOTH], ids=["on", "off", "both"])
 def test_against_pair_sums(cuda, kind, na, sites):
-    """Both sides of the atom counts where blocks, a second gather and grouped blocks begin; ragged boxes."""
+    """Both sides of the atom count where blocks begin (256), further gathers; ragged boxes."""
     atoms, prm = _system(na, kind, 12.0)
     _check(kind, atoms, prm, (97, 65, 81), (-12.0, -5.0, -4.0), (0.1, 0, 0), (0, 0.1, 0), (0, 0, 0.1), sites)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("na", [31, 32, 57, 120, 255])
+def test_molecules_are_summed_directly(cuda, kind, na):
+    """Below 256 atoms a node's bits are those of its own pair sums: the box around it does not matter (a
+    spacing of 1/8, so that both boxes have the same node coordinates)."""
+    atoms, prm = _system(na, kind, 6.0)
+    h, n, cut = 0.125, (70, 61, 66), (5, 3, 7)
+    vec = [np.array(v, np.float32) for v in ((h, 0, 0, 0), (0, h, 0, 0), (0, 0, h, 0))]
+    Qs, QZs = (np.array(v, np.float32) for v in BOTH)
+    p0 = np.array([-4.5, -3.75, -1.0, 0], np.float32)
+    whole = gpu.grid_build(kind, atoms, prm, n, p0, *vec, Qs, QZs)
+    p1 = p0 + np.array([*(h * c for c in cut), 0], np.float32)
+    part = gpu.grid_build(kind, atoms, prm, tuple(a - c for a, c in zip(n, cut)), p1, *vec, Qs, QZs)
+    assert torch.equal(whole[cut[2]:, cut[1]:, cut[0]:], part)
 
 
 @pytest.mark.parametrize("n", [(1, 1, 1), (15, 16, 17), (33, 2, 64), (200, 3, 31)])
