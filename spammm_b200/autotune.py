@@ -2,7 +2,7 @@
 
 Every batched stage reads only its own fields of ``spm_batch_shape``:
 
-  grid build   gb_ty (CTA rows: 32 x gb_ty threads), gb_zb (z-nodes per thread); molecules below 256 atoms
+  grid build   gb_ty (CTA rows: 32 x gb_ty threads), gb_zb (z-nodes per thread); Morse, and LJ below 256 atoms
   relaxation   rx_sync (z-synchronised warp tiles, independent lanes, or -- warm polished fits --
                a Newton-only pass in tiles and a FIRE pass over the strokes it stopped),
                rx_threads (CTA size), rx_tile_h (pixel tile (32/h) x h per warp

@@ -19,8 +19,8 @@
 //     non-zero offset get their own rsqrt.
 // Transcendentals use MUFU approximations (rsqrt.approx, ex2.approx).
 //
-// That direct sum is for molecules.  From SPM_FAR_MIN_ATOMS atoms on (slabs) the
-// nodes are built in blocks of 16^3, each atom at a block's nodes only when it is
+// That direct sum is for molecules and for Morse.  LJ systems of SPM_FAR_MIN_ATOMS
+// atoms or more (slabs): the nodes are built in blocks of 16^3, each atom at a block's nodes only when it is
 // near the block; the smooth field of the distant atoms is evaluated at 8^3
 // Chebyshev points of the block and interpolated (build_cell below).
 #include "spm_internal.cuh"
@@ -289,14 +289,15 @@ grid_build_kernel(int na, const float4* __restrict__ atoms, const float* __restr
 // tensor product along x, y and z; near atoms are summed at the nodes as in
 // build_tile, on top of the interpolated values.
 //
-// Interpolation error of one atom relative to its largest value in the block
-// (float64, worst direction, at 9 half-edges): 1/r^2 4e-9, r^-7 3e-7, the LJ and
-// Morse laws 1e-7 and 5e-7, falling as the eighth power of the distance -- not
-// above the rounding of the direct float32 sum (rsqrt.approx alone puts 8e-7 on
-// r^-7), and the sums are 2-17 times shorter.  Morse exponentials grow with |K| times the half-edge,
-// not with the distance: an atom with |K| h > FAR_KH is near everywhere.  Measured error of the forces at the
-// nodes a probe reaches (|E| < 0.5 eV), relative to their norm, direct sum -> blocks: 1200 LJ atoms on an
-// ionic slab 1.98e-6 -> 1.89e-6 (energy 2.9e-6 -> 1.7e-6), 57 Morse atoms with offset charges 7.7e-7 -> 7.7e-7.
+// Interpolation error of one atom relative to its own force at the node (float64, worst corner and direction,
+// at 9 half-edges): 1/r^2 3e-9, r^-7 1e-6, and much less over most of the block, falling as the eighth power of
+// the distance -- the direct float32 sum rounds r^-7 by 8e-7 (rsqrt.approx), and the sums are 2-17 times
+// shorter.  Measured error of the forces at the nodes a probe reaches (|E| < 0.5 eV), relative to their norm,
+// direct sum -> blocks: 1200 LJ atoms on an ionic slab 1.98e-6 -> 1.89e-6 (energy 2.9e-6 -> 1.7e-6).
+//
+// LJ only.  A Morse exponential varies with |K| times the half-edge, at any distance: at 0.1 A (|K| h = 1.35)
+// its interpolation errs by 4e-6 of the local force, at |K| h = 1.5 by 1.7e-5, where the direct sum errs by up
+// to 3e-6.  Morse grids are direct sums.
 //
 // The blocks come in groups of 2^3 whose common far atoms (FAR_RATIO group half-edges
 // away) are summed once at the group's Chebyshev points; a block takes that field at
@@ -321,9 +322,9 @@ struct FarShared {
 };
 
 // Far of the cube: the pair law and every off-node charge (seen from the node moved by its offset).
-// A NaN position or parameter is near.
-template <int KIND, int NOFF>
-__device__ __forceinline__ bool is_far(const FarCube& C, const TipSites& S, float4 a, const float* __restrict__ pr) {
+// A NaN position is near.
+template <int NOFF>
+__device__ __forceinline__ bool is_far(const FarCube& C, const TipSites& S, float4 a) {
     const float dx = C.x - a.x, dy = C.y - a.y, dz = C.z - a.z;
     const float dxy2 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
     bool far = __fmaf_rn(dz, dz, dxy2) >= C.lim2;
@@ -332,13 +333,12 @@ __device__ __forceinline__ bool is_far(const FarCube& C, const TipSites& S, floa
         const float dk = __fadd_rn(dz, S.qz[k]);
         far = far && __fmaf_rn(dk, dk, dxy2) >= C.lim2;
     }
-    if (KIND == SPM_KIND_MORSE) far = far && __fmul_rn(fabsf(__ldg(pr + 2)), C.h) <= FAR_KH;
     return far;
 }
 
-// Stages the atoms of [c0, c0 + FAR_CHUNK) that satisfy pick(atom, parameter row), in atom order; returns
+// Stages the atoms of [c0, c0 + FAR_CHUNK) that satisfy pick(atom), in atom order; returns
 // their number to every thread.
-template <int KIND, int NOFF, class Pick>
+template <int NOFF, class Pick>
 __device__ __forceinline__ int gather_atoms(FarShared<NOFF>& M, int tid, int nthr, int c0, int na,
                                             const float4* __restrict__ atoms, const float* __restrict__ params,
                                             int pstride, const TipSites& S, const Pick& pick) {
@@ -348,11 +348,10 @@ __device__ __forceinline__ int gather_atoms(FarShared<NOFF>& M, int tid, int nth
     for (int b = c0; b < c1; b += nthr) {
         const int j = b + tid;
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float* pr = params + (size_t)(j < c1 ? j : c0) * pstride;
         bool take = false;
         if (j < c1) {
             a = __ldg(atoms + j);
-            take = pick(a, pr);
+            take = pick(a);
         }
         const unsigned m = __ballot_sync(0xffffffffu, take);
         __syncthreads();  // the previous round's warp counts and the previous chunk's atoms are read
@@ -366,7 +365,7 @@ __device__ __forceinline__ int gather_atoms(FarShared<NOFF>& M, int tid, int nth
         }
         if (take) {
             M.pos[at] = make_float4(a.x, a.y, a.z, a.w * S.qs_on);
-            M.prm[at] = atom_params<KIND>(pr);
+            M.prm[at] = atom_params<SPM_KIND_LJ>(params + (size_t)j * pstride);
 #pragma unroll
             for (int k = 0; k < NOFF; k++) M.q[k][at] = a.w * S.qs[k];
         }
@@ -377,11 +376,11 @@ __device__ __forceinline__ int gather_atoms(FarShared<NOFF>& M, int tid, int nth
 
 template <class Pick>
 __device__ __forceinline__ int count_atoms(int tid, int nthr, int na, const float4* __restrict__ atoms,
-                                           const float* __restrict__ params, int pstride, const Pick& pick) {
+                                           const Pick& pick) {
     int n = 0;
     for (int b = 0; b < na; b += nthr) {
         const int j = b + tid;
-        n += __syncthreads_count(j < na && pick(__ldg(atoms + j), params + (size_t)(j < na ? j : 0) * pstride));
+        n += __syncthreads_count(j < na && pick(__ldg(atoms + j)));
     }
     return n;
 }
@@ -390,14 +389,14 @@ __device__ __forceinline__ int count_atoms(int tid, int nthr, int na, const floa
 // ky).  Four runs of consecutive atoms go side by side and are added in a fixed order (consecutive: the
 // charges of an ionic crystal listed in lattice order alternate, and every fourth of them would add up to a
 // partial sum far above the total).
-template <int KIND, bool ON, int NOFF, class Pick>
+template <bool ON, int NOFF, class Pick>
 __device__ __forceinline__ void far_points(FarShared<NOFF>& M, int tid, int nthr, int na,
                                            const float4* __restrict__ atoms, const float* __restrict__ params,
                                            int pstride, const GridGeom& G, const TipSites& S, const FarCube& C,
                                            const Pick& pick) {
     constexpr int ZP = FP / 2;
     for (int c0 = 0; c0 < na; c0 += FAR_CHUNK) {
-        const int n = gather_atoms<KIND, NOFF>(M, tid, nthr, c0, na, atoms, params, pstride, S, pick);
+        const int n = gather_atoms<NOFF>(M, tid, nthr, c0, na, atoms, params, pstride, S, pick);
         for (int i = tid; i < 4 * FP * FP; i += nthr) {
             const int g = i >> 6, col = i & 63;
             const float ux = C.half * M.tab.c[col >> 3], uy = C.half * M.tab.c[col & 7];
@@ -416,7 +415,7 @@ __device__ __forceinline__ void far_points(FarShared<NOFF>& M, int tid, int nthr
                 float q[NOFF > 0 ? NOFF : 1];
 #pragma unroll
                 for (int k = 0; k < NOFF; k++) q[k] = M.q[k][j];
-                add_atom<KIND, ON, NOFF, ZP>(M.pos[j], M.prm[j], q, px, py, pz, S, fx, fy, fz, fe);
+                add_atom<SPM_KIND_LJ, ON, NOFF, ZP>(M.pos[j], M.prm[j], q, px, py, pz, S, fx, fy, fz, fe);
             }
 #pragma unroll
             for (int p = 0; p < ZP; p++) {
@@ -461,7 +460,7 @@ __device__ __forceinline__ float4 far_axis(const float (*W)[FP], const float4* i
 
 // Blocks [child0, child1) of the 2^3 of one lattice cell (x0, y0, z0: its first node), nodes inside the box B
 // stored as build_tile does.  ZB: nodes along z per thread in the near sums, 8 or 16.
-template <int KIND, bool ON, int NOFF, int ZB, int LAYOUT>
+template <bool ON, int NOFF, int ZB, int LAYOUT>
 __device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int child1, int na,
                                            const float4* __restrict__ atoms, const float* __restrict__ params,
                                            int pstride, float4* __restrict__ out, const GridGeom& G, const TipSites& S,
@@ -469,10 +468,10 @@ __device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int c
     constexpr int ZP = ZB / 2;
     const int nthr = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
     const FarCube C2 = far_cube(G, x0, y0, z0, SPM_FAR_CELL);
-    auto far2 = [&](float4 a, const float* pr) { return is_far<KIND, NOFF>(C2, S, a, pr); };
-    const bool use2 = count_atoms(tid, nthr, na, atoms, params, pstride, far2) >= FAR_FEWEST;
+    auto far2 = [&](float4 a) { return is_far<NOFF>(C2, S, a); };
+    const bool use2 = count_atoms(tid, nthr, na, atoms, far2) >= FAR_FEWEST;
     if (use2) {
-        far_points<KIND, ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C2, far2);
+        far_points<ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C2, far2);
         for (int i = tid; i < FN; i += nthr) M.group[i] = M.part[0][i];
     }
     for (int child = child0; child < child1; child++) {
@@ -483,16 +482,16 @@ __device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int c
             continue;  // CTA-uniform: no node of this block is stored
         const FarCube C1 = far_cube(G, bx, by, bz, FB);
         // an atom of this block alone: not in the group's field
-        auto own = [&](float4 a, const float* pr) { return !(use2 && is_far<KIND, NOFF>(C2, S, a, pr)); };
-        auto far1 = [&](float4 a, const float* pr) { return own(a, pr) && is_far<KIND, NOFF>(C1, S, a, pr); };
-        const int nfar = count_atoms(tid, nthr, na, atoms, params, pstride, far1);
+        auto own = [&](float4 a) { return !(use2 && is_far<NOFF>(C2, S, a)); };
+        auto far1 = [&](float4 a) { return own(a) && is_far<NOFF>(C1, S, a); };
+        const int nfar = count_atoms(tid, nthr, na, atoms, far1);
         const bool use1 = nfar >= FAR_FEWEST, field = use1 || use2;
-        auto near1 = [&](float4 a, const float* pr) {
-            return own(a, pr) && !(use1 && is_far<KIND, NOFF>(C1, S, a, pr));
+        auto near1 = [&](float4 a) {
+            return own(a) && !(use1 && is_far<NOFF>(C1, S, a));
         };
         float4* stage = M.part[1];  // 1024 float4: parts 1 and 2
         __syncthreads();            // the group's copy, the previous block's stage
-        if (use1) far_points<KIND, ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C1, far1);
+        if (use1) far_points<ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C1, far1);
         if (use2) {
             for (int i = tid; i < FN; i += nthr) M.part[1][i] = far_axis(M.tab.T[sx], M.group, i, 8);
             __syncthreads();
@@ -567,14 +566,14 @@ __device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int c
                 }
             }
             for (int c0 = 0; c0 < na; c0 += FAR_CHUNK) {
-                const int nnear = gather_atoms<KIND, NOFF>(M, tid, nthr, c0, na, atoms, params, pstride, S, near1);
+                const int nnear = gather_atoms<NOFF>(M, tid, nthr, c0, na, atoms, params, pstride, S, near1);
                 if (active) {
 #pragma unroll 1
                     for (int j = 0; j < nnear; j++) {
                         float q[NOFF > 0 ? NOFF : 1];
 #pragma unroll
                         for (int k = 0; k < NOFF; k++) q[k] = M.q[k][j];
-                        add_atom<KIND, ON, NOFF, ZP>(M.pos[j], M.prm[j], q, px, py, pz, S, fx, fy, fz, fe);
+                        add_atom<SPM_KIND_LJ, ON, NOFF, ZP>(M.pos[j], M.prm[j], q, px, py, pz, S, fx, fy, fz, fe);
                     }
                 }
             }
@@ -602,7 +601,7 @@ constexpr long long FAR_CTAS = 222;  // CTAs that fill a 148-SM part one and a h
 
 // A whole grid: one CTA per lattice cell, or per 4, 2 or 1 blocks of a group while the groups alone would
 // leave SMs idle (each CTA then sums the group's field itself: the same values).
-template <int KIND, bool ON, int NOFF>
+template <bool ON, int NOFF>
 __global__ void __launch_bounds__(FAR_THREADS, 2)
 grid_block_kernel(int split, int na, const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
                   float4* __restrict__ grid, GridGeom G, TipSites S, const __grid_constant__ FarTab tab) {
@@ -611,15 +610,15 @@ grid_block_kernel(int split, int na, const float4* __restrict__ atoms, const flo
     load_far_tab(M, tab);
     const StoreBox B = {0, G.nx, 0, G.ny, 0, G.nz};
     const int e = SPM_FAR_CELL, nb = 8 / split, part = blockIdx.x % split;
-    build_cell<KIND, ON, NOFF, GB_ZB, 1>(M, part * nb, (part + 1) * nb, na, atoms, params, pstride, grid, G, S, B,
+    build_cell<ON, NOFF, GB_ZB, 1>(M, part * nb, (part + 1) * nb, na, atoms, params, pstride, grid, G, S, B,
                                          blockIdx.x / split * e, blockIdx.y * e, blockIdx.z * e);
 }
 
-template <int KIND, bool ON, int NOFF>
+template <bool ON, int NOFF>
 int launch_blocks(int na, const float4* atoms, const float* params, int pstride, float4* out, const GridGeom& G,
                   const TipSites& S, cudaStream_t st) {
     static const FarTab tab = make_far_tab();
-    const auto kern = grid_block_kernel<KIND, ON, NOFF>;
+    const auto kern = grid_block_kernel<ON, NOFF>;
     const size_t smem = sizeof(FarShared<NOFF>);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return set_error(SPM_ERR_CUDA, "spm_grid_build: cannot enable %zu B of shared memory", smem);
@@ -635,13 +634,13 @@ int launch_blocks(int na, const float4* atoms, const float* params, int pstride,
 template <int KIND, bool ON>
 int launch_noff(int noff, dim3 grd, dim3 block, cudaStream_t st, int na, const float4* atoms, const float* params,
                 int pstride, float4* out, const GridGeom& G, const TipSites& S) {
-    if (na >= SPM_FAR_MIN_ATOMS) {
+    if (KIND == SPM_KIND_LJ && na >= SPM_FAR_MIN_ATOMS) {
         switch (noff) {
-            case 0: return launch_blocks<KIND, ON, 0>(na, atoms, params, pstride, out, G, S, st);
-            case 1: return launch_blocks<KIND, ON, 1>(na, atoms, params, pstride, out, G, S, st);
-            case 2: return launch_blocks<KIND, ON, 2>(na, atoms, params, pstride, out, G, S, st);
-            case 3: return launch_blocks<KIND, ON, 3>(na, atoms, params, pstride, out, G, S, st);
-            default: return launch_blocks<KIND, ON, 4>(na, atoms, params, pstride, out, G, S, st);
+            case 0: return launch_blocks<ON, 0>(na, atoms, params, pstride, out, G, S, st);
+            case 1: return launch_blocks<ON, 1>(na, atoms, params, pstride, out, G, S, st);
+            case 2: return launch_blocks<ON, 2>(na, atoms, params, pstride, out, G, S, st);
+            case 3: return launch_blocks<ON, 3>(na, atoms, params, pstride, out, G, S, st);
+            default: return launch_blocks<ON, 4>(na, atoms, params, pstride, out, G, S, st);
         }
     }
     switch (noff) {
@@ -692,7 +691,7 @@ batch_grid_build_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
                         const float* __restrict__ params, int pstride, float4* __restrict__ grid, TipSites S) {
     const long long tile = blockIdx.x;
     const spm_batch_mol* D = mols + SPM_MOL_BY(tile_off, mols, n_mol, tile);
-    if (D->n_atoms >= SPM_FAR_MIN_ATOMS) return;  // built by batch_grid_block_kernel
+    if (KIND == SPM_KIND_LJ && D->n_atoms >= SPM_FAR_MIN_ATOMS) return;  // built by batch_grid_block_kernel
     const int ty = blockDim.y;
     const int z_lo = D->z_lo, nzs = D->nz_slab;
     const StoreBox B = {D->x_lo, D->nx_slab, D->y_lo, D->ny_slab, z_lo, z_lo + nzs};
@@ -717,10 +716,10 @@ batch_grid_build_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
                                            z_lo + (int)bz * ZB);
 }
 
-// The molecules of SPM_FAR_MIN_ATOMS atoms or more: persistent CTAs over their lattice cells (block_off:
+// The LJ molecules of SPM_FAR_MIN_ATOMS atoms or more: persistent CTAs over their lattice cells (block_off:
 // prefix of cells over the batch), each cell's nodes inside the molecule's box as grid_block_kernel builds
 // them.
-template <int KIND, bool ON, int NOFF, int LAYOUT>
+template <bool ON, int NOFF, int LAYOUT>
 __global__ void __launch_bounds__(256, 2)
 batch_grid_block_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const float4* __restrict__ atoms,
                         const float* __restrict__ params, int pstride, float4* __restrict__ grid, TipSites S,
@@ -743,7 +742,7 @@ batch_grid_block_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
         G.dB = ld4f(D->dB);
         G.dC = ld4f(D->dC);
         const int ao = D->atom_off;
-        build_cell<KIND, ON, NOFF, 8, LAYOUT>(M, 0, 8, D->n_atoms, atoms + ao, params + (size_t)ao * pstride, pstride,
+        build_cell<ON, NOFF, 8, LAYOUT>(M, 0, 8, D->n_atoms, atoms + ao, params + (size_t)ao * pstride, pstride,
                                               grid + LAYOUT * D->grid_off, G, S, B, (cx0 + lc % ncx) * e,
                                               (cy0 + lc / ncx % ncy) * e, (cz0 + lc / ncx / ncy) * e);
         __syncthreads();  // the next cell reuses the shared memory
@@ -767,8 +766,9 @@ template <int KIND, bool ON, int NOFF, int ZB, int LAYOUT>
 int launch_batch_z(const BatchLaunch& L, const TipSites& S) {
     batch_grid_build_kernel<KIND, ON, NOFF, ZB, LAYOUT><<<L.blocks, L.block, 0, L.st>>>(
         L.n_mol, L.mols, L.atoms, L.params, L.pstride, L.grid, S);
+    if (KIND != SPM_KIND_LJ) return check_launch("spm_batch_grid_build");
     static const FarTab tab = make_far_tab();
-    const auto kern = batch_grid_block_kernel<KIND, ON, NOFF, LAYOUT>;
+    const auto kern = batch_grid_block_kernel<ON, NOFF, LAYOUT>;
     const size_t smem = sizeof(FarShared<NOFF>);
     const int threads = (int)(L.block.x * L.block.y);
     int dev = 0, sms = 0, per_sm = 0;

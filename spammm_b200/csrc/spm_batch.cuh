@@ -11,7 +11,7 @@
 
 namespace spm {
 
-// Atoms from which a force grid is built in blocks with a far field (grid_build.cu); the same for a batch's
+// Atoms from which an LJ force grid is built in blocks with a far field (grid_build.cu); the same for a batch's
 // molecules and a single grid.
 constexpr int SPM_FAR_MIN_ATOMS = 256;
 constexpr int SPM_FAR_BLOCK = 16;                // nodes per block edge

@@ -11,7 +11,6 @@ constexpr int FB = SPM_FAR_BLOCK;
 constexpr int FP = 8;
 constexpr int FN = FP * FP * FP;
 constexpr float FAR_RATIO = 9.f;
-constexpr float FAR_KH = 1.5f;
 constexpr int FAR_FEWEST = 8;        // far atoms that pay for an interpolation (it costs about 4 atoms at the nodes)
 
 // Lagrange weights of the Chebyshev points c at the nodes of a block (L), and of a

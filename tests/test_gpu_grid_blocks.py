@@ -2,9 +2,9 @@
 Chebyshev points (build_cell, grid_build.cu), against the FP64 pair sums.
 
 Bound per channel: 1e-5 S (S the sum of the atoms' contribution magnitudes) + the float32 node-coordinate
-term of test_gpu_scale.py.  A pair term errs by up to 2e-6 (rsqrt.approx to the 13th power) or, for Morse,
-4e-6 (the float32 exponent of up to 40), the interpolation adds at most 5e-7 of an atom's largest value in
-a block, which is less than four times its value at any node of a block nine half-edges away.
+term of test_gpu_scale.py.  A pair term errs by up to 2e-6 (rsqrt.approx to the 13th power) or, for Morse
+(direct sums), 4e-6 (the float32 exponent of up to 40); the interpolation adds at most 1e-6 of an LJ atom's
+force at the node.
 """
 import numpy as np
 import pytest
@@ -62,13 +62,12 @@ def test_against_pair_sums(cuda, kind, na, sites):
     _check(kind, atoms, prm, (97, 65, 81), (-12.0, -5.0, -4.0), (0.1, 0, 0), (0, 0.1, 0), (0, 0, 0.1), sites)
 
 
-@pytest.mark.parametrize("kind", [0, 1])
-@pytest.mark.parametrize("na", [31, 32, 57, 120, 255])
-def test_molecules_are_summed_directly(cuda, kind, na):
-    """Below 256 atoms a node's bits are those of its own pair sums: the box around it does not matter (a
-    spacing of 1/8, so that both boxes have the same node coordinates)."""
+@pytest.mark.parametrize("kind,na", [(k, na) for k in (0, 1) for na in (31, 32, 57, 120, 255)] + [(1, 256), (1, 600)])
+def test_molecules_and_morse_are_summed_directly(cuda, kind, na):
+    """Below 256 atoms, and for Morse at any size, a node's bits are those of its own pair sums: the box around it
+    does not matter (spacings of 1/8 and 1/16, so that both boxes have the same node coordinates)."""
     atoms, prm = _system(na, kind, 6.0)
-    h, n, cut = 0.125, (70, 61, 66), (5, 3, 7)
+    h, n, cut = 0.0625 if kind else 0.125, (70, 61, 66), (5, 3, 7)
     vec = [np.array(v, np.float32) for v in ((h, 0, 0, 0), (0, h, 0, 0), (0, 0, h, 0))]
     Qs, QZs = (np.array(v, np.float32) for v in BOTH)
     p0 = np.array([-4.5, -3.75, -1.0, 0], np.float32)
