@@ -322,12 +322,17 @@ struct FarShared {
 };
 
 // Far of the cube: the pair law and every off-node charge (seen from the node moved by its offset).
-// A NaN position is near.
+// Alone, r^-13 varies too fast for the points at this ratio (9e-5 of the local force): the distance must also be
+// at least 1.9 times that of the law's minimum, (2 c12 / c6)^(1/6), which holds by itself from about 0.1 A spacing
+// on.  Worst error of the LJ force at both limits 2e-7; without the second one 2e-6 at 0.08 A, 4e-5 at 0.05, 9e-5 at
+// 0.02.  Laws of another shape (c6 <= 0 or c12 < 0) and NaN positions or parameters are near.
 template <int NOFF>
-__device__ __forceinline__ bool is_far(const FarCube& C, const TipSites& S, float4 a) {
+__device__ __forceinline__ bool is_far(const FarCube& C, const TipSites& S, float4 a, const float* __restrict__ pr) {
     const float dx = C.x - a.x, dy = C.y - a.y, dz = C.z - a.z;
     const float dxy2 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
-    bool far = __fmaf_rn(dz, dz, dxy2) >= C.lim2;
+    const float r2 = __fmaf_rn(dz, dz, dxy2);
+    const float c12 = __ldg(pr + 1);
+    bool far = r2 >= C.lim2 && c12 >= 0.f && 94.f * c12 <= __ldg(pr) * r2 * r2 * r2;
 #pragma unroll
     for (int k = 0; k < NOFF; k++) {
         const float dk = __fadd_rn(dz, S.qz[k]);
@@ -336,7 +341,7 @@ __device__ __forceinline__ bool is_far(const FarCube& C, const TipSites& S, floa
     return far;
 }
 
-// Stages the atoms of [c0, c0 + FAR_CHUNK) that satisfy pick(atom), in atom order; returns
+// Stages the atoms of [c0, c0 + FAR_CHUNK) that satisfy pick(atom, parameter row), in atom order; returns
 // their number to every thread.
 template <int NOFF, class Pick>
 __device__ __forceinline__ int gather_atoms(FarShared<NOFF>& M, int tid, int nthr, int c0, int na,
@@ -351,7 +356,7 @@ __device__ __forceinline__ int gather_atoms(FarShared<NOFF>& M, int tid, int nth
         bool take = false;
         if (j < c1) {
             a = __ldg(atoms + j);
-            take = pick(a);
+            take = pick(a, params + (size_t)j * pstride);
         }
         const unsigned m = __ballot_sync(0xffffffffu, take);
         __syncthreads();  // the previous round's warp counts and the previous chunk's atoms are read
@@ -376,11 +381,11 @@ __device__ __forceinline__ int gather_atoms(FarShared<NOFF>& M, int tid, int nth
 
 template <class Pick>
 __device__ __forceinline__ int count_atoms(int tid, int nthr, int na, const float4* __restrict__ atoms,
-                                           const Pick& pick) {
+                                           const float* __restrict__ params, int pstride, const Pick& pick) {
     int n = 0;
     for (int b = 0; b < na; b += nthr) {
         const int j = b + tid;
-        n += __syncthreads_count(j < na && pick(__ldg(atoms + j)));
+        n += __syncthreads_count(j < na && pick(__ldg(atoms + j), params + (size_t)(j < na ? j : 0) * pstride));
     }
     return n;
 }
@@ -468,8 +473,8 @@ __device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int c
     constexpr int ZP = ZB / 2;
     const int nthr = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
     const FarCube C2 = far_cube(G, x0, y0, z0, SPM_FAR_CELL);
-    auto far2 = [&](float4 a) { return is_far<NOFF>(C2, S, a); };
-    const bool use2 = count_atoms(tid, nthr, na, atoms, far2) >= FAR_FEWEST;
+    auto far2 = [&](float4 a, const float* pr) { return is_far<NOFF>(C2, S, a, pr); };
+    const bool use2 = count_atoms(tid, nthr, na, atoms, params, pstride, far2) >= FAR_FEWEST;
     if (use2) {
         far_points<ON, NOFF>(M, tid, nthr, na, atoms, params, pstride, G, S, C2, far2);
         for (int i = tid; i < FN; i += nthr) M.group[i] = M.part[0][i];
@@ -482,12 +487,12 @@ __device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int c
             continue;  // CTA-uniform: no node of this block is stored
         const FarCube C1 = far_cube(G, bx, by, bz, FB);
         // an atom of this block alone: not in the group's field
-        auto own = [&](float4 a) { return !(use2 && is_far<NOFF>(C2, S, a)); };
-        auto far1 = [&](float4 a) { return own(a) && is_far<NOFF>(C1, S, a); };
-        const int nfar = count_atoms(tid, nthr, na, atoms, far1);
+        auto own = [&](float4 a, const float* pr) { return !(use2 && is_far<NOFF>(C2, S, a, pr)); };
+        auto far1 = [&](float4 a, const float* pr) { return own(a, pr) && is_far<NOFF>(C1, S, a, pr); };
+        const int nfar = count_atoms(tid, nthr, na, atoms, params, pstride, far1);
         const bool use1 = nfar >= FAR_FEWEST, field = use1 || use2;
-        auto near1 = [&](float4 a) {
-            return own(a) && !(use1 && is_far<NOFF>(C1, S, a));
+        auto near1 = [&](float4 a, const float* pr) {
+            return own(a, pr) && !(use1 && is_far<NOFF>(C1, S, a, pr));
         };
         float4* stage = M.part[1];  // 1024 float4: parts 1 and 2
         __syncthreads();            // the group's copy, the previous block's stage

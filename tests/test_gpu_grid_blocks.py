@@ -17,6 +17,7 @@ from test_gpu_scale import pos_term
 
 pytestmark = pytest.mark.gpu
 
+NONE = ([0, 0, 0, 0], [0, 0, 0, 0])
 ON = ([-0.05, 0, 0, 0], [0, 0, 0, 0])
 OFF = ([0, -0.1, 0.1, 0], [0, 1.8, 3.6, 0])
 BOTH = ([-0.05, 0.2, -0.1, 0.05], [0, -0.7, 1.8, 3.6])
@@ -34,7 +35,7 @@ def _system(na, kind, extent, seed=3):
     return atoms, prm.astype(np.float32)
 
 
-def _check(kind, atoms, prm, n, p0, dA, dB, dC, sites):
+def _check(kind, atoms, prm, n, p0, dA, dB, dC, sites, tol_sum=1e-5, tol_rel=2e-5):
     p0, dA, dB, dC = (np.array([*v, 0], np.float32) for v in (p0, dA, dB, dC))
     Qs, QZs = (np.array(v, np.float32) for v in sites)
     g = gpu.grid_build(kind, atoms, prm, n, p0, dA, dB, dC, Qs, QZs).cpu().numpy().reshape(-1, 4).astype(np.float64)
@@ -49,7 +50,7 @@ def _check(kind, atoms, prm, n, p0, dA, dB, dC, sites):
     cap = np.minimum(1.0, 100.0 / np.abs(ref[:, 3]))[:, None]
     ref, S = ref * cap, O.pair_fe_abs(kind, a64, p64, q, Qs, QZs) * cap
     err = np.abs(g - ref)
-    bad = err > 1e-5 * S + 2e-5 * np.abs(ref) + pos_term(q, a64, ref)
+    bad = err > tol_sum * S + tol_rel * np.abs(ref) + pos_term(q, a64, ref)
     assert not bad.any(), f"{bad.sum()} values out of bound, worst err/S {(err / S).max():.2e}"
 
 
@@ -90,6 +91,28 @@ def test_spacings_and_skew_cells(cuda, kind):
     _check(kind, atoms, prm, (70, 50, 60), (-14.0, -9.0, 1.0), (0.05, 0, 0), (0, 0.16, 0), (0, 0, 0.1), ON)
     _check(kind, atoms, prm, (90, 80, 50), (-8.0, -8.0, 2.0), (0.1, 0, 0.01), (0.05, 0.0866, -0.01), (0, 0, 0.12), BOTH)
     _check(kind, atoms, prm, (40, 40, 30), (-14.0, -14.0, 1.0), (0.35, 0, 0), (0, 0.35, 0), (0, 0, 0.35), ON)
+
+
+@pytest.mark.parametrize("h", [0.02, 0.03, 0.05, 0.08, 0.1])
+@pytest.mark.parametrize("sites", [NONE, ON], ids=["none", "on"])
+def test_fine_spacings(cuda, h, sites):
+    """Nine half-edges of a block are 1.4 to 6.8 A here: the core of the LJ law must not be interpolated.  Bound: a
+    pair term's 2e-6 and the interpolation's 1e-6, of the terms' magnitudes."""
+    atoms, prm = _system(300, 0, 6.0)
+    n = (160, 160, 128)
+    _check(0, atoms, prm, n, (-80 * h, -80 * h, 3.0), (h, 0, 0), (0, h, 0), (0, 0, h), sites, tol_sum=3e-6, tol_rel=0.0)
+
+
+def test_laws_of_another_shape(cuda):
+    """Atoms without a minimum (no attraction, no repulsion, signs turned) and charges alone, on fine nodes."""
+    atoms, prm = _system(320, 0, 9.0)
+    prm[0::5, 0] = 0.0
+    prm[1::5, 1] = 0.0
+    prm[2::5] *= -1.0
+    prm[3::5] = 0.0
+    for h in (0.03, 0.1):
+        _check(0, atoms, prm, (96, 96, 64), (-48 * h, -48 * h, 3.4), (h, 0, 0), (0, h, 0), (0, 0, h), ON, tol_sum=3e-6,
+               tol_rel=0.0)
 
 
 def test_atoms_that_are_not_finite_stay_in_the_sum(cuda):
