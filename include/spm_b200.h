@@ -428,7 +428,7 @@ typedef struct spm_batch_mol {
 /* Launch shapes; spm_batch_default_shape() gives a valid default, the
  * autotuner in the Python package searches the rest. */
 typedef struct spm_batch_shape {
-    int gb_ty;          /* grid build by direct sums (Morse; LJ below 256 atoms): CTA = 32 x gb_ty threads, gb_ty in {2,4,8} */
+    int gb_ty;          /* grid build by direct sums (molecules, Morse): CTA = 32 x gb_ty threads, gb_ty in {2,4,8} */
     int gb_zb;          /* the same: nodes along z per thread, 8 or 16 */
     int rx_threads;     /* relaxation CTA size: 64, 128 or 256 */
     int rx_tile_h;      /* relaxation pixel tile: (32/rx_tile_h) x rx_tile_h pixels, power of two <= 32 */

@@ -19,10 +19,10 @@
 //     non-zero offset get their own rsqrt.
 // Transcendentals use MUFU approximations (rsqrt.approx, ex2.approx).
 //
-// That direct sum is for molecules and for Morse.  LJ systems of SPM_FAR_MIN_ATOMS
-// atoms or more (slabs): the nodes are built in blocks of 16^3, each atom at a block's nodes only when it is
-// near the block; the smooth field of the distant atoms is evaluated at 8^3
-// Chebyshev points of the block and interpolated (build_cell below).
+// That direct sum is for molecules and for Morse.  The nodes of larger LJ systems
+// (far_grid: slabs of 256 atoms or more) are built in blocks of 16^3, each atom at a
+// block's nodes only when it is near the block; the smooth field of the distant atoms
+// is evaluated at 8^3 Chebyshev points of the block and interpolated (build_cell below).
 #include "spm_internal.cuh"
 #include "spm_batch.cuh"
 #include "spm_f32x2.cuh"
@@ -639,7 +639,7 @@ int launch_blocks(int na, const float4* atoms, const float* params, int pstride,
 template <int KIND, bool ON>
 int launch_noff(int noff, dim3 grd, dim3 block, cudaStream_t st, int na, const float4* atoms, const float* params,
                 int pstride, float4* out, const GridGeom& G, const TipSites& S) {
-    if (KIND == SPM_KIND_LJ && na >= SPM_FAR_MIN_ATOMS) {
+    if (KIND == SPM_KIND_LJ && far_grid(na, G.nx, G.ny, &G.dA.x, &G.dB.x, &G.dC.x)) {
         switch (noff) {
             case 0: return launch_blocks<ON, 0>(na, atoms, params, pstride, out, G, S, st);
             case 1: return launch_blocks<ON, 1>(na, atoms, params, pstride, out, G, S, st);
@@ -696,7 +696,7 @@ batch_grid_build_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
                         const float* __restrict__ params, int pstride, float4* __restrict__ grid, TipSites S) {
     const long long tile = blockIdx.x;
     const spm_batch_mol* D = mols + SPM_MOL_BY(tile_off, mols, n_mol, tile);
-    if (KIND == SPM_KIND_LJ && D->n_atoms >= SPM_FAR_MIN_ATOMS) return;  // built by batch_grid_block_kernel
+    if (KIND == SPM_KIND_LJ && far_grid(*D)) return;  // built by batch_grid_block_kernel
     const int ty = blockDim.y;
     const int z_lo = D->z_lo, nzs = D->nz_slab;
     const StoreBox B = {D->x_lo, D->nx_slab, D->y_lo, D->ny_slab, z_lo, z_lo + nzs};
@@ -721,7 +721,7 @@ batch_grid_build_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
                                            z_lo + (int)bz * ZB);
 }
 
-// The LJ molecules of SPM_FAR_MIN_ATOMS atoms or more: persistent CTAs over their lattice cells (block_off:
+// The LJ molecules that take blocks (far_grid): persistent CTAs over their lattice cells (block_off:
 // prefix of cells over the batch), each cell's nodes inside the molecule's box as grid_block_kernel builds
 // them.
 template <bool ON, int NOFF, int LAYOUT>

@@ -11,15 +11,29 @@
 
 namespace spm {
 
-// Atoms from which an LJ force grid is built in blocks with a far field (grid_build.cu); the same for a batch's
-// molecules and a single grid.
 constexpr int SPM_FAR_MIN_ATOMS = 256;
 constexpr int SPM_FAR_BLOCK = 16;                // nodes per block edge
 constexpr int SPM_FAR_CELL = 2 * SPM_FAR_BLOCK;  // lattice cells: groups of 2^3 blocks
 
-// Lattice cells that a molecule's box of stored nodes meets; 0 below SPM_FAR_MIN_ATOMS.
+// Whether an LJ force grid (nx, ny: of the full grid) is built in blocks with a far field (grid_build.cu); the
+// same for a batch's molecules and a single grid.  Not where it would not pay: a grid of fewer rows or columns
+// than a block leaves its threads idle (256 atoms, 1000 x 1 x 100 nodes: 101 us directly, 131 in blocks; 500 x 8 x
+// 100 128 and 133; 500 x 16 x 100 208 and 148; from 400 to 1200 atoms 138 and 148 to 330 and 221), and on coarse
+// nodes nothing is far (400 atoms, 0.35 A: 1468 and 1311 us, 1 A: 5% longer in blocks, 2 A 41%).  Comparisons
+// only: host and device decide alike.
+__host__ __device__ inline bool far_grid(int na, int nx, int ny, const float* dA, const float* dB, const float* dC) {
+    if (na < SPM_FAR_MIN_ATOMS || (na < 2 * SPM_FAR_MIN_ATOMS && (nx < SPM_FAR_BLOCK || ny < SPM_FAR_BLOCK))) return false;
+    for (int k = 0; k < 3; k++)
+        if (!(fabsf(dA[k]) <= 0.5f && fabsf(dB[k]) <= 0.5f && fabsf(dC[k]) <= 0.5f)) return false;
+    return true;
+}
+__host__ __device__ inline bool far_grid(const spm_batch_mol& D) {
+    return far_grid(D.n_atoms, D.nx, D.ny, D.dA, D.dB, D.dC);
+}
+
+// Lattice cells that a molecule's box of stored nodes meets; 0 without a far field.
 __host__ __device__ inline long long far_cells(const spm_batch_mol& D) {
-    if (D.n_atoms < SPM_FAR_MIN_ATOMS) return 0;
+    if (!far_grid(D)) return 0;
     const int e = SPM_FAR_CELL;
     return ((long long)(D.x_lo + D.nx_slab - 1) / e - D.x_lo / e + 1) *
            ((long long)(D.y_lo + D.ny_slab - 1) / e - D.y_lo / e + 1) *

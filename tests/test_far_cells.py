@@ -31,3 +31,16 @@ def test_block_prefix_covers_each_box(nas):
             cells *= len({i // 32 for i in range(lo, lo + n)})
         at += cells
     assert ctypes.sizeof(_lib.BatchMol) % 8 == 0
+
+
+@pytest.mark.parametrize("na,n,step,far", [(300, (40, 15, 64), 0.1, False), (300, (40, 16, 64), 0.1, True),
+                                           (511, (15, 40, 64), 0.1, False), (512, (15, 15, 64), 0.1, True),
+                                           (600, (40, 40, 40), 0.5, True), (600, (40, 40, 40), 0.55, False),
+                                           (255, (64, 64, 64), 0.1, False), (256, (64, 64, 64), 0.1, True)])
+def test_which_grids_take_blocks(na, n, step, far):
+    xs = (np.arange(4) * step).astype(np.float32)
+    plan = BatchPlan([BatchItem(atoms=np.zeros((k, 4), np.float32), params=np.ones((k, 2), np.float32),
+                                origin=np.array([-1.5 * step, -1.5 * step, 0.0]), step=step, ngrid=n, xs=xs, ys=xs,
+                                z_top=step * 30, nz=2) for k in (na, 4)])
+    plan.prepare(_lib.lib().spm_batch_default_shape())
+    assert (plan.mols[1].block_off > 0) == far

@@ -65,10 +65,20 @@ def test_against_pair_sums(cuda, kind, na, sites):
 
 @pytest.mark.parametrize("kind,na", [(k, na) for k in (0, 1) for na in (31, 32, 57, 120, 255)] + [(1, 256), (1, 600)])
 def test_molecules_and_morse_are_summed_directly(cuda, kind, na):
-    """Below 256 atoms, and for Morse at any size, a node's bits are those of its own pair sums: the box around it
-    does not matter (spacings of 1/8 and 1/16, so that both boxes have the same node coordinates)."""
+    """Below 256 atoms, and for Morse at any size, a node's bits are those of its own pair sums."""
+    _same_in_any_box(kind, na, 0.0625 if kind else 0.125, (70, 61, 66))
+
+
+@pytest.mark.parametrize("na,n,h", [(300, (200, 15, 66), 0.125), (511, (15, 200, 66), 0.125), (300, (90, 61, 66), 0.75)])
+def test_thin_and_coarse_boxes_are_summed_directly(cuda, na, n, h):
+    """Grids where blocks do not pay: fewer columns than a block's and not many atoms, or nodes half an Angstrom apart."""
+    _same_in_any_box(0, na, h, n)
+
+
+def _same_in_any_box(kind, na, h, n):
+    """The box around a node does not matter (dyadic spacings, so that both boxes have the same node coordinates)."""
     atoms, prm = _system(na, kind, 6.0)
-    h, n, cut = 0.0625 if kind else 0.125, (70, 61, 66), (5, 3, 7)
+    cut = (5, 3, 7)
     vec = [np.array(v, np.float32) for v in ((h, 0, 0, 0), (0, h, 0, 0), (0, 0, h, 0))]
     Qs, QZs = (np.array(v, np.float32) for v in BOTH)
     p0 = np.array([-4.5, -3.75, -1.0, 0], np.float32)
