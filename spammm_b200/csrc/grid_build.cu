@@ -163,8 +163,9 @@ __device__ __forceinline__ float4 atom_params(const float* __restrict__ pr) {
 }
 
 // The ZP node pairs of column (xl, yl) (box indices) from layer ic0 on, capped, into the box's storage;
-// layers outside the box are left out.
-template <int ZP, int LAYOUT>
+// layers above the box are left out, and with BELOW those below it (build_tile starts inside the box: the extra
+// test there costs 2.6% of a batch's slabs).
+template <int ZP, int LAYOUT, bool BELOW>
 __device__ __forceinline__ void store_column(float4* __restrict__ out, const StoreBox& B, int xl, int yl, int ic0,
                                              const f2 (&fx)[ZP], const f2 (&fy)[ZP], const f2 (&fz)[ZP],
                                              const f2 (&fe)[ZP]) {
@@ -179,7 +180,7 @@ __device__ __forceinline__ void store_column(float4* __restrict__ out, const Sto
         for (int h = 0; h < 2; h++) {
             const int ic = ic0 + 2 * p + h;
             if (ic >= B.zst_hi) break;
-            if (ic < B.zst_lo) continue;
+            if (BELOW && ic < B.zst_lo) continue;
             float4 o = make_float4(x[h], y[h], z[h], e[h]);
             // |E| > 100 cap of the reference builders (AFM.cl:1053-1054)
             // (the division only where it can scale: 100/|E| < 1 needs |E| > 100; NaN compares false)
@@ -268,7 +269,7 @@ __device__ __forceinline__ void build_tile(int na, const float4* __restrict__ at
         __syncthreads();
     }
     if (!active) return;
-    store_column<ZP, LAYOUT>(out, B, xl, yl, ic0, fx, fy, fz, fe);
+    store_column<ZP, LAYOUT, false>(out, B, xl, yl, ic0, fx, fy, fz, fe);
 }
 
 template <int KIND, bool ON, int NOFF>
@@ -582,7 +583,7 @@ __device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int c
                     }
                 }
             }
-            if (active) store_column<ZP, LAYOUT>(out, B, xl, yl, ic0, fx, fy, fz, fe);
+            if (active) store_column<ZP, LAYOUT, true>(out, B, xl, yl, ic0, fx, fy, fz, fe);
         }
     }
 }
@@ -602,7 +603,6 @@ __device__ __forceinline__ void load_far_tab(FarShared<NOFF>& M, const FarTab& t
 // x 240 grid (128 threads 2.25, 8 nodes each 2.36; 0.47 ms against 0.71 and 0.44 on 527 atoms, 243 x 138 x
 // 98).  The differences from one point cost 2% since.
 constexpr int FAR_THREADS = 256;
-constexpr long long FAR_CTAS = 222;  // CTAs that fill a 148-SM part one and a half times
 
 // A whole grid: one CTA per lattice cell, or per 4, 2 or 1 blocks of a group while the groups alone would
 // leave SMs idle (each CTA then sums the group's field itself: the same values).
@@ -629,8 +629,11 @@ int launch_blocks(int na, const float4* atoms, const float* params, int pstride,
         return set_error(SPM_ERR_CUDA, "spm_grid_build: cannot enable %zu B of shared memory", smem);
     const int e = SPM_FAR_CELL;
     const long long cells = (long long)((G.nx + e - 1) / e) * ((G.ny + e - 1) / e) * ((G.nz + e - 1) / e);
-    int split = 1;
-    while (split < 8 && cells * split < FAR_CTAS) split *= 2;
+    int dev = 0, sms = 0, split = 1;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return set_error(SPM_ERR_CUDA, "spm_grid_build: cannot query the device");
+    while (split < 8 && cells * split < 3LL * sms / 2) split *= 2;
     kern<<<dim3((G.nx + e - 1) / e * split, (G.ny + e - 1) / e, (G.nz + e - 1) / e), FAR_THREADS, smem, st>>>(
         split, na, atoms, params, pstride, out, G, S, tab);
     return check_launch("spm_grid_build");
@@ -724,15 +727,18 @@ batch_grid_build_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const
 // The LJ molecules that take blocks (far_grid): persistent CTAs over their lattice cells (block_off:
 // prefix of cells over the batch), each cell's nodes inside the molecule's box as grid_block_kernel builds
 // them.
+constexpr int BATCH_FAR_THREADS = 128;  // 16 molecules of 300 to 600 atoms: 7.2 ms, 256 threads 7.4, 64 12.0
+
 template <bool ON, int NOFF, int LAYOUT>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(BATCH_FAR_THREADS, 4)
 batch_grid_block_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, const float4* __restrict__ atoms,
                         const float* __restrict__ params, int pstride, float4* __restrict__ grid, TipSites S,
                         const __grid_constant__ FarTab tab) {
     extern __shared__ __align__(16) unsigned char far_smem[];
     FarShared<NOFF>& M = *reinterpret_cast<FarShared<NOFF>*>(far_smem);
-    load_far_tab(M, tab);
     const long long total = (long long)mols[n_mol - 1].block_off + far_cells(mols[n_mol - 1]);
+    if (blockIdx.x >= total) return;  // a batch of molecules only: 5 us for the launch
+    load_far_tab(M, tab);
     for (long long c = blockIdx.x; c < total; c += gridDim.x) {
         const spm_batch_mol* D = mols + SPM_MOL_BY(block_off, mols, n_mol, c);
         const int e = SPM_FAR_CELL;
@@ -775,15 +781,14 @@ int launch_batch_z(const BatchLaunch& L, const TipSites& S) {
     static const FarTab tab = make_far_tab();
     const auto kern = batch_grid_block_kernel<ON, NOFF, LAYOUT>;
     const size_t smem = sizeof(FarShared<NOFF>);
-    const int threads = (int)(L.block.x * L.block.y);
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
         cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BATCH_FAR_THREADS, smem) != cudaSuccess)
         return set_error(SPM_ERR_CUDA, "spm_batch_grid_build: cannot prepare the block kernel");
-    kern<<<sms * (per_sm > 0 ? per_sm : 1), L.block, smem, L.st>>>(L.n_mol, L.mols, L.atoms, L.params, L.pstride,
-                                                                   L.grid, S, tab);
+    kern<<<sms * (per_sm > 0 ? per_sm : 1), BATCH_FAR_THREADS, smem, L.st>>>(L.n_mol, L.mols, L.atoms, L.params,
+                                                                             L.pstride, L.grid, S, tab);
     return check_launch("spm_batch_grid_build");
 }
 
