@@ -346,9 +346,9 @@ int spm_adjoint_grid_params(int kind, int n_atoms, const float* atoms, const flo
 long long spm_adjoint_grid_scratch_bytes(int n_atoms, long long n_state);
 
 /* The same gradients node by node: the states' w*ubar are summed onto the
- * nx*ny*nz grid nodes (64-bit fixed point, scale 2^42 / max|ubar|: exact, at
- * most 2^20 states per node), each touched node then contracted once per atom
- * (FP64 sums, fixed order) instead of once per state and corner.  Results as
+ * nx*ny*nz grid nodes (64-bit fixed point in units of 2^-42 max|ubar|, coarser
+ * beyond 2^20 states so that no sum can wrap), each touched node then contracted
+ * once per atom (FP64 sums, fixed order) instead of once per state and corner.  Results as
  * spm_adjoint_grid_params up to rounding.  1 <= n_atoms, n_state; scratch >=
  * spm_adjoint_grid_nodes_scratch_bytes (32 bytes per grid node; only the box of
  * touched nodes is used), 16-byte aligned, its content arbitrary. */

@@ -1034,6 +1034,13 @@ batch_scatter_tile_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, uns
 // its evaluations and conversions to FP64: the call with 38 atoms takes 826 -> 233 us, with 120 atoms on 128 x
 // 128 x 40 states 3917 -> 491, on 24 x 24 x 20 states 108 either way.
 // Only the box of touched nodes is cleared and read.
+// The sums' unit is 2^-bits of the scan's largest |ubar| (the next power of two): bits = 42, less where more than
+// 2^20 states could add up on one node beyond 2^62.
+inline int nodes_bits(long long n_state) {
+    int bits = 42;
+    while (bits > 0 && n_state > (1LL << (62 - bits))) bits--;
+    return bits;
+}
 constexpr int GN_THREADS = 256;
 constexpr int GN_CTAS = 592;  // four per SM of a 148-SM part; fixed, so that the sums' order is
 
@@ -1110,9 +1117,9 @@ grid_nodes_clear_kernel(GridView G, const NodesHead* __restrict__ H, ulonglong2*
 // Thread per state.  Consecutive lanes are consecutive z-steps of a stroke: a lane whose cell sits on the next
 // lane's (same column, one layer above) takes over that lane's upper-layer sums, as batch_scatter_kernel does.
 __global__ void __launch_bounds__(GN_THREADS)
-grid_nodes_scatter_kernel(GridView G, int nz_steps, long long n_state, const float4* __restrict__ PPs,
-                          const float4* __restrict__ ubar, const NodesHead* __restrict__ H,
-                          unsigned long long* __restrict__ q) {
+grid_nodes_scatter_kernel(GridView G, int nz_steps, long long n_state, int bits,
+                          const float4* __restrict__ PPs, const float4* __restrict__ ubar,
+                          const NodesHead* __restrict__ H, unsigned long long* __restrict__ q) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const long long st = (long long)blockIdx.x * GN_THREADS + threadIdx.x;
@@ -1125,7 +1132,7 @@ grid_nodes_scatter_kernel(GridView G, int nz_steps, long long n_state, const flo
         C = corners_of<false>(G, mk3(pp.x, pp.y, pp.z));
         valid = C.ok;
     }
-    const double scale = pow2(42 - scale_exp(H->umax));
+    const double scale = pow2(bits - scale_exp(H->umax));
     const long long stroke = st / nz_steps;
     auto above = [&](bool v, long long s, int x, int y, int z1) {  // that lane's lower layer is (s, x, y, z1)'s upper
         return valid && v && s == stroke && x == C.x[0] && y == C.y[0] && z1 == C.z[0];
@@ -1165,7 +1172,7 @@ grid_nodes_scatter_kernel(GridView G, int nz_steps, long long n_state, const flo
 template <int KIND>
 __global__ void __launch_bounds__(GN_THREADS, 3)
 grid_nodes_atoms_kernel(int na, const float4* __restrict__ atoms, const float* __restrict__ params, int pstride,
-                        Sites S, NodeGeom NG, GridView G, const NodesHead* __restrict__ H,
+                        Sites S, NodeGeom NG, GridView G, int bits, const NodesHead* __restrict__ H,
                         const ulonglong2* __restrict__ q, double* __restrict__ partial) {
     __shared__ float4 s_p[GN_THREADS], s_g[GN_THREADS];
     __shared__ int s_w[GN_THREADS / 32];
@@ -1173,7 +1180,7 @@ grid_nodes_atoms_kernel(int na, const float4* __restrict__ atoms, const float* _
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const NodesBox B(H, G);
     const long long total = B.total();
-    const double inv = pow2(scale_exp(H->umax) - 42);
+    const double inv = pow2(scale_exp(H->umax) - bits);
     for (int a0 = 0; a0 < na; a0 += GN_THREADS) {
         const int nslot = min(na - a0, GN_THREADS), P = GN_THREADS / nslot, ph = t / nslot;
         const bool act = ph < P;
@@ -2195,14 +2202,15 @@ extern "C" int spm_adjoint_grid_params_nodes(int kind, int n_atoms, const float*
     const float4* a4 = reinterpret_cast<const float4*>(atoms);
     const int pstride = kind == SPM_KIND_MORSE ? 4 : 2;
     const GridView G = view_of(nullptr, nx, ny, nz, p);
+    const int bits = nodes_bits(n_state);
     cudaStream_t st = as_stream(stream);
     if (cudaMemsetAsync(H, 0, sizeof(NodesHead), st) != cudaSuccess)
         return set_error(SPM_ERR_CUDA, "spm_adjoint_grid_params_nodes: memset failed");
     grid_nodes_box_kernel<<<(unsigned)(blocks < GN_CTAS ? blocks : GN_CTAS), GN_THREADS, 0, st>>>(G, n_state, pp4, ub4, H);
     grid_nodes_clear_kernel<<<GN_CTAS, GN_THREADS, 0, st>>>(G, H, reinterpret_cast<ulonglong2*>(q));
-    grid_nodes_scatter_kernel<<<(unsigned)blocks, GN_THREADS, 0, st>>>(G, p->nz, n_state, pp4, ub4, H, q);
+    grid_nodes_scatter_kernel<<<(unsigned)blocks, GN_THREADS, 0, st>>>(G, p->nz, n_state, bits, pp4, ub4, H, q);
     const auto kern = kind == SPM_KIND_MORSE ? grid_nodes_atoms_kernel<SPM_KIND_MORSE> : grid_nodes_atoms_kernel<SPM_KIND_LJ>;
-    kern<<<GN_CTAS, GN_THREADS, 0, st>>>(n_atoms, a4, params, pstride, S, NG, G, H,
+    kern<<<GN_CTAS, GN_THREADS, 0, st>>>(n_atoms, a4, params, pstride, S, NG, G, bits, H,
                                          reinterpret_cast<const ulonglong2*>(q), part);
     fold_chunks_kernel<<<dim3((unsigned)n_atoms, 6), 256, 0, st>>>(part, GN_CTAS, 6, grad);
     sum_rows_kernel<<<(unsigned)rb, 256, 0, st>>>(reinterpret_cast<const float4*>(dk), n_state, dkpart);

@@ -77,3 +77,18 @@ def test_no_weight_and_weights_that_are_not_finite(cuda, monkeypatch):
         args[12] = ub.copy()
         args[12][33, 2] = v
         assert not torch.isfinite(gpu.adjoint_grid_params(*args)[0]).any()
+
+
+@pytest.mark.parametrize("n_state", [(1 << 20) + 1, (1 << 22) + 12345])
+def test_every_state_on_one_node(cuda, n_state, monkeypatch):
+    """Like-signed adjoints of equal size on one node: 64-bit sums in units of 2^-42 would wrap beyond 2^21 states."""
+    args = list(_case(0, 9, 2, 1, seed=3))
+    n, o, step = (70, 66, 60), np.array([-7.0, -6.6, 2.0]), 0.2
+    PP = np.zeros((n_state, 4), np.float32)
+    PP[:, :3], PP[:, 3] = o + step * np.array([31, 33, 24]), 5
+    ub = np.tile(np.array([[0.0019, -0.00195, 0.0018, 0.0011]], np.float32), (n_state, 1))
+    args[11], args[12], args[13] = PP, ub, np.zeros_like(ub)
+    a, b = _both(tuple(args), monkeypatch)
+    for c in range(6):
+        d, s = float((a[0][:, c] - b[0][:, c]).norm()), float(a[0][:, c].norm())
+        assert d <= 5e-6 * s, f"column {c}: {d / max(s, 1e-300):.1e}"
