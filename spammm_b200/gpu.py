@@ -190,9 +190,14 @@ def adjoint_grid_params(kind, atoms, params_atoms, p0, dA, dB, dC, Qs, QZs, grid
     grad = torch.empty((na, 6), dtype=F64, device=atoms.device)
     dk_sum = torch.empty((4,), dtype=F64, device=atoms.device)
     hv = [hostvec(v) for v in (p0, dA, dB, dC, Qs, QZs)]
-    if na and n_state * na >= NODES_MIN_PAIRS and scan_params.nz and nx * ny * nz <= NODES_MAX_GRID:
+    scratch = None
+    if na and n_state * na >= NODES_MIN_PAIRS and scan_params.nz > 0 and nx * ny * nz <= NODES_MAX_GRID:
         nbytes = int(lib().spm_adjoint_grid_nodes_scratch_bytes(na, n_state, nx, ny, nz))
-        scratch = torch.empty(((nbytes + 15) // 16, 2), dtype=F64, device=atoms.device)
+        try:
+            scratch = torch.empty(((nbytes + 15) // 16, 2), dtype=F64, device=atoms.device)
+        except torch.OutOfMemoryError:
+            pass  # the gather needs a few MB
+    if scratch is not None:
         rc = lib().spm_adjoint_grid_params_nodes(int(kind), na, ptr(atoms), ptr(prm), *[hptr(h) for h in hv], nx, ny, nz,
                                                  ctypes.byref(scan_params), ptr(PPs), ptr(ubar), ptr(dk), n_state,
                                                  ptr(grad), ptr(dk_sum), ptr(scratch), stream_ptr())

@@ -92,3 +92,22 @@ def test_every_state_on_one_node(cuda, n_state, monkeypatch):
     for c in range(6):
         d, s = float((a[0][:, c] - b[0][:, c]).norm()), float(a[0][:, c].norm())
         assert d <= 5e-6 * s, f"column {c}: {d / max(s, 1e-300):.1e}"
+
+
+def test_gather_where_the_node_sums_do_not_fit(cuda, monkeypatch):
+    """The scratch of the node sums (32 bytes per grid node) cannot be had: the gather's gradients, as before."""
+    args = _case(0, 38, 200, 20, seed=5)
+    ref, nodes = _both(args, monkeypatch)
+    empty, refused = torch.empty, []
+
+    def short(*a, **k):
+        t = empty(*a, **k)
+        if t.numel() * t.element_size() > 8_000_000:
+            refused.append(t.numel())
+            raise torch.OutOfMemoryError("no memory")
+        return t
+
+    monkeypatch.setattr(torch, "empty", short)
+    got = gpu.adjoint_grid_params(*args)
+    assert refused and torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+    assert not torch.equal(nodes[0], ref[0])
