@@ -19,6 +19,7 @@
 // the per-atom parameter partials with a CTA per (atom, 128-scan chunk) that
 // reduces in shared memory in a fixed order; a second pass folds the chunks in
 // a fixed order.  No floating-point atomics: the gradient is bit-reproducible.
+#include <cmath>
 #include "spm_internal.cuh"
 #include "spm_fire.cuh"
 
@@ -199,7 +200,7 @@ __device__ __noinline__ double group_force2_f64(V3 p, V3 tip, int na, int sub, u
 // |x| ln 2 < 1.5e-6 |x|, and the force 2 K E0 e (e - 1), whose difference cancels near the minimum, by that
 // times e (1 + e) plus 2e-6 for its own products; a charge site's force by 2e-6 and by 4e-7 (|dz| + |qz|) / r
 // for the rounded offset; the sum of na terms adds na 2^-24 of their magnitudes.  The spring: 4e-7 of the
-// lengths times their stiffnesses (rotations, root, products) and of the force itself.
+// lengths times their stiffnesses (rotations by an orthonormal frame, root, products) and of the force itself.
 template <int NS, int LPP>
 __device__ __noinline__ float group_force_bound(V3 p, V3 tip, int na, int sub, unsigned gmask, const float4* s_pos,
                                                 const float4* s_m, const float* s_q, const Sites& S, float4 kk,
@@ -238,13 +239,14 @@ __device__ __noinline__ float group_force_bound(V3 p, V3 tip, int na, int sub, u
 // whole molecule staged in shared memory; each group runs its pixel's (z-step, FIRE step) sequence
 // with the stroke state held identically by every lane of the group.  Convergence is tested before
 // the update, and an FP32 "converged" is confirmed in FP64 -- unless the FP32 force is below the threshold by
-// more than its error bound, where FP64 cannot decide otherwise (most confirmations of molecules; beyond
-// BOUND_ATOMS atoms the bound of the sum's rounding nears the threshold and is not tried).  38 atoms, 100 x
+// more than its error bound, where FP64 cannot decide otherwise (most confirmations of molecules; `bound`: not
+// beyond BOUND_ATOMS atoms, where the bound of the sum's rounding nears the threshold, and not with a tip frame
+// that is not orthonormal, which stretches the spring's roundings).  38 atoms, 100 x
 // 100 pixels x 40 z-steps, at 16 lanes per pixel: 1686 -> 1405 us.  ident: the tip frame is x, y, z (the rotations change no value).
 template <int NS, int LPP, int HALVES>
 __global__ void __launch_bounds__(DX_THREADS)
 relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __restrict__ cMs,
-                    const float4* __restrict__ pts, int n_scan, spm_scan_params P, Sites S,
+                    const float4* __restrict__ pts, int n_scan, spm_scan_params P, Sites S, bool bound,
                     float4* __restrict__ FEs, float4* __restrict__ PPs) {
     extern __shared__ float4 smem[];
     float4* s_pos = smem;
@@ -299,7 +301,7 @@ relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __re
             const float f2 = dot3(f, f);
             bool below = false;
             if (f2 < P.f2conv) {
-                if (na <= BOUND_ATOMS) {
+                if (bound) {
                     const float far = sqrtf(f2) + group_force_bound<NS, LPP>(pos, tip, na, sub, gmask, s_pos, s_m, s_q,
                                                                              S, kk, d0, surf);
                     below = far * far < 0.999f * P.f2conv;
@@ -632,6 +634,16 @@ Sites make_sites(const float* Qs, const float* QZs, bool compact, int* ns) {
     return S;
 }
 
+bool orthonormal(const spm_scan_params& P) {
+    const float* r[3] = {P.tipA, P.tipB, P.tipC};
+    for (int i = 0; i < 3; i++)
+        for (int j = i; j < 3; j++) {
+            const float d = r[i][0] * r[j][0] + r[i][1] * r[j][1] + r[i][2] * r[j][2];
+            if (!(fabsf(d - (i == j ? 1.f : 0.f)) <= 1e-3f)) return false;
+        }
+    return true;
+}
+
 // Lanes per pixel of a scan: `atoms` atoms per lane, at least 4 and at most 32 lanes, more while the scan
 // leaves the GPU short of warps (fewer than ~8 warps per SM of a 148-SM part).
 int direct_lpp(int na, int n_scan, int atoms) {
@@ -668,7 +680,7 @@ int launch_direct(int na, const float* atoms, const float* cMs, const float* poi
     kern<<<blocks, threads, smem, st>>>(na, reinterpret_cast<const float4*>(atoms),
                                            reinterpret_cast<const float4*>(cMs),
                                            reinterpret_cast<const float4*>(points), n_scan, P, S,
-                                           reinterpret_cast<float4*>(FEs), reinterpret_cast<float4*>(PPs));
+                                           na <= BOUND_ATOMS && orthonormal(P), reinterpret_cast<float4*>(FEs), reinterpret_cast<float4*>(PPs));
     return check_launch("spm_relax_direct_morse");
 }
 
