@@ -25,6 +25,7 @@
 // This translation unit is compiled with -fmad=false: the only fused
 // multiply-adds are the explicit __fmaf_rn calls shared with the CPU oracle.
 #include <climits>
+#include <cmath>
 #include <type_traits>
 #include "spm_internal.cuh"
 #include "spm_fire.cuh"
@@ -190,7 +191,7 @@ __device__ __forceinline__ void pp_emit(const GridView& G, const PPFrame& F, V3 
         S.ident = PLAIN;
         newton_polish(FullCellFetchCached<IDX, PLAIN>{G, cache}, T, S, tip, pos, fe);
     }
-    const V3 r = PLAIN ? mk3(fe.x, fe.y, fe.z) : rotmat(mk3(fe.x, fe.y, fe.z), F.a, F.b, F.c);
+    const V3 r = rotmat(mk3(fe.x, fe.y, fe.z), F.a, F.b, F.c);
     *fe_out = make_float4(r.x, r.y, r.z, fe.w);
     const bool finite = isfinite(fe.x) && isfinite(fe.y) && isfinite(fe.z) && isfinite(fe.w) && isfinite(pos.x) &&
                         isfinite(pos.y) && isfinite(pos.z);
@@ -497,7 +498,7 @@ relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_sc
                     } else {
                         float4 g = interp_fe<IDX>(G, pos);
                         if constexpr (POLISH) polish_state<MODE, IDX, PLAIN>(G, a, b, c, kk, d0, surf, tip, q, g, T);
-                        const V3 r = PLAIN ? mk3(g.x, g.y, g.z) : rotmat(mk3(g.x, g.y, g.z), a, b, c);
+                        const V3 r = rotmat(mk3(g.x, g.y, g.z), a, b, c);
                         FEs[o] = make_float4(r.x, r.y, r.z, g.w);
                     }
                 }
@@ -603,13 +604,14 @@ int persistent_blocks(K kern, long long warps, int threads, int& blocks) {
     return SPM_OK;
 }
 
-// The scans relax_tile_kernel's PLAIN form covers.
+// The scans relax_tile_kernel's PLAIN form covers (a bias that is not finite reaches the other components through the
+// frame's zeros).
 bool plain_scan(int mode, const spm_scan_params& P) {
     const bool axis = P.dinvA[1] == 0.f && P.dinvA[2] == 0.f && P.dinvB[0] == 0.f && P.dinvB[2] == 0.f &&
                       P.dinvC[0] == 0.f && P.dinvC[1] == 0.f;
     const bool frame = P.tipA[0] == 1.f && P.tipA[1] == 0.f && P.tipA[2] == 0.f && P.tipB[0] == 0.f &&
                        P.tipB[1] == 1.f && P.tipB[2] == 0.f && P.tipC[0] == 0.f && P.tipC[1] == 0.f && P.tipC[2] == 1.f;
-    return axis && (mode == SPM_RELAX_STROKES || frame) && P.stiffness[3] == 0.f && (P.flags & SPM_FLAG_FIRE);
+    return axis && (mode == SPM_RELAX_STROKES || (frame && std::isfinite(P.surfFF[0]))) && P.stiffness[3] == 0.f && (P.flags & SPM_FLAG_FIRE);
 }
 
 // Pixels per warp of a scan of n pixels: 32, halved while that gives fewer than WARPS_PER_SCHEDULER warps
