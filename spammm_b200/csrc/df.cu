@@ -435,6 +435,16 @@ bool make_tile(const DfGeom& P, bool list, TileTaps& Q) {
     return true;
 }
 
+// A short height list node by node (df_amp_dir_kernel): the tile forms A at every height of its columns, whatever
+// the list.  Times as fitted on volumes of 200^2 and 480^2 pixels x 60 heights, in us: node by node 100 (latency) at
+// three axes + 2.8e-6 per row read, the tile 5.6e-7 per tap.  480 x 480 x 60, three axes: 1 height 478 us and 1315 by
+// tiles, 3 1033 and 1316, 4 1323 and 1317; 101 x 97 x 41 is by tiles from one height on.
+bool list_by_nodes(const DfGeom& P, const TileTaps& Q, int n_out) {
+    const double pix = (double)P.nx * P.ny, points = (double)Q.a[0] * Q.a[1] * Q.a[2] / ((double)Q.t[0] * Q.t[1]);
+    const double nodes = 33.0 * P.nact + pix * n_out * P.nact * (2.0 * DFT_MAX) * 2.8e-6;
+    return nodes < pix * points * Q.n * 5.6e-7;
+}
+
 template <typename T>
 int launch_df_tile(const T* FEs, const DfGeom& P, const TileTaps& Q, const int* out_iz, int n_out, float* df,
                    cudaStream_t st) {
@@ -660,7 +670,7 @@ extern "C" int spm_df_amp_dir(const void* FEs, int fes_dtype, int nx, int ny, in
         return check_launch("spm_df_amp_dir");
     }
     TileTaps Q;
-    if (make_tile(P, out_iz != nullptr, Q)) {
+    if (make_tile(P, out_iz != nullptr, Q) && !(out_iz && list_by_nodes(P, Q, n_out))) {
         if (fes_dtype == SPM_F32)
             return launch_df_tile(static_cast<const float*>(FEs), P, Q, out_iz, n_out, df, as_stream(stream));
         return launch_df_tile(static_cast<const double*>(FEs), P, Q, out_iz, n_out, df, as_stream(stream));

@@ -57,3 +57,40 @@ def test_height_outside_the_volume_is_nan(cuda):
     for d in ((0., 0., 1.), (0.1, 0., 1.)):
         got = gpu.df_amp_dir(F, 0.1, d, 0.5, out_iz=[-1, 3, 12]).cpu().numpy()
         assert np.isnan(got[..., [0, 2]]).all() and np.isfinite(got[..., 1]).all()
+
+
+@pytest.mark.parametrize("heights", [[17], [0, 39], list(range(0, 40, 4))])
+def test_tilted_height_list_of_a_large_volume(cuda, heights):
+    """Short lists are evaluated node by node, longer ones and the whole volume from tiles."""
+    F = np.random.default_rng(2).standard_normal((260, 250, 40, 4)).astype(np.float32)
+    d = (0.2, 0.1, 1.0)
+    got = gpu.df_amp_dir(F, 0.1, d, 1.0, out_iz=heights).cpu().numpy()
+    ref = gpu.df_amp_dir(F, 0.1, d, 1.0).cpu().numpy()[:, :, heights]
+    np.testing.assert_allclose(got, ref, rtol=2e-7, atol=1e-11 * np.abs(F).max() / 0.1)
+
+
+def _linear_without_zero_weights(F, coords):
+    """Linear interpolation with clamped indices; a corner of weight zero is not read."""
+    f = np.floor(coords)
+    out = np.zeros(F.shape)
+    for c in np.ndindex(2, 2, 2):
+        w = np.prod([np.where(c[d], coords[d] - f[d], 1.0 - (coords[d] - f[d])) for d in range(3)], axis=0)
+        v = F[tuple(np.clip(f[d].astype(int) + c[d], 0, F.shape[d] - 1) for d in range(3))]
+        out += np.where(w == 0.0, 0.0, v * w)
+    return out
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("direction", [(0., 0., 1.), (0., 0., -1.), (0.2, 0., 1.), (0.3, 0.2, 1.), (0., 1., 0.)])
+@pytest.mark.parametrize("amp", [0.1, 0.37])
+def test_samples_that_are_not_finite(cuda, value, direction, amp, monkeypatch):
+    """They reach the outputs that they reach node by node: the same NaN, infinities and finite values."""
+    rng = np.random.default_rng(7)
+    F = rng.standard_normal((9, 8, 40, 4)).astype(np.float32)
+    for x, y, z, c in ((4, 4, 20, 2), (0, 0, 0, 2), (8, 7, 39, 2), (2, 6, 5, 0), (6, 2, 33, 1), (4, 1, 12, 3)):
+        F[x, y, z, c] = value
+    monkeypatch.setattr(O, "_linear_nearest", _linear_without_zero_weights)
+    with np.errstate(invalid="ignore"):
+        ref = O.compute_df_amp_dir(F.astype(np.float64), 0.1, direction, amp)
+    got = gpu.df_amp_dir(F, 0.1, direction, amp).cpu().numpy()
+    np.testing.assert_allclose(got, ref, rtol=2e-7, atol=1e-9)
