@@ -125,9 +125,28 @@ def test_laws_of_another_shape(cuda):
                tol_rel=0.0)
 
 
+@pytest.mark.parametrize("column,value", [("x", np.inf), ("x", 1e30), ("q", np.nan), ("q", np.inf), ("c6", np.nan),
+                                          ("c6", np.inf), ("c12", np.nan), ("c12", np.inf)])
+def test_values_that_are_not_finite_as_in_direct_sums(cuda, column, value):
+    """One atom's coordinate, charge or parameter, far from the box and in it: NaN where the plain sum has NaN, finite
+    elsewhere."""
+    for at in (3, 200):
+        atoms, prm = _system(300, 0, 9.0)
+        atoms[at, :3] = (30.0, 2.0, 1.0) if at == 3 else (0.5, 0.5, 4.0)
+        {"x": atoms[:, 0], "q": atoms[:, 3], "c6": prm[:, 0], "c12": prm[:, 1]}[column][at] = value
+        vec = [np.array([*v, 0], np.float32) for v in ((-3, -3, 3), (0.125, 0, 0), (0, 0.125, 0), (0, 0, 0.125))]
+        Qs, QZs = (np.array(v, np.float32) for v in ON)
+        g = gpu.grid_build(0, atoms, prm, (48, 48, 40), *vec, Qs, QZs)
+        # the direct sums of a subset small enough for them, with the same atom
+        keep = np.r_[0:150] if at == 3 else np.r_[100:250]
+        d = gpu.grid_build(0, atoms[keep], prm[keep], (48, 48, 40), *vec, Qs, QZs)
+        assert torch.equal(torch.isfinite(g), torch.isfinite(d))
+        assert torch.equal(torch.isnan(g), torch.isnan(d))
+
+
 def test_atoms_that_are_not_finite_stay_in_the_sum(cuda):
     """A NaN coordinate is near every block: every node is NaN, as in the plain sum."""
-    atoms, prm = _system(64, 0, 8.0)
+    atoms, prm = _system(264, 0, 8.0)
     atoms[40, 0] = np.nan
     g = gpu.grid_build(0, atoms, prm, (40, 20, 20), *(np.array([*v, 0], np.float32) for v in
                        ((-20, -20, 5), (0.1, 0, 0), (0, 0.1, 0), (0, 0, 0.1))), np.array(ON[0], np.float32),
