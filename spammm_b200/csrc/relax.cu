@@ -713,7 +713,8 @@ __device__ __forceinline__ float4 sample_z(const AxisView& G, V3 p, TexelCache& 
     else return interp_fe_cell<IDX, LAYOUT>(G, p);
 }
 
-// PLAIN: FIRE without a radial bond (the tests left out of the loop: 64-molecule forward 27.2 -> 26.3 ms).
+// PLAIN: FIRE without a radial bond (the tests left out of the loop: strokes of the 64-molecule forward 23.4 -> 21.8
+// ms, polished 33.5 -> 32.4).
 template <typename IDX, bool CACHE, int LAYOUT, bool PLAIN = false>
 __device__ __forceinline__ bool pp_iter_z(const AxisView& G, TexelCache& T, const spm_scan_params& P, V3 tip,
                                           V3& pos, V3& v, float& dt, float& damp, float4& fe, int& it, int& total_it,
@@ -970,7 +971,7 @@ __device__ __forceinline__ void batch_polish_setup(const AxisView& G, const spm_
 // Newton's method finishes from the previous equilibrium is done; any other
 // returns false with nothing stored and L unchanged, for the FIRE pass to
 // redo from the same state.
-template <bool CACHE, int LAYOUT, bool POLISH, bool PREFIX>
+template <bool CACHE, int LAYOUT, bool POLISH, bool PREFIX, bool PLAIN>
 __device__ __forceinline__ bool stroke_zstep(const AxisView& G, TexelCache& T, const spm_scan_params& P,
                                              const PolishSpring& S, const float (&Tc)[3][3], StrokeLane& L,
                                              long long o, float dz, float4* __restrict__ FEs,
@@ -1019,14 +1020,8 @@ __device__ __forceinline__ bool stroke_zstep(const AxisView& G, TexelCache& T, c
     }
     L.total_it += it;
     if (!newton_done) {
-        if (P.stiffness[3] == 0.f && (P.flags & SPM_FLAG_FIRE)) {
-            while (!pp_iter_z<unsigned, CACHE, LAYOUT, true>(G, T, P, L.tip, pos, L.v, L.dt, L.damp, fe, it, L.total_it,
-                                                             conv)) {
-            }
-        } else {
-            while (!pp_iter_z<unsigned, CACHE, LAYOUT>(G, T, P, L.tip, pos, L.v, L.dt, L.damp, fe, it, L.total_it,
-                                                       conv)) {
-            }
+        while (!pp_iter_z<unsigned, CACHE, LAYOUT, PLAIN>(G, T, P, L.tip, pos, L.v, L.dt, L.damp, fe, it, L.total_it,
+                                                          conv)) {
         }
         if (!conv) fe = sample_z<unsigned, CACHE, LAYOUT>(G, pos, T);  // the position moved after the last sample
     }
@@ -1079,7 +1074,7 @@ __device__ __forceinline__ StrokeLane stroke_start(const float4* __restrict__ pt
 // POLISH: each z-step's equilibrium Newton-polished before it is stored (the
 // stroke continues from the unpolished position, as relax_pp_pixel and the
 // per-image kernels do).
-template <bool CACHE, int LAYOUT, bool POLISH>
+template <bool CACHE, int LAYOUT, bool POLISH, bool PLAIN>
 __device__ __forceinline__ void relax_tile_stroke(const spm_batch_mol* D, const float* __restrict__ grid,
                                                   const float4* __restrict__ pts, const spm_scan_params& P,
                                                   float4* __restrict__ FEs, float4* __restrict__ PPs,
@@ -1095,7 +1090,7 @@ __device__ __forceinline__ void relax_tile_stroke(const spm_batch_mol* D, const 
     float Tc[3][3];
     if constexpr (POLISH) batch_polish_setup(G, P, S, Tc);
     for (int iz = 0; iz < nzs; ++iz) {
-        stroke_zstep<CACHE, LAYOUT, POLISH, false>(G, T, P, S, Tc, L, sbase + iz, dz, FEs, PPs);
+        stroke_zstep<CACHE, LAYOUT, POLISH, false, PLAIN>(G, T, P, S, Tc, L, sbase + iz, dz, FEs, PPs);
         __syncwarp(members);  // the tile's lanes start the next z-step together
     }
     if (iter_count) iter_count[pix] = L.total_it;
@@ -1158,7 +1153,7 @@ batch_relax_prefix_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, uns
             batch_polish_setup(G, P, S, Tc);
             bool active = true;
             for (int iz = 0; iz < nzs; ++iz) {  // every member runs every z-step: the ballots stay uniform
-                const bool fail = active && !stroke_zstep<CACHE, LAYOUT, true, true>(G, T, P, S, Tc, L, sbase + iz,
+                const bool fail = active && !stroke_zstep<CACHE, LAYOUT, true, true, false>(G, T, P, S, Tc, L, sbase + iz,
                                                                                       dz, FEs, PPs);
                 const unsigned fm = __ballot_sync(members, fail);
                 if (fm) {
@@ -1224,7 +1219,8 @@ batch_relax_tail_kernel(const spm_batch_mol* __restrict__ mols, const float* __r
             const int steps = nzs - e.iz;
             const int rounds = __reduce_max_sync(members, steps);
             for (int r = 0; r < rounds; ++r) {  // the same count on every member
-                if (r < steps) stroke_zstep<CACHE, LAYOUT, true, false>(G, T, P, S, Tc, L, sbase + e.iz + r, dz, FEs, PPs);
+                if (r < steps)
+                    stroke_zstep<CACHE, LAYOUT, true, false, false>(G, T, P, S, Tc, L, sbase + e.iz + r, dz, FEs, PPs);
                 __syncwarp(members);
             }
             if (iter_count) iter_count[pix] = L.total_it;
@@ -1233,7 +1229,9 @@ batch_relax_tail_kernel(const spm_batch_mol* __restrict__ mols, const float* __r
     }
 }
 
-template <int MINB, bool CACHE, int LAYOUT, bool POLISH>
+// PLAIN (pp_iter_z) as a kernel of its own: both loops in one kernel cost the z-step's epilogue its registers (96
+// bytes spilled for 48): 64 molecules' strokes at 36 FIRE steps per z-step 22.4 ms (21.8 apart), at one step 4.7 (3.4).
+template <int MINB, bool CACHE, int LAYOUT, bool POLISH, bool PLAIN>
 __global__ void __launch_bounds__(MINB == 5 ? 128 : 256, MINB)
 batch_relax_sync_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, unsigned n_slots, int th_log2,
                         const float* __restrict__ grid, const float4* __restrict__ pts, spm_scan_params P,
@@ -1251,9 +1249,29 @@ batch_relax_sync_kernel(int n_mol, const spm_batch_mol* __restrict__ mols, unsig
         int k;
         const bool valid = slot_pixel(D, base + lane - (unsigned)D->slot_off, th_log2, k) && lane < (unsigned)lanes;
         const unsigned members = __ballot_sync(0xffffffffu, valid);
-        if (valid) relax_tile_stroke<CACHE, LAYOUT, POLISH>(D, grid, pts, P, FEs, PPs, iter_count, k, dz, members);
+        if (valid) relax_tile_stroke<CACHE, LAYOUT, POLISH, PLAIN>(D, grid, pts, P, FEs, PPs, iter_count, k, dz, members);
         __syncwarp();  // the whole warp draws the next tile
     }
+}
+
+using SyncKern = decltype(&batch_relax_sync_kernel<3, false, 2, false, false>);
+
+// The z-synchronised variants, [grid_layout][rx_regs].
+template <bool POLISH, bool PLAIN>
+SyncKern sync_variant(int layout, int regs) {
+    static const SyncKern table[2][5] = {
+        {batch_relax_sync_kernel<3, false, 2, POLISH, PLAIN>, batch_relax_sync_kernel<4, false, 2, POLISH, PLAIN>,
+         batch_relax_sync_kernel<2, true, 2, POLISH, PLAIN>, batch_relax_sync_kernel<3, true, 2, POLISH, PLAIN>,
+         batch_relax_sync_kernel<5, true, 2, POLISH, PLAIN>},
+        {batch_relax_sync_kernel<3, false, 4, POLISH, PLAIN>, batch_relax_sync_kernel<4, false, 4, POLISH, PLAIN>,
+         batch_relax_sync_kernel<2, true, 4, POLISH, PLAIN>, batch_relax_sync_kernel<3, true, 4, POLISH, PLAIN>,
+         batch_relax_sync_kernel<5, true, 4, POLISH, PLAIN>}};
+    return table[layout][regs];
+}
+
+SyncKern sync_kernel(int layout, int regs, bool polish, bool plain) {
+    if (polish) return plain ? sync_variant<true, true>(layout, regs) : sync_variant<true, false>(layout, regs);
+    return plain ? sync_variant<false, true>(layout, regs) : sync_variant<false, false>(layout, regs);
 }
 
 // ---- z-slab staging in shared memory through the bulk-copy (TMA) engine ----
@@ -1547,28 +1565,14 @@ extern "C" int spm_batch_relax(int n_mol, const spm_batch_mol* mols, long long n
     const bool two_pass = shape->rx_sync == 2 && (p->flags & SPM_FLAG_POLISH) && (p->flags & SPM_FLAG_WARM);
     const int sync = shape->rx_sync == 2 ? 1 : shape->rx_sync;
     using Kern = decltype(&batch_relax_kernel<3, false, 2>);
-    // [rx_sync][grid_layout][rx_regs]: 0 = 80 registers, 1 = 64, 2 = texel cache at up to 128,
+    // rx_sync = 0, [grid_layout][rx_regs]: 0 = 80 registers, 1 = 64, 2 = texel cache at up to 128,
     // 3 = texel cache squeezed to 80 (some values spilled, 50% more warps), 4 = texel cache at up to 102
     // (128-thread CTAs)
-    static const Kern table[2][2][5] = {
-        {{batch_relax_kernel<3, false, 2>, batch_relax_kernel<4, false, 2>, batch_relax_kernel<2, true, 2>,
-          batch_relax_kernel<3, true, 2>, batch_relax_kernel<5, true, 2>},
-         {batch_relax_kernel<3, false, 4>, batch_relax_kernel<4, false, 4>, batch_relax_kernel<2, true, 4>,
-          batch_relax_kernel<3, true, 4>, batch_relax_kernel<5, true, 4>}},
-        {{batch_relax_sync_kernel<3, false, 2, false>, batch_relax_sync_kernel<4, false, 2, false>,
-          batch_relax_sync_kernel<2, true, 2, false>, batch_relax_sync_kernel<3, true, 2, false>,
-          batch_relax_sync_kernel<5, true, 2, false>},
-         {batch_relax_sync_kernel<3, false, 4, false>, batch_relax_sync_kernel<4, false, 4, false>,
-          batch_relax_sync_kernel<2, true, 4, false>, batch_relax_sync_kernel<3, true, 4, false>,
-          batch_relax_sync_kernel<5, true, 4, false>}}};
-    // the polished z-synchronised variants, [grid_layout][rx_regs]
-    static const Kern polished[2][5] = {
-        {batch_relax_sync_kernel<3, false, 2, true>, batch_relax_sync_kernel<4, false, 2, true>,
-         batch_relax_sync_kernel<2, true, 2, true>, batch_relax_sync_kernel<3, true, 2, true>,
-         batch_relax_sync_kernel<5, true, 2, true>},
-        {batch_relax_sync_kernel<3, false, 4, true>, batch_relax_sync_kernel<4, false, 4, true>,
-         batch_relax_sync_kernel<2, true, 4, true>, batch_relax_sync_kernel<3, true, 4, true>,
-         batch_relax_sync_kernel<5, true, 4, true>}};
+    static const Kern lane_by_lane[2][5] = {
+        {batch_relax_kernel<3, false, 2>, batch_relax_kernel<4, false, 2>, batch_relax_kernel<2, true, 2>,
+         batch_relax_kernel<3, true, 2>, batch_relax_kernel<5, true, 2>},
+        {batch_relax_kernel<3, false, 4>, batch_relax_kernel<4, false, 4>, batch_relax_kernel<2, true, 4>,
+         batch_relax_kernel<3, true, 4>, batch_relax_kernel<5, true, 4>}};
     // the two-pass schedule's passes, [grid_layout][rx_regs]
     static const Kern prefix[2][5] = {
         {batch_relax_prefix_kernel<3, false, 2>, batch_relax_prefix_kernel<4, false, 2>,
@@ -1585,8 +1589,9 @@ extern "C" int spm_batch_relax(int n_mol, const spm_batch_mol* mols, long long n
          batch_relax_tail_kernel<2, true, 4>, batch_relax_tail_kernel<3, true, 4>, batch_relax_tail_kernel<5, true, 4>}};
     const Kern kern = shape->rx_regs == 5 ? batch_relax_staged_kernel
                       : two_pass ? prefix[shape->grid_layout][shape->rx_regs]
-                      : (p->flags & SPM_FLAG_POLISH) ? polished[shape->grid_layout][shape->rx_regs]
-                                                      : table[sync][shape->grid_layout][shape->rx_regs];
+                      : sync == 0 ? lane_by_lane[shape->grid_layout][shape->rx_regs]
+                                  : sync_kernel(shape->grid_layout, shape->rx_regs, (p->flags & SPM_FLAG_POLISH) != 0,
+                                                p->stiffness[3] == 0.f && (p->flags & SPM_FLAG_FIRE) != 0);
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
