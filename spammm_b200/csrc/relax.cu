@@ -36,7 +36,6 @@ namespace spm {
 namespace {
 
 constexpr int RX_THREADS = 128;
-constexpr int WARPS_PER_SCHEDULER = 1;
 
 // Pixel of this thread under the static schedule (one pixel per lane), or -1.
 __device__ __forceinline__ int pixel_of_thread(int n_scan, int raster_ny) {
@@ -384,20 +383,20 @@ struct DissArgs {
 // (49% of the lanes active per instruction on the 480x480-pixel scan), the
 // lanes of a warp run that code together: 3.81 -> 2.30 ms on that scan.
 //
-// lanes: pixels of a tile, 32 or, for scans that leave the schedulers short of
-// warps, a smaller power of two (tile_lanes; the other lanes idle).  A step
+// lanes: pixels of a tile, 32 or, for scans that leave schedulers without a
+// warp, a smaller power of two (tile_lanes; the other lanes idle).  A step
 // costs a warp the cell loads of any of its lanes, and a z-step the steps of its
 // slowest lane: fewer pixels per warp shorten both.  The polish reads its cells
-// through the texel cache of the FIRE loop (480 x 480 x 60 polished 3.03 -> 2.71
-// ms).  The
+// through the texel cache of the FIRE loop.  The
 // per-lane sequence is relax_kernel's (the same iteration, emit and texel
 // cache), so the results are the same bits.
 //
 // PLAIN (plain_scan): FIRE on an axis-aligned grid without a radial bond, the tilted modes with the frame x,
 // y, z -- the usual scan.  The transform's and the rotations' zero and unit terms and the per-step tests of
 // the flags are left out: the loop is bound by its instructions (157 per step, 3.7 cycles each with one warp
-// per scheduler), the same values up to the sign of a zero.  480 x 480 x 60: 2.11 -> 1.97 ms, with polished
-// PP bookkeeping 3.04 -> 2.52; 100 x 100 x 40: 648 -> 573 us.
+// per scheduler), the same values up to the sign of a zero.  General form -> this one, medians over five surfaces:
+// 480 x 480 pixels x 60 z-steps over 1200 atoms 2.35 -> 2.12 ms, with polished PP bookkeeping 3.17 -> 2.61 (3.79 before
+// the cached polish).
 template <int MODE, typename IDX, bool POLISH, bool PLAIN, bool DISS = false>
 __global__ void __launch_bounds__(RX_THREADS)
 relax_tile_kernel(GridView G, const float4* __restrict__ pts, int n_scan, spm_scan_params P,
@@ -614,16 +613,17 @@ bool plain_scan(int mode, const spm_scan_params& P) {
     return axis && (mode == SPM_RELAX_STROKES || (frame && std::isfinite(P.surfFF[0]))) && P.stiffness[3] == 0.f && (P.flags & SPM_FLAG_FIRE);
 }
 
-// Pixels per warp of a scan of n pixels: 32, halved while that gives fewer than WARPS_PER_SCHEDULER warps
-// for each of the GPU's schedulers.  100 x 100 pixels x 40 z-steps: 32 pixels per warp 893 us, at least one
-// warp per scheduler (16 pixels) 658, two (8) 718, four (4) 980; 24 x 24 x 20: 358 -> 311.
+// Pixels per warp of a scan of n pixels: 32, halved while that leaves every scheduler at most one warp (of a second
+// one the first would wait for issue).  Axis-aligned loop over 40 z-steps of 38 atoms, in us with 32 pixels per
+// warp / by this rule / with half as many again: 24 x 24 x 20 279 / 240 (1 pixel); 64 x 64 552 / 507 (8) / 563; 80 x
+// 80 549 / 524 (16) / 573; 100 x 100 550 (32) / 582.
 int tile_lanes(long long n, int& lanes) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return set_error(SPM_ERR_CUDA, "relax: cannot query the device");
     lanes = 32;
-    while (lanes > 1 && (n + lanes - 1) / lanes < (long long)WARPS_PER_SCHEDULER * 4 * sms) lanes /= 2;
+    while (lanes > 1 && (n + lanes / 2 - 1) / (lanes / 2) <= 4LL * sms) lanes /= 2;
     return SPM_OK;
 }
 
