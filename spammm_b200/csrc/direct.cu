@@ -194,17 +194,16 @@ __device__ __noinline__ double group_force2_f64(V3 p, V3 tip, int na, int sub, u
     return fx * fx + fy * fy + fz * fz;
 }
 
-// Bound of |F32 - F64| of the total force at p, summed over the group: what the FP32 evaluation above can be
-// off from group_force2_f64, from its roundings.  Per atom, with x the exponent of the Morse factor e:
+// Bounds of |F32 - F64| of the total force at p: what the FP32 evaluation above can be off from
+// group_force2_f64, from its roundings.  group_pair_error, summed over the group: per atom, with x the exponent of the Morse factor e:
 // differences, r^2, rsqrt.approx and r = r^2 rsqrt err by at most 8e-7 of r, so e errs by (8e-7 + 2^-23)
 // |x| ln 2 < 1.5e-6 |x|, and the force 2 K E0 e (e - 1), whose difference cancels near the minimum, by that
 // times e (1 + e) plus 2e-6 for its own products; a charge site's force by 2e-6 and by 4e-7 (|dz| + |qz|) / r
-// for the rounded offset; the sum of na terms adds na 2^-24 of their magnitudes.  The spring: 4e-7 of the
+// for the rounded offset; the sum of na terms adds na 2^-24 of their magnitudes.  spring_error: 4e-7 of the
 // lengths times their stiffnesses (rotations by an orthonormal frame, root, products) and of the force itself.
 template <int NS, int LPP>
-__device__ __noinline__ float group_force_bound(V3 p, V3 tip, int na, int sub, unsigned gmask, const float4* s_pos,
-                                                const float4* s_m, const float* s_q, const Sites& S, float4 kk,
-                                                float4 d0, float surf) {
+__device__ __noinline__ float group_pair_error(V3 p, int na, int sub, unsigned gmask, const float4* s_pos,
+                                               const float4* s_m, const float* s_q, const Sites& S) {
     float err = 0.f, mag = 0.f;
     for (int j = sub; j < na; j += LPP) {
         const float4 a = s_pos[j];
@@ -228,11 +227,13 @@ __device__ __noinline__ float group_force_bound(V3 p, V3 tip, int na, int sub, u
     }
     err = group_sum<LPP>(err, gmask);
     mag = group_sum<LPP>(mag, gmask);
-    const V3 d = sub3(p, tip);
+    return err + 6e-8f * (float)(na + 8) * mag;
+}
+
+__device__ __forceinline__ float spring_error(V3 d, float4 kk, float4 d0, float surf) {
     const float len = sqrtf(dot3(d, d)), l0 = fabsf(d0.x) + fabsf(d0.y) + fabsf(d0.z);
     const float k3 = fmaxf(fabsf(kk.x), fmaxf(fabsf(kk.y), fabsf(kk.z)));
-    const float spring = k3 * (len + l0) + fabsf(kk.w) * (len + 0.25f * fabsf(len - fabsf(d0.w))) + fabsf(surf);
-    return err + 6e-8f * (float)(na + 8) * mag + 4e-7f * spring;
+    return 4e-7f * (k3 * (len + l0) + fabsf(kk.w) * (len + 0.25f * fabsf(len - fabsf(d0.w))) + fabsf(surf));
 }
 
 // Groups of LPP lanes, one pixel per group (blockDim / LPP pixels per CTA, in raster order); the
@@ -302,9 +303,13 @@ relax_direct_kernel(int na, const float4* __restrict__ atoms, const float4* __re
             bool below = false;
             if (f2 < P.f2conv) {
                 if (bound) {
-                    const float far = sqrtf(f2) + group_force_bound<NS, LPP>(pos, tip, na, sub, gmask, s_pos, s_m, s_q,
-                                                                             S, kk, d0, surf);
-                    below = far * far < 0.999f * P.f2conv;
+                    // where the spring's share alone leaves no room, the atoms' is not summed: slow strokes step over
+                    // the threshold by a percent and need FP64 anyway
+                    const float most = sqrtf(f2) + spring_error(d, kk, d0, surf);
+                    if (most * most < 0.98f * P.f2conv) {
+                        const float far = most + group_pair_error<NS, LPP>(pos, na, sub, gmask, s_pos, s_m, s_q, S);
+                        below = far * far < 0.999f * P.f2conv;
+                    }
                 }
                 below = below ||
                         group_force2_f64<LPP>(pos, tip, na, sub, gmask, atoms, cMs, S, a, b, c, kk, d0,
@@ -658,13 +663,15 @@ int launch_direct(int na, const float* atoms, const float* cMs, const float* poi
                   const spm_scan_params& P, const Sites& S, float* FEs, float* PPs, cudaStream_t st) {
     const size_t smem = (size_t)na * (2 * sizeof(float4) + NS * sizeof(float));
     // The order of the atom sums is that of four atoms per lane (unpolished strokes stop elsewhere within their
-    // threshold in another order); the launch takes eight, half the lanes with two partial sums each.  38 atoms,
-    // 100 x 100 pixels x 40 z-steps: 16 lanes per pixel 1405 us, 8 lanes in this order 1247 (1163 in their own
-    // order), 4 lanes 1850 (two warps per scheduler); with 64 x 50 pixels half as many warps cost 638 us
-    // against 466.
-    const int lpp = direct_lpp(na, n_scan, 8);
-    const bool two = direct_lpp(na, n_scan, 4) != lpp;  // twice as many then
-    auto kern = lpp == 4    ? (two ? relax_direct_kernel<NS, 4, 2> : relax_direct_kernel<NS, 4, 1>)
+    // threshold in another order).  From 33 atoms on the launch takes half the lanes with two partial sums each where
+    // that pads fewer atoms or the scan still gives every scheduler eight warps.  Full width / half, 20 z-steps, us: 38
+    // atoms on 100 x 100 pixels 639 / 595, 50 1174 / 802, 80 1216 / 945; 64 atoms (no padding) on 80 x 80 615 / 663, on
+    // 180 x 180 2221 / 1816; 20 atoms on 100 x 100 434 / 601.
+    const int width = direct_lpp(na, n_scan, 4), half = direct_lpp(na, n_scan, 8);
+    const bool fewer = (na + half - 1) / half * half < (na + width - 1) / width * width;
+    const int lpp = na > 32 && (fewer || (long long)n_scan * half >= 148LL * 4 * 8 * 32) ? half : width;
+    const bool two = width != lpp;  // twice as many then
+    auto kern = lpp == 4    ? relax_direct_kernel<NS, 4, 1>
                 : lpp == 8  ? (two ? relax_direct_kernel<NS, 8, 2> : relax_direct_kernel<NS, 8, 1>)
                 : lpp == 16 ? (two ? relax_direct_kernel<NS, 16, 2> : relax_direct_kernel<NS, 16, 1>)
                             : relax_direct_kernel<NS, 32, 1>;

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 # pixels on both sides of the scan sizes at which the molecule's lane count halves
-@pytest.mark.parametrize("na,few,many", [(17, 4800, 9600), (32, 4800, 9600), (38, 2400, 4800), (64, 2400, 4800),
+@pytest.mark.parametrize("na,few,many", [(17, 4800, 9600), (32, 4800, 9600), (33, 2400, 4800), (38, 2400, 4800), (64, 2400, 4800),
                                          (65, 1200, 2400), (101, 1200, 2400), (128, 1200, 2400)])
 @pytest.mark.parametrize("sites", [0, 1, 2])
 def test_scan_size_does_not_change_bits(cuda, na, few, many, sites):
