@@ -171,9 +171,12 @@ def adjoint_grid_state(grid, params, points, PPs, dL_dFEs):
 
 
 # adjoint_grid_params takes the node-major form from so many (state, atom) pairs on -- 4.4e5 pairs take 108 us
-# either way, 1.2e6 128 us against the gather's 147, 1.5e7 233 against 826 -- on grids whose node sums take up
-# to 2 GB
+# either way, 1.2e6 128 us against the gather's 147, 1.5e7 233 against 826 -- where there are atoms and states
+# enough for it: 1.6e6 states with one atom 266 us against 184, with three 262 against 330; 1000 atoms with 1440
+# states 194 against 164, with 9000 350 against 527.  Its node sums take up to 2 GB (the gather where they cannot be had).
 NODES_MIN_PAIRS = 1 << 20
+NODES_MIN_ATOMS = 3
+NODES_MIN_STATES = 1 << 12
 NODES_MAX_GRID = 1 << 26
 
 
@@ -191,7 +194,8 @@ def adjoint_grid_params(kind, atoms, params_atoms, p0, dA, dB, dC, Qs, QZs, grid
     dk_sum = torch.empty((4,), dtype=F64, device=atoms.device)
     hv = [hostvec(v) for v in (p0, dA, dB, dC, Qs, QZs)]
     scratch = None
-    if na and n_state * na >= NODES_MIN_PAIRS and scan_params.nz > 0 and nx * ny * nz <= NODES_MAX_GRID:
+    if (na >= NODES_MIN_ATOMS and n_state >= NODES_MIN_STATES and n_state * na >= NODES_MIN_PAIRS and scan_params.nz > 0
+            and nx * ny * nz <= NODES_MAX_GRID):
         nbytes = int(lib().spm_adjoint_grid_nodes_scratch_bytes(na, n_state, nx, ny, nz))
         try:
             scratch = torch.empty(((nbytes + 15) // 16, 2), dtype=F64, device=atoms.device)

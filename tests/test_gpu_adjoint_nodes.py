@@ -40,6 +40,8 @@ def _case(kind, na, nxy, nz, seed, n=(70, 66, 60), step=0.2, spread=6.0, sites=(
 
 def _both(args, monkeypatch):
     out = []
+    monkeypatch.setattr(gpu, "NODES_MIN_ATOMS", 1)
+    monkeypatch.setattr(gpu, "NODES_MIN_STATES", 1)
     for limit in (1 << 62, 0):
         monkeypatch.setattr(gpu, "NODES_MIN_PAIRS", limit)
         out.append(gpu.adjoint_grid_params(*args))
@@ -60,6 +62,7 @@ def test_matches_state_major(cuda, kind, na, nxy, nz, monkeypatch):
 def test_repeats_bit_for_bit_and_ignores_the_scratch(cuda, monkeypatch):
     args = _case(0, 38, 200, 20, seed=5)
     monkeypatch.setattr(gpu, "NODES_MIN_PAIRS", 0)
+    monkeypatch.setattr(gpu, "NODES_MIN_STATES", 1)
     a = gpu.adjoint_grid_params(*args)
     junk = torch.full((40 << 20,), 3.7e5, device="cuda")  # what the next scratch may be made of
     del junk
@@ -70,6 +73,7 @@ def test_repeats_bit_for_bit_and_ignores_the_scratch(cuda, monkeypatch):
 def test_no_weight_and_weights_that_are_not_finite(cuda, monkeypatch):
     args = list(_case(0, 38, 50, 20, seed=7))
     monkeypatch.setattr(gpu, "NODES_MIN_PAIRS", 0)
+    monkeypatch.setattr(gpu, "NODES_MIN_STATES", 1)
     ub = args[12]
     args[12] = np.zeros_like(ub)
     assert torch.count_nonzero(gpu.adjoint_grid_params(*args)[0]) == 0
