@@ -435,14 +435,19 @@ bool make_tile(const DfGeom& P, bool list, TileTaps& Q) {
     return true;
 }
 
-// A short height list node by node (df_amp_dir_kernel): the tile forms A at every height of its columns, whatever
-// the list.  Times as fitted on volumes of 200^2 and 480^2 pixels x 60 heights, in us: node by node 100 (latency) at
-// three axes + 2.8e-6 per row read, the tile 5.6e-7 per tap.  480 x 480 x 60, three axes: 1 height 478 us and 1315 by
-// tiles, 3 1033 and 1316, 4 1323 and 1317; 101 x 97 x 41 is by tiles from one height on.
-bool list_by_nodes(const DfGeom& P, const TileTaps& Q, int n_out) {
-    const double pix = (double)P.nx * P.ny, points = (double)Q.a[0] * Q.a[1] * Q.a[2] / ((double)Q.t[0] * Q.t[1]);
-    const double nodes = 33.0 * P.nact + pix * n_out * P.nact * (2.0 * DFT_MAX) * 2.8e-6;
-    return nodes < pix * points * Q.n * 5.6e-7;
+// Node by node (df_amp_dir_kernel) where the tiles would do more: they form A at every height of their columns,
+// whatever the list, and a long reach across stages hundreds of points per output.  Times as fitted on volumes of 64^2
+// to 480^2 pixels, in us: node by node 33 per axis (latency) + 1.8e-6 per row read (2.8e-6 for the scattered heights of
+// a list); tiles 5.9e-6 per staged point + 3e-7 per tap.  Three axes, 480 x 480 x 60: 1 height 478 us and 1315 by
+// tiles, 3 1033 and 1316, 4 1323 and 1317, all 12742 and 1230; along (1, 1, 0) with a reach of 9 samples, 64 x 64 x
+// 100: 150 and 555.
+bool by_nodes(const DfGeom& P, const TileTaps& Q, int n_out, bool list) {
+    double tiles = 1.0;
+    const int dims[3] = {P.nx, P.ny, P.nz};
+    for (int d = 0; d < 3; d++) tiles *= (dims[d] + Q.t[d] - 1) / Q.t[d];
+    const double staged = (double)Q.f[0] * Q.f[1] * Q.f[2], points = (double)Q.a[0] * Q.a[1] * Q.a[2];
+    const double rows = (double)P.nx * P.ny * n_out * P.nact * (2.0 * DFT_MAX);
+    return 33.0 * P.nact + rows * (list ? 2.8e-6 : 1.8e-6) < tiles * (staged * 5.9e-6 + points * Q.n * 3e-7);
 }
 
 template <typename T>
@@ -670,7 +675,7 @@ extern "C" int spm_df_amp_dir(const void* FEs, int fes_dtype, int nx, int ny, in
         return check_launch("spm_df_amp_dir");
     }
     TileTaps Q;
-    if (make_tile(P, out_iz != nullptr, Q) && !(out_iz && list_by_nodes(P, Q, n_out))) {
+    if (make_tile(P, out_iz != nullptr, Q) && !by_nodes(P, Q, n_out, out_iz != nullptr)) {
         if (fes_dtype == SPM_F32)
             return launch_df_tile(static_cast<const float*>(FEs), P, Q, out_iz, n_out, df, as_stream(stream));
         return launch_df_tile(static_cast<const double*>(FEs), P, Q, out_iz, n_out, df, as_stream(stream));

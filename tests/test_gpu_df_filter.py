@@ -80,6 +80,12 @@ def _linear_without_zero_weights(F, coords):
     return out
 
 
+def test_long_reach_across(cuda):
+    """A reach of nine samples in the plane: node by node where tiles would stage hundreds of points per output."""
+    _check((64, 64, 100), 0.1, (1.0, 1.0, 0.0), 1.25, np.float32)
+    _check((64, 64, 40), 0.1, (1.0, 1.0, 0.0), 1.25, np.float32)
+
+
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 @pytest.mark.parametrize("direction", [(0., 0., 1.), (0., 0., -1.), (0.2, 0., 1.), (0.3, 0.2, 1.), (0., 1., 0.)])
 @pytest.mark.parametrize("amp", [0.1, 0.37])
