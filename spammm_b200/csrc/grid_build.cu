@@ -293,8 +293,12 @@ grid_build_kernel(int na, const float4* __restrict__ atoms, const float* __restr
 // Interpolation error of one atom relative to its own force at the node (float64, worst corner and direction,
 // at 9 half-edges): 1/r^2 3e-9, r^-7 1e-6, and much less over most of the block, falling as the eighth power of
 // the distance -- the direct float32 sum rounds r^-7 by 8e-7 (rsqrt.approx), and the sums are 2-17 times
-// shorter.  Measured error of the forces at the nodes a probe reaches (|E| < 0.5 eV), relative to their norm,
-// direct sum -> blocks: 1200 LJ atoms on an ionic slab 1.98e-6 -> 1.89e-6 (energy 2.9e-6 -> 1.7e-6).
+// shorter.  Measured against 64 bits over 256 to 1200 atoms on ionic slabs, spacings of 0.02 to 0.5 A and three sets of
+// tip charges: the error of the forces at the nodes a probe reaches (|E| < 0.5 eV), relative to their norm, is 0.94 of
+// the direct sum's (0.82 to 1.01 by spacing and size), over all nodes and relative to the terms' magnitudes 0.91; of
+// the energies 0.94 and 0.85 (single systems where few atoms are far up to 1.2: alternating charges cancel less in
+// another order).  1200 atoms at 0.1 A: 3.0e-6 -> 2.9e-6 over the
+// whole grid.
 //
 // LJ only.  A Morse exponential varies with |K| times the half-edge, at any distance: at 0.1 A (|K| h = 1.35)
 // its interpolation errs by 4e-6 of the local force, at |K| h = 1.5 by 1.7e-5, where the direct sum errs by up
@@ -307,7 +311,9 @@ grid_build_kernel(int na, const float4* __restrict__ atoms, const float* __restr
 // SPM_FAR_MIN_ATOMS: molecules keep the direct sum's order and bits.  Unpolished FIRE strokes stop where their
 // force falls below the threshold, so a grid that differs in its last bits moves their images by 1e-4 (64
 // molecules of 10 to 120 atoms), and with few atoms most are near most blocks: 38 atoms on 200^3 nodes take
-// 187 us directly and 124 in blocks, 256 1223 against 461, 1200 on 480 x 480 x 240 32.0 ms against 2.28.
+// 187 us directly and 124 in blocks, 256 1223 against 461, 1200 on 480 x 480 x 240 32.0 ms against 2.37.  Of the
+// latter's time the near sums take 0.67 ms, the far points 0.91, the interpolation along y and z 0.18, and
+// classification, gathers, the interpolation along x and the stores the rest (each left out in turn).
 constexpr int FAR_REF = 3 * 64 + 3 * 8 + 3;  // the point whose value is interpolated as a constant
 constexpr int FAR_CHUNK = 256;       // atoms gathered at a time
 
@@ -512,8 +518,7 @@ __device__ __forceinline__ void build_cell(FarShared<NOFF>& M, int child0, int c
             __syncthreads();
         }
         // the interpolation acts on the differences from one point's value, which is added last: its rounding
-        // is relative to the field's variation over the block, not to the field (error of the FE samples of 100 x
-        // 100 x 40 polished states over a 38-atom molecule, six seeds: 8.6e-7 -> 8.3e-7; 8.0e-7 with direct sums)
+        // is relative to the field's variation over the block, not to the field
         float4 ref = make_float4(0.f, 0.f, 0.f, 0.f);
         if (field) {  // along x: points (ky, kz) x 16 nodes
             ref = M.part[0][FAR_REF];
@@ -599,9 +604,9 @@ __device__ __forceinline__ void load_far_tab(FarShared<NOFF>& M, const FarTab& t
     __syncthreads();
 }
 
-// 256 threads, 16 nodes along z each, at 128 registers (two CTAs per SM): 2.24 ms on the 1200-atom 480 x 480
-// x 240 grid (128 threads 2.25, 8 nodes each 2.36; 0.47 ms against 0.71 and 0.44 on 527 atoms, 243 x 138 x
-// 98).  The differences from one point cost 2% since.
+// 256 threads, 16 nodes along z each, at 128 registers (two CTAs per SM, 60 to 150 bytes spilled): measured in turn on
+// the 1200-atom 480 x 480 x 240 grid 2.24 ms, 128 threads 2.25, 8 nodes each (no spills) 2.36; on 527 atoms, 243 x
+// 138 x 98, 0.47, 0.71 and 0.44.
 constexpr int FAR_THREADS = 256;
 
 // A whole grid: one CTA per lattice cell, or per 4, 2 or 1 blocks of a group while the groups alone would
